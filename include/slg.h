@@ -322,7 +322,7 @@ int slg_autotune_transport(slg_ctx* ctx, const slg_transport_in* in, const slg_p
 /* Select the transport kernel variant (0..3, register budget / resident
  * blocks, as slg_autotune_transport times them) of both precisions explicitly,
  * e.g. after timing each on full launches of the caller's own workload.  A new
- * context starts with FP64 variant 2 and mixed variant 3, the fastest on whole
+ * context starts with FP64 variant 0 (1 for several models) and mixed variant 3, the fastest on whole
  * steps of a large batched workload. */
 int slg_set_transport_variant(slg_ctx* ctx, int32_t variant);
 /* radtemp, prt and isvacant on the device; emit and nvol are host arrays. */
@@ -351,7 +351,7 @@ typedef struct slg_grid_dev {
  * counterpart in the reference: an addition of this library).  Same semantics
  * as slg_dev_particle_advance, but needs no context and calls no allocator:
  * every input and output is a caller-owned device pointer, and the per-cell
- * tables and counters live in one fixed 6.5 MiB __device__ array that every GPU
+ * tables and counters live in one fixed 15.5 MiB __device__ array that every GPU
  * loading the library holds until exit.  Grids beyond SLG_STATIC_MAX_CELLS
  * shells or SLG_STATIC_MAX_CELLGROUPS (shells x groups) return
  * SLG_ERR_TOO_LARGE.  Runs on `stream` (a cudaStream_t, NULL = default) on the

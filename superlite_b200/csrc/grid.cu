@@ -346,6 +346,7 @@ struct TabArgs {
   double tauddmc, taulump;
   CellTables T;
   const int4* cellmap = nullptr;  // as LeakArgs::cellmap
+  int fp64 = 1;                   // build what only the FP64 loop reads
 };
 
 // Arguments seen from cell c (see leak_view); *ic is the 1-based shell.
@@ -365,10 +366,62 @@ __device__ inline TabArgs tab_view(TabArgs A, int c, int* ic) {
     A.T.specarr += cg; A.T.glumps += cg; A.T.cdf_dop += cg; A.T.cdf_left += cg; A.T.cdf_right += cg;
     A.T.cdf_scat += cg; A.T.emitcum += cg;
     if (A.T.guide) A.T.guide += (size_t)co * 4 * (A.T.guide_m + 1);
+    if (A.T.fine) A.T.fine += (size_t)co * kFineTables * A.T.fine_m;
     A.T.nlump += co;
     A.T.scal += (size_t)SCAL_N * co;
   }
   return A;
+}
+
+// CdfEntry::info of group ig of cell l (1-based; c: its opacity, dist: its width).
+__device__ inline int group_info(const TabArgs& A, int l, double dist, int ig, double c) {
+  if ((A.sig[l - 1] + c) * dist < A.tauddmc) return ig | kInfoImc;
+  const bool lumped = c * dist >= A.taulump && A.opaclump[(size_t)11 * (l - 1) + 6] != 0.0;
+  return lumped ? ig | kInfoLumped : ig;
+}
+
+// In-place running sum in index order by one thread.  A chain of dependent FP64
+// additions; the terms of the next round are loaded while a round is added
+// (a load per addition made it wait on memory each time).
+__device__ inline void running_sum(CdfEntry* __restrict__ a, int n) {
+  constexpr int N = 16;
+  double v[N], s = 0.0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) v[j] = j < n ? a[j].sum : 0.0;
+  for (int q = 0; q < n; q += N) {
+    double w[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) w[j] = q + N + j < n ? a[q + N + j].sum : 0.0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      s = s + v[j];
+      if (q + j < n) a[q + j].sum = s;
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = w[j];
+  }
+}
+
+// 1 / (sum of the branch rates) and the branch limits {P(Doppler), P(Doppler) +
+// P(left leak)} (diffusion11.f90:232-278).
+__device__ inline double2 ddmc_rates(double o1, double o2, double emitlump, double caplump, double doplump,
+                                     double* denom) {
+  double d = (o1 + o2) + (1.0 - emitlump) * caplump + doplump;
+  d = 1.0 / d;
+  *denom = d;
+  const double pdop = doplump * d;
+  return make_double2(pdop, pdop + o1 * d);
+}
+
+// number of leading entries of a (n, non-decreasing) not above v
+__device__ inline int count_le(const CdfEntry* __restrict__ a, int n, double v) {
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (a[mid].sum <= v) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
 }
 
 // Per-cell transport tables (see CellTables).  Phase A computes every term in
@@ -454,10 +507,10 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
   }
   __syncthreads();  // glumps and specarr visible to the block
   const double divv = A.divv[ix - 1];
-  double* cdop = A.T.cdf_dop + off;
-  double* cleft = A.T.cdf_left + off;
-  double* cright = A.T.cdf_right + off;
-  double* cscat = A.T.cdf_scat + off;
+  CdfEntry* cdop = A.T.cdf_dop + off;
+  CdfEntry* cleft = A.T.cdf_left + off;
+  CdfEntry* cright = A.T.cdf_right + off;
+  CdfEntry* cscat = A.T.cdf_scat + off;
   double* ecum = A.T.emitcum + off;
   // ---- phase A: terms
   if (nlump > 0) {
@@ -468,8 +521,11 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
       // Doppler (diffusion11.f90:290-314): position q in loop order
       if (q <= nlump) {
         double t = 0.0;
+        int from, to;  // the resolved group and the one it shifts to
         if (divv >= 0.0) {
           const int iiig = glumps[q - 1];
+          from = iiig;
+          to = min(iiig + 1, ng);
           if (!(iiig == ng) && !((double)capc[iiig] * dist >= A.taulump)) {
             const double res = dopspeccalc(tinv, A.wlinv, iiig) * divv / (3.0 * pc_c);
             t = res * speclump * hdop;
@@ -477,12 +533,14 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
         } else {
           const int iig = nlump + 1 - q;
           const int iiig = glumps[iig - 1];
+          from = iiig;
+          to = max(iiig - 1, 1);
           if (!(iiig == 1) && !((double)capc[iiig - 2] * dist >= A.taulump)) {
             const double res = dopspeccalc(tinv, A.wlinv, iiig - 1) * divv / (3.0 * pc_c);
             t = -(res * speclump * hdop);
           }
         }
-        cdop[q - 1] = t;
+        cdop[q - 1] = CdfEntry{t, from | (group_info(A, ic, dist, to, (double)capc[to - 1]) & ~0xffff), 0};
         // left leak (:378-397)
         const int iiig = glumps[q - 1];
         const double specig = specarr[iiig - 1];
@@ -500,10 +558,11 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
             const double mfphelp = (sigc + capi) * dist + (A.sig[l - 1] + capl) * dxl;
             res = 2.0 * sq(X0) / (mfphelp * dx3);
           }
-          cleft[q - 1] = specig * res * speclump * hl;
+          cleft[q - 1] = CdfEntry{specig * res * speclump * hl, group_info(A, l, dxl, iiig, capl), 0};
         }
         // right leak: boundary (:450-460) or interior (:492-511)
         double res;
+        int info = iiig;
         if (ix == A.nx) {
           const double mfphelp = (capi + sigc) * dist;
           const double ppr = 4.0 / (3.0 * mfphelp + 6.0 * pc_dext);
@@ -512,6 +571,7 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
           const int l = ix + 1;
           const double capl = (double)A.cap[(size_t)(l - 1) * ng + iiig - 1];
           const double dxr = A.xarr[ix + 1] - A.xarr[ix];
+          info = group_info(A, l, dxr, iiig, capl);
           if ((capl + A.sig[l - 1]) * dxr < A.tauddmc) {
             const double mfphelp = (capi + sigc) * dist;
             const double ppr = 4.0 / (3.0 * mfphelp + 6.0 * pc_dext);
@@ -521,65 +581,204 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
             res = 2.0 * sq(X1) / (mfphelp * dx3);
           }
         }
-        cright[q - 1] = specig * res * speclump * hr;
+        cright[q - 1] = CdfEntry{specig * res * speclump * hr, info, 0};
       }
       // effective scattering over unlumped groups (:571-584), loop order q
       if (q <= ng - nlump) {
         const int iig = ng + 1 - q;
         const int iiig = glumps[iig - 1];
         const double help = specarr[iiig - 1] * (double)capc[iiig - 1] * capgreyinv;
-        cscat[q - 1] = help * denom2;
+        cscat[q - 1] = CdfEntry{help * denom2, group_info(A, ic, dist, iiig, (double)capc[iiig - 1]), 0};
       }
     }
   }
-  // emitgroup within-bin running sums (emitgroup.f:303-320), one thread per bin
-  const double* ep = A.emitprob + (size_t)A.nep * (ic - 1);
-  for (int iep = threadIdx.x; iep <= A.nep; iep += GB) {
-    const int ig0 = iep * A.nepg + 1;
-    const int igp1 = min(ig0 + A.nepg - 1, ng);
-    double prob = iep == 0 ? 0.0 : ep[iep - 1];
-    for (int g = ig0; g <= igp1 - 1; ++g) {
-      prob = prob + specarr[g - 1] * (double)capc[g - 1];
-      ecum[g - 1] = prob;
+  // emitgroup's thresholds (emitgroup.f:303-320), one thread per emission bin.
+  // The reference takes the bin iep = number of ep(1:nep-1) not above r1 and in
+  // it the first group whose running sum from ep(iep) exceeds r1, else the
+  // bin's last.  Flattened over the bins, entry g-1 is the r1 from which the
+  // answer passes group g: the running sum inside a bin, kept from passing the
+  // next bin's start (which rounding could otherwise do), and that start at
+  // the bin's last group.  The entries are non-decreasing, so the answer is
+  // one plus the number of entries not above r1.
+  if (A.fp64) {
+    const double* ep = A.emitprob + (size_t)A.nep * (ic - 1);
+    const int last = emit_last_group(A.nep, A.nepg, ng);
+    for (int iep = threadIdx.x; iep < A.nep; iep += GB) {
+      const int ig0 = iep * A.nepg + 1;
+      const int igp1 = min(ig0 + A.nepg - 1, last);
+      double prob = iep == 0 ? 0.0 : ep[iep - 1];
+      const bool end = iep == A.nep - 1;
+      const double next = end ? DBL_MAX : ep[iep];
+      for (int g = ig0; g <= igp1 - 1; ++g) {
+        prob = prob + specarr[g - 1] * (double)capc[g - 1];
+        ecum[g - 1] = !end && prob > next ? next : prob;
+      }
+      if (igp1 >= ig0 && igp1 < last) ecum[igp1 - 1] = next;
     }
   }
   __syncthreads();
   // ---- phase B: running sums
   if (nlump > 0) {
-    if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int q = 0; q < nlump; ++q) { s = s + cdop[q]; cdop[q] = s; }
-    } else if (threadIdx.x == 32 && ix > 1) {
-      double s = 0.0;
-      for (int q = 0; q < nlump; ++q) { s = s + cleft[q]; cleft[q] = s; }
-    } else if (threadIdx.x == 64) {
-      double s = 0.0;
-      for (int q = 0; q < nlump; ++q) { s = s + cright[q]; cright[q] = s; }
-    } else if (threadIdx.x == 96) {
-      double s = 0.0;
-      for (int q = 0; q < ng - nlump; ++q) { s = s + cscat[q]; cscat[q] = s; }
-    }
+    if (threadIdx.x == 0) running_sum(cdop, nlump);
+    else if (threadIdx.x == 32 && ix > 1) running_sum(cleft, nlump);
+    else if (threadIdx.x == 64) running_sum(cright, nlump);
+    else if (threadIdx.x == 96) running_sum(cscat, ng - nlump);
   }
-  // ---- phase C: guide tables of the four running sums (see CellTables::guide)
-  if (A.T.guide && nlump > 0) {
-    __syncthreads();
+  // ---- phase C: guide tables: the mixed loop's (CellTables::guide) or the FP64 loop's
+  __syncthreads();
+  if (!A.fp64 && A.T.guide && nlump > 0) {
     const int gm = A.T.guide_m;
     int16_t* gd = A.T.guide + (size_t)(ic - 1) * 4 * (gm + 1);
     for (int t = 0; t < 4; ++t) {
-      const double* a = t == 0 ? cdop : (t == 1 ? cleft : (t == 2 ? cright : cscat));
+      const CdfEntry* a = t == 0 ? cdop : (t == 1 ? cleft : (t == 2 ? cright : cscat));
       const int n = t == 3 ? ng - nlump : nlump;
-      for (int k = threadIdx.x; k <= gm; k += blockDim.x) {
-        const double v = (double)k / (double)gm;  // exact: gm is a power of two
-        int lo = 0, hi = (t == 1 && ix == 1) ? 0 : n;  // no left leak from the first shell
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (a[mid] <= v) lo = mid + 1;
-          else hi = mid;
-        }
-        gd[t * (gm + 1) + k] = (int16_t)lo;
-      }
+      for (int k = threadIdx.x; k <= gm; k += blockDim.x)  // no left leak from the first shell
+        gd[t * (gm + 1) + k] = (int16_t)count_le(a, t == 1 && ix == 1 ? 0 : n, (double)k / (double)gm);
     }
   }
+  if (A.fp64 && A.T.fine) {
+    const int fm = A.T.fine_m;
+    short2* fd = A.T.fine + (size_t)(ic - 1) * kFineTables * fm;
+    if (nlump > 0) {
+      for (int t = 0; t < 4; ++t) {
+        const CdfEntry* a = t == 0 ? cdop : (t == 1 ? cleft : (t == 2 ? cright : cscat));
+        const int n = t == 1 && ix == 1 ? 0 : (t == 3 ? ng - nlump : nlump);
+        for (int k = threadIdx.x; k < fm; k += blockDim.x)  // k / fm is exact: fm is a power of two
+          fd[t * fm + k] = make_short2((short)count_le(a, n, (double)k / (double)fm),
+                                       (short)count_le(a, n, (double)(k + 1) / (double)fm));
+      }
+    }
+    // the emission thresholds against (k / fine_m) capgrey, rounded as a draw's
+    // product by capgrey is
+    const int n = emit_last_group(A.nep, A.nepg, ng) - 1;
+    const double cg = A.capgrey[ic - 1];
+    const int one = emit_only_group(A.nep, A.nepg, ng, cg != cg);
+    for (int k = threadIdx.x; k < fm; k += blockDim.x) {
+      int r[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const double v = ((double)(k + j) / (double)fm) * cg;
+        int lo = 0, hi = n;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (ecum[mid] > v) hi = mid;
+          else lo = mid + 1;
+        }
+        r[j] = one ? one - 1 : lo;
+      }
+      fd[4 * fm + k] = make_short2((short)r[0], (short)r[1]);
+    }
+  }
+}
+
+// TrnCell records of the FP64 loop, one thread per cell, after cell_tables_kernel.
+__global__ void trn_cell_kernel(const TabArgs A0, int nc, TrnCell* __restrict__ out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= nc) return;
+  int ix;
+  const TabArgs A = tab_view(A0, c, &ix);
+  const double* X = A.xarr;
+  const double* sc = A.T.scal + (size_t)SCAL_N * (ix - 1);
+  TrnCell r;
+  r.xa = X[ix - 1];
+  r.xb = X[ix];
+  r.vxa = A.vxarr[ix - 1];
+  r.vxb = A.vxarr[ix];
+  r.dist = r.xb - r.xa;
+  r.sig = A.sig[ix - 1];
+  r.divv = A.divv[ix - 1];
+  r.capgrey = A.capgrey[ix - 1];
+  r.x0 = X[0];
+  r.far = sc[SCAL_FAR];
+  r.dvdr = sc[SCAL_DVDR];
+  r.vhelp = r.vxa - r.dvdr * r.xa;
+  r.dopc = 3.0 * pc_c / r.divv;
+  r.sigl = ix > 1 ? A.sig[ix - 2] : 0.0;
+  r.dxl = ix > 1 ? X[ix - 1] - X[ix - 2] : 0.0;
+  r.divvl = ix > 1 ? A.divv[ix - 2] : 0.0;
+  r.sigr = ix < A.nx ? A.sig[ix] : 0.0;
+  r.dxr = ix < A.nx ? X[ix + 1] - X[ix] : 0.0;
+  r.divvr = ix < A.nx ? A.divv[ix] : 0.0;
+  r.xa3 = cube(r.xa);
+  r.xb3 = cube(r.xb);
+  r.nlump = A.T.nlump[ix - 1];
+  r.pad = 0;
+  const double* OL = A.opaclump + (size_t)11 * (ix - 1);
+  const double2 lo = ddmc_rates(OL[0], OL[1], sc[SCAL_EMITLUMP], sc[SCAL_CAPLUMP], sc[SCAL_DOPLUMP], &r.denom);
+  r.pdop = lo.x;
+  r.pleft = lo.y;
+  r.pleak = lo.x + (OL[0] * r.denom + OL[1] * r.denom);
+  out[c] = r;
+}
+
+// CellTables::rates, one thread per (cell, group): the branch rates that
+// diffusion11.f90:154-278 forms for every event, once per entry (two exp and
+// eight divisions), with the expressions in the reference's order.
+__global__ void __launch_bounds__(256) ddmc_rate_kernel(const TabArgs A0, int nc, double2* __restrict__ out) {
+  const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int ng = A0.ng;
+  if (k >= (size_t)nc * ng) return;
+  const int c = (int)(k / ng), ig = (int)(k - (size_t)c * ng) + 1;
+  int ix;
+  const TabArgs A = tab_view(A0, c, &ix);
+  const double* X = A.xarr;
+  const float* cap = A.cap + (size_t)(ix - 1) * ng + (ig - 1);
+  const double Xa = X[ix - 1], Xb = X[ix], dist = Xb - Xa;
+  const double sigc = A.sig[ix - 1], capc = (double)cap[0];
+  double2 lo, hi = make_double2(0.0, 0.0);
+  if ((sigc + capc) * dist < A.tauddmc) {
+    lo = make_double2(__hiloint2double(kRateImcHi, 0), 0.0);
+  } else if (capc * dist >= A.taulump && A.T.nlump[ix - 1] > 0) {
+    lo = make_double2(__hiloint2double(kRateLumpedHi, 0), 0.0);
+  } else {
+    const double* sc = A.T.scal + (size_t)SCAL_N * (ix - 1);
+    const double tinv = A.tempinv[ix - 1], divv = A.divv[ix - 1], dx3 = sc[SCAL_DX3];
+    const double emitlump = specint0(tinv, A.wlinv, ig) * sc[SCAL_CAPGREYINV] * capc;
+    const double spec_ig = A.T.specarr[(size_t)(ix - 1) * ng + ig - 1];
+    double doplump;
+    if (ig != ng && divv >= 0.0) {
+      doplump = dopspeccalc(tinv, A.wlinv, ig) * divv / (spec_ig * 3.0 * pc_c);
+    } else if (ig != 1 && divv < 0.0) {
+      doplump = -1.0 * dopspeccalc(tinv, A.wlinv, ig - 1) * divv / (spec_ig * 3.0 * pc_c);
+    } else {
+      doplump = 0.0;
+    }
+    double o1 = 0.0, o2;
+    if (ix > 1) {
+      const double capl = (double)cap[-ng], sigl = A.sig[ix - 2];
+      const double dxl = Xa - X[ix - 2];
+      if ((capl + sigl) * dxl < A.tauddmc) {
+        const double mfphelp = (capc + sigc) * dist;
+        const double ppl = 4.0 / (3.0 * mfphelp + 6.0 * pc_dext);
+        o1 = 1.5 * ppl * sq(Xa) / dx3;
+      } else {
+        const double mfphelp = (sigc + capc) * dist + (sigl + capl) * dxl;
+        o1 = 2.0 * sq(Xa) / (mfphelp * dx3);
+      }
+    }
+    bool lhelp = true;
+    double capl = 0.0, sigl = 0.0, dxl = 0.0;
+    if (ix != A.nx) {
+      capl = (double)cap[ng];
+      sigl = A.sig[ix];
+      dxl = X[ix + 1] - Xb;
+      lhelp = (capl + sigl) * dxl < A.tauddmc;
+    }
+    if (lhelp) {
+      const double mfphelp = (capc + sigc) * dist;
+      const double ppr = 4.0 / (3.0 * mfphelp + 6.0 * pc_dext);
+      o2 = 1.5 * ppr * sq(Xb) / dx3;
+    } else {
+      const double mfphelp = (sigc + capc) * dist + (sigl + capl) * dxl;
+      o2 = 2.0 * sq(Xb) / (mfphelp * dx3);
+    }
+    double denom;
+    const double2 d = ddmc_rates(o1, o2, emitlump, capc, doplump, &denom);
+    lo = make_double2(denom, d.x);
+    hi = make_double2(d.y, d.x + (o1 * denom + o2 * denom));
+  }
+  out[2 * k] = lo;
+  out[2 * k + 1] = hi;
 }
 
 }  // namespace
@@ -623,6 +822,16 @@ int launch_emitprob(slg_ctx* ctx, const double* tempinv, const float* cap, const
   return cuda_check(ctx, cudaGetLastError(), "emission_probability launch");
 }
 
+namespace {
+void launch_tables(cudaStream_t st, int nx, const TabArgs& A) {
+  cell_tables_kernel<<<nx, GB, 0, st>>>(A);
+  if (!A.fp64) return;
+  trn_cell_kernel<<<(nx + 127) / 128, 128, 0, st>>>(A, nx, A.T.cell);
+  const size_t n = (size_t)nx * A.ng;
+  ddmc_rate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A, nx, A.T.rates);
+}
+}  // namespace
+
 int build_cell_tables(slg_ctx* ctx, const slg_transport_in* in) {
   const int nx = ctx->nx, ng = ctx->ng;
   const size_t n = (size_t)nx * ng;
@@ -630,18 +839,22 @@ int build_cell_tables(slg_ctx* ctx, const slg_transport_in* in) {
   if (T.nx != nx || T.ng != ng) {
     T.specarr = (double*)scratch(ctx, 12, sizeof(double) * n);
     T.glumps = (int16_t*)scratch(ctx, 13, sizeof(int16_t) * n);
-    T.cdf_dop = (double*)scratch(ctx, 14, sizeof(double) * n);
-    T.cdf_left = (double*)scratch(ctx, 15, sizeof(double) * n);
-    T.cdf_right = (double*)scratch(ctx, 16, sizeof(double) * n);
-    T.cdf_scat = (double*)scratch(ctx, 17, sizeof(double) * n);
+    T.cdf_dop = (CdfEntry*)scratch(ctx, 14, sizeof(CdfEntry) * n);
+    T.cdf_left = (CdfEntry*)scratch(ctx, 15, sizeof(CdfEntry) * n);
+    T.cdf_right = (CdfEntry*)scratch(ctx, 16, sizeof(CdfEntry) * n);
+    T.cdf_scat = (CdfEntry*)scratch(ctx, 17, sizeof(CdfEntry) * n);
     T.emitcum = (double*)scratch(ctx, 18, sizeof(double) * n);
     T.nlump = (int32_t*)scratch(ctx, 19, sizeof(int32_t) * nx);
     T.scal = (double*)scratch(ctx, 20, sizeof(double) * SCAL_N * nx);
     // guide entries are int16 positions
     T.guide_m = guide_size(ng);
     T.guide = ng < 32768 ? (int16_t*)scratch(ctx, 72, sizeof(int16_t) * 4 * (T.guide_m + 1) * (size_t)nx) : nullptr;
+    T.rates = (double2*)scratch(ctx, 91, sizeof(double2) * 2 * n);
+    T.cell = (TrnCell*)scratch(ctx, 92, sizeof(TrnCell) * (size_t)nx);
+    T.fine_m = fine_size(ng);
+    T.fine = ng < 32768 ? (short2*)scratch(ctx, 93, sizeof(short2) * kFineTables * T.fine_m * (size_t)nx) : nullptr;
     if (!T.specarr || !T.glumps || !T.cdf_dop || !T.cdf_left || !T.cdf_right || !T.cdf_scat ||
-        !T.emitcum || !T.nlump || !T.scal || (ng < 32768 && !T.guide)) {
+        !T.emitcum || !T.nlump || !T.scal || !T.rates || !T.cell || (ng < 32768 && (!T.guide || !T.fine))) {
       T.nx = T.ng = 0;
       return SLG_ERR_OOM;
     }
@@ -655,7 +868,8 @@ int build_cell_tables(slg_ctx* ctx, const slg_transport_in* in) {
   A.emitprob = in->emitprob; A.cap = in->cap; A.tauddmc = in->tauddmc; A.taulump = in->taulump;
   A.T = T;
   A.cellmap = ctx->nmodel > 1 ? ctx->d_cellmap : nullptr;
-  cell_tables_kernel<<<nx, GB, 0, ctx->stream>>>(A);
+  A.fp64 = in->precision == 0;  // the mixed loop has its own rates and emission CDF
+  launch_tables(ctx->stream, nx, A);
   return cuda_check(ctx, cudaGetLastError(), "cell tables launch");
 }
 
@@ -673,7 +887,7 @@ int launch_cell_tables_raw(cudaStream_t st, int nx, int ng, int nep, int nepg, c
   A.tempinv = in->tempinv; A.sig = in->sig; A.capgrey = in->capgrey; A.opaclump = in->opaclump;
   A.emitprob = in->emitprob; A.cap = in->cap; A.tauddmc = in->tauddmc; A.taulump = in->taulump;
   A.T = T;
-  cell_tables_kernel<<<nx, GB, 0, st>>>(A);
+  launch_tables(st, nx, A);
   return cudaGetLastError() == cudaSuccess ? SLG_OK : SLG_ERR_CUDA;
 }
 }  // namespace slg

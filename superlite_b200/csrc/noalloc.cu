@@ -43,7 +43,11 @@ constexpr size_t kNlumpBytes = align256(sizeof(int32_t) * kMaxCells);
 constexpr size_t kScalBytes = align256(sizeof(double) * slg::SCAL_N * kMaxCells);
 constexpr size_t kTabBytes = align256(sizeof(double) * kMaxCellGroups);
 constexpr size_t kGlumpBytes = align256(sizeof(int16_t) * kMaxCellGroups);
-constexpr size_t kScratchBytes = kAccBytes + kNlumpBytes + kScalBytes + 6 * kTabBytes + kGlumpBytes;
+constexpr size_t kCdfBytes = align256(sizeof(slg::CdfEntry) * kMaxCellGroups);
+constexpr size_t kCellBytes = align256(sizeof(slg::TrnCell) * kMaxCells);
+constexpr size_t kRateBytes = align256(2 * sizeof(double2) * kMaxCellGroups);
+constexpr size_t kScratchBytes =
+    kAccBytes + kNlumpBytes + kScalBytes + 2 * kTabBytes + 4 * kCdfBytes + kGlumpBytes + kCellBytes + kRateBytes;
 
 static __device__ __align__(256) unsigned char g_static_scratch[kScratchBytes];
 
@@ -94,18 +98,19 @@ extern "C" int slg_particle_advance_static(const slg_grid_dev* grid, const slg_t
   p += kNlumpBytes;
   T.scal = (double*)p;
   p += kScalBytes;
-  double* tabs[6];
-  for (int k = 0; k < 6; ++k) {
-    tabs[k] = (double*)p;
-    p += kTabBytes;
+  T.specarr = (double*)p;
+  p += kTabBytes;
+  T.emitcum = (double*)p;
+  p += kTabBytes;
+  for (CdfEntry** t : {&T.cdf_dop, &T.cdf_left, &T.cdf_right, &T.cdf_scat}) {
+    *t = (CdfEntry*)p;
+    p += kCdfBytes;
   }
-  T.specarr = tabs[0];
-  T.cdf_dop = tabs[1];
-  T.cdf_left = tabs[2];
-  T.cdf_right = tabs[3];
-  T.cdf_scat = tabs[4];
-  T.emitcum = tabs[5];
   T.glumps = (int16_t*)p;
+  p += kGlumpBytes;
+  T.cell = (TrnCell*)p;
+  p += kCellBytes;
+  T.rates = (double2*)p;
   T.nx = (int)nx;
   T.ng = (int)ng;
   const int nep = (int)lround(std::sqrt((double)ng));          // gridmod.f:121

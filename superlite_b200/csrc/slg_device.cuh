@@ -233,6 +233,14 @@ __device__ inline double u52_to_unit(uint32_t w0, uint32_t w1) {
   return ((double)m + 0.5) * 0x1p-52;
 }
 
+// (m + 1/2) 2^-52 of the 52-bit integer m made of two words: 1 + m 2^-52 (m as
+// the mantissa under the exponent of 1) minus 1 - 2^-53, exact (the result has
+// at most 53 bits and both operands lie in [1/2, 2)).  The same value as
+// u52_to_unit without an integer conversion.
+__device__ inline double u52_from_bits(uint32_t w0, uint32_t w1) {
+  return __hiloint2double((int)(0x3ff00000u | (w0 >> 12)), (int)((w0 << 20) | (w1 >> 12))) - (1.0 - 0x1p-53);
+}
+
 // Per-particle stream: draw k uses counter (k/2, pid, stream), words (0,1) for
 // even k and (2,3) for odd k; the odd half is kept for the next draw.
 struct PhiloxStream {
@@ -256,6 +264,48 @@ struct PhiloxStream {
     ++k;
     return r;
   }
+};
+
+// The same stream for the FP64 event loop, as a queue of up to three draws.
+// begin_event(), called where the warp's lanes are converged, makes one block
+// for every lane that holds fewer than two; a third draw of an event makes one
+// more block in place for the lanes that ran out.  (With a block made wherever
+// a lane's half block ran out, lanes out of step ran the ten rounds at every
+// draw site.)  k0, k1 are the key; pid the particle; nb the next block.
+struct PhiloxEventStream {
+  uint32_t nb, avail;
+  uint32_t q[6];
+  __device__ inline void init() { nb = 0; avail = 0; }
+  __device__ inline void begin_event(uint32_t k0, uint32_t k1, uint64_t pid, uint32_t stream) {
+    if (avail >= 2u) return;
+    const u32x4 o = philox4x32_10(u32x4{nb, (uint32_t)pid, (uint32_t)(pid >> 32), stream}, k0, k1);
+    ++nb;
+    if (avail == 0u) {
+      q[0] = o.a; q[1] = o.b; q[2] = o.c; q[3] = o.d;
+    } else {
+      q[2] = o.a; q[3] = o.b; q[4] = o.c; q[5] = o.d;
+    }
+    avail += 2u;
+  }
+  __device__ inline double draw(uint32_t k0, uint32_t k1, uint64_t pid, uint32_t stream) {
+    if (avail == 0u) {
+      const u32x4 o = philox4x32_10_call(nb, (uint32_t)pid, (uint32_t)(pid >> 32), stream, k0, k1);
+      ++nb;
+      q[0] = o.a; q[1] = o.b; q[2] = o.c; q[3] = o.d;
+      avail = 2u;
+    }
+    const double r = u52_from_bits(q[0], q[1]);
+    q[0] = q[2]; q[1] = q[3]; q[2] = q[4]; q[3] = q[5];
+    --avail;
+    return r;
+  }
+};
+// One particle's draws: the queue with the particle's key and number bound.
+struct EventDraws {
+  PhiloxEventStream& s;
+  uint32_t k0, k1, stream;
+  uint64_t pid;
+  __device__ inline double draw() { return s.draw(k0, k1, pid, stream); }
 };
 
 __device__ inline uint64_t fnv_mix(uint64_t h, int32_t v) {

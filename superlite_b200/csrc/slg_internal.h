@@ -15,22 +15,71 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
+// High words of the sentinels in CellTables::rates (quiet NaNs with payloads
+// that arithmetic does not produce): the group is IMC in this shell, or one of
+// its lumped groups (whose values are the record's).
+constexpr int kRateImcHi = 0x7ff8dd01, kRateLumpedHi = 0x7ff8dd02;
+
+// Per-cell record of the FP64 particle loop: what an event reads about its
+// shell apart from per-group values, in two 128-byte lines instead of a dozen
+// arrays; quotients and powers of the shell alone are formed once here, by the
+// event's expressions.
+struct alignas(256) TrnCell {
+  double xa, xb, vxa, vxb;       // shell edges and edge velocities
+  double dist, sig, divv, capgrey;
+  double denom, pdop, pleft, pleak;  // the lumped groups' entry of CellTables::rates
+  double x0;                     // the model's inner edge
+  double far, dvdr, vhelp;       // vhelp = vxa - dvdr xa
+  double dopc;                   // 3 c / divv
+  double sigl, sigr, dxl, dxr;   // neighbours (0 at the model's ends)
+  double divvl, divvr;
+  double xa3, xb3;               // cubed edges
+  int nlump, pad;
+};
+static_assert(sizeof(TrnCell) == 256, "TrnCell is two 128-byte lines");
+
+// Entry of a resolved-group running sum: the sum, the group that its position
+// resolves to, and in bit 16 whether that group is lumped, in bit 17 whether
+// it is IMC, in the shell where the particle continues (for a Doppler shift:
+// of the group it shifts to).
+struct __align__(16) CdfEntry {
+  double sum;
+  int info, pad;
+};
+constexpr int kInfoLumped = 1 << 16, kInfoImc = 1 << 17;
+
 // Device-resident per-cell tables used by the transport kernels (built by
 // build_cell_tables from grd_cap, grd_sig, grd_opaclump ...).  All tables
 // are cell-major: entry (ic-1)*ng + k.
 struct CellTables {
   double* specarr = nullptr;  // specintv mode-0 Planck weights
   int16_t* glumps = nullptr;  // diffusion11.f90:103-124 ordering (1-based groups)
-  double* cdf_dop = nullptr;  // Doppler resolved-group partial sums (:290-314)
-  double* cdf_left = nullptr; // left-leak resolved-group partial sums (:375-398)
-  double* cdf_right = nullptr;// right-leak partial sums (:447-460 at ix==nx, :489-511 else)
-  double* cdf_scat = nullptr; // effective-scatter partial sums over unlumped groups (:571-584)
-  double* emitcum = nullptr;  // emitgroup within-bin running sums (emitgroup.f:311-320)
+  // resolved-group running sums, each entry with the group it resolves to
+  CdfEntry* cdf_dop = nullptr;  // Doppler (:290-314)
+  CdfEntry* cdf_left = nullptr; // left leak (:375-398)
+  CdfEntry* cdf_right = nullptr;// right leak (:447-460 at ix==nx, :489-511 else)
+  CdfEntry* cdf_scat = nullptr; // effective scatter over unlumped groups (:571-584)
+  // emitgroup's thresholds (emitgroup.f:3-54): entry g-1 is the draw (times
+  // capgrey) from which group g+1 is emitted, see cell_tables_kernel
+  double* emitcum = nullptr;
+  // FP64 loop: DDMC branch probabilities per (cell, group), two double2 each
+  // {1/R, P(Doppler)}, {P(Doppler) + P(left), P(Doppler) + P(either leak)} with
+  // R the sum of the branch rates, or a sentinel in the first word (kRate*Hi);
+  // per-cell records
+  double2* rates = nullptr;
+  TrnCell* cell = nullptr;
+  // guide tables of the FP64 loop: fine_m entries per cell and table (four
+  // running sums and emitcum), entry k = the range {first, last} of answers for
+  // draws in [k, k+1)/fine_m.  fine_m is a power of two (r * fine_m is exact)
+  // near ng, so most ranges hold one or two entries and a search is one load
+  // of the range and one round of loads (null: search the whole table)
+  short2* fine = nullptr;
+  int fine_m = 0;
   // per-cell scalars: nlump, emitlump, caplump, doplump, capgreyinv, speclump
   int32_t* nlump = nullptr;
   double* scal = nullptr;     // 8 doubles per cell (see SCAL_*)
-  // guide tables of the four running sums above (dop, left, right, scat):
-  // per cell and table guide_m+1 entries, entry k = number of sums <= k/guide_m,
+  // guide tables of the mixed loop's searches, of the four running sums above
+  // (dop, left, right, scat): per cell and table guide_m+1 entries, entry k = number of sums <= k/guide_m,
   // so a draw r in [k, k+1)/guide_m is searched only between entries k and k+1
   // (null: plain search over the whole table).  guide_m is a power of two
   // (so r * guide_m and k / guide_m are exact) near ng/4: a range of a few
@@ -43,6 +92,24 @@ struct CellTables {
   float *cdf32_dop = nullptr, *cdf32_left = nullptr, *cdf32_right = nullptr, *cdf32_scat = nullptr;
   int nx = 0, ng = 0;
 };
+// emitgroup's last reachable group, and its constant answer where it has one
+// (0: none): one emission bin, or a draw that is not a number (nan).
+__host__ __device__ inline int emit_last_group(int nep, int nepg, int ng) {
+  const long long n = nep == 1 ? nepg + 1 : (long long)nep * nepg;
+  return n < ng ? (int)n : ng;
+}
+__host__ __device__ inline int emit_only_group(int nep, int nepg, int ng, bool nan) {
+  if (nep == 1) return emit_last_group(nep, nepg, ng);
+  return nan ? (nepg < ng ? nepg : ng) : 0;
+}
+
+constexpr int kFineMax = 2048;
+inline int fine_size(int ng) {
+  int m = 16;
+  while (m < kFineMax && m < ng) m *= 2;
+  return m;
+}
+constexpr int kFineTables = 5;  // dop, left, right, scat, emitcum
 constexpr int kGuideMax = 256;
 inline int guide_size(int ng) {
   int m = 16;
@@ -130,7 +197,7 @@ struct slg_ctx {
   double* d_amass = nullptr;  // element masses [amu] of the differentiable opacity
   int amass_n = 0;
   // derived per-call scratch
-  slg::DevBuf scratch[96];
+  slg::DevBuf scratch[128];
   slg::CellTables tables;
   slg::TransportAcc* d_acc = nullptr;
   slg::TransportAcc* h_acc = nullptr;  // pinned
@@ -138,9 +205,10 @@ struct slg_ctx {
   uint64_t* trace_hash = nullptr;
   int32_t* trace_nstep = nullptr;
   // transport kernel variants until slg_autotune_transport or
-  // slg_set_transport_variant choose: the ones measured fastest on whole
-  // steps of the batched 128-model workload at full particle budgets
-  int trn_variant = 2;  // FP64 transport kernel variant (see launch_transport_variant)
+  // slg_set_transport_variant choose: the ones measured fastest.  FP64 (-1):
+  // variant 0 for one model, 1 for several (launch_transport_variant); mixed:
+  // whole steps of the batched 128-model workload at full particle budgets
+  int trn_variant = -1;
   int mix_variant = 3;  // mixed-precision variant (see launch_transport_mixed)
   // transport_out of a queued slg_dev_particle_advance, completed by slg_sync
   slg_transport_out* pending_out = nullptr;

@@ -43,10 +43,23 @@ __device__ inline void store_flux_packet(slg_packet* p, double mu, double e, dou
   reinterpret_cast<double2*>(p)[3] = make_double2(e0, wl);
 }
 
+// Bound by instruction latency and issue: a history is one dependent chain of
+// events, and a launch of few histories per lane lasts as long as its longest
+// one.  What an event needs of its shell and group is therefore read from
+// tables made once per launch instead of formed per event (grid.cu): the DDMC
+// branch probabilities (two exp and eight divisions of an unlumped event), the
+// shell's record, and guide ranges that leave one or two entries to compare;
+// a resolved-group entry also says what the particle's next event would look
+// up.  Measured on B200, per-event against tables (same event sequences): pure
+// lumped DDMC, 256 shells x 2000 groups, 4e6 particles 745 -> 534 ms, 55 -> 32
+// warp instructions per particle-step; 64 models of 100 groups 3.47 -> 1.80 s;
+// 64 shells x 100 groups, 1e6 particles at 6 d 75 -> 48 ms.
+//
 // MINB = minimum resident blocks per SM requested from the register
-// allocator: 1 -> up to 255 registers (the compiler settles on 128),
-// 5 -> 96, 6 -> 80, 8 -> 64 registers with some spilling.  The autotuner
-// (slg_autotune_transport) picks the fastest on the caller's workload.
+// allocator: 1 -> up to 255 registers (the compiler settles on 124, 134 with
+// MODELS), 5 -> 96, 6 -> 80, 8 -> 64 registers with some spilling.  The
+// autotuner (slg_autotune_transport) picks the fastest on the caller's
+// workload; launch_transport_variant says which runs without it.
 // MODELS: the slots belong to several independent models (slg_set_models);
 // each particle finds its model once, draws from its model's random key with
 // the model-local slot as counter (as the model would alone), and tallies
@@ -64,11 +77,15 @@ __global__ void __launch_bounds__(TRN_BLOCK, MINB) particle_advance_kernel(const
   // the particle ends, so few registers carry them through the loop
   double evelo = 0.0;
   unsigned nd_p = 0, nsw_p = 0;
+  unsigned long long nd8 = 0;
   // current particle
   long long ip = -1;
   bool have = false;
   Ptcl p;
-  PhiloxStream rng;
+  PhiloxEventStream queue;
+  // the random key and the model's first slot (one model: of the launch)
+  uint32_t key0 = (uint32_t)A.seed, key1 = (uint32_t)(A.seed >> 32);
+  long long poff = 0;
   // replays of a captured graph draw from counter word 3 = stream | replay << 2
   const uint32_t sw = A.epoch ? (uint32_t)(*A.epoch << 2) : 0u;
   int istep = 0;
@@ -106,8 +123,6 @@ __global__ void __launch_bounds__(TRN_BLOCK, MINB) particle_advance_kernel(const
             double x, y, z, mu, om, e, e0, wl;
             load_packet(A.prt + ip, x, y, z, mu, om, e, e0, wl);
             atomicAdd(&s_cnt[0], 1ull);
-            int m = 0;
-            long long poff = 0;
             if (MODELS) {  // models own consecutive slot ranges
               int lo = 0, hi = A.nmodel - 1;
               while (lo < hi) {
@@ -115,15 +130,17 @@ __global__ void __launch_bounds__(TRN_BLOCK, MINB) particle_advance_kernel(const
                 if (__ldg(&A.models[mid].poff) <= ip) lo = mid;
                 else hi = mid - 1;
               }
-              m = lo;
-              poff = __ldg(&A.models[m].poff);
-              vnx = __ldg(&A.models[m].nx);
-              vco = __ldg(&A.models[m].co);
-              vxo = __ldg(&A.models[m].xo);
+              poff = __ldg(&A.models[lo].poff);
+              vnx = __ldg(&A.models[lo].nx);
+              vco = __ldg(&A.models[lo].co);
+              vxo = __ldg(&A.models[lo].xo);
+              const unsigned long long key = A.seed + (unsigned long long)lo * kModelSeedStride;
+              key0 = (uint32_t)key;
+              key1 = (uint32_t)(key >> 32);
             }
             const double* X = A.xarr + vxo;
             const double* VX = A.vxarr + vxo;
-            p.x = x; p.mu = mu; p.e = e; p.e0 = e0; p.wl = wl; p.dist = 0.0;
+            p.x = x; p.mu = mu; p.e = e; p.e0 = e0; p.wl = wl;
             p.ix = binsrch(x, X, vnx + 1, false);
             p.ig = binsrch(wl, A.wl, A.ng + 1, false);
             if (p.ix < 1 || p.ig < 1) {  // NaN position or wavelength: library code 1002
@@ -148,7 +165,8 @@ __global__ void __launch_bounds__(TRN_BLOCK, MINB) particle_advance_kernel(const
             istep = 0;
             nd_p = 0;
             nsw_p = 0;
-            rng.init(A.seed + (unsigned long long)m * kModelSeedStride, (uint64_t)(ip - poff), sw);
+            p.lumped = 0;
+            queue.init();
             if (TRACE) h = 1469598103934665603ull;
             have = !bad;
           }
@@ -159,6 +177,8 @@ __global__ void __launch_bounds__(TRN_BLOCK, MINB) particle_advance_kernel(const
     if (!have) continue;
     // ---- one event, particle_advance.f90:204-268
     istep++;
+    EventDraws rng{queue, key0, key1, sw, (uint64_t)(ip - poff)};
+    queue.begin_event(key0, key1, rng.pid, sw);
     const MView v{vnx, vco, vxo};
     const int icold = vco + p.ix, igold = p.ig;  // cell over all models, 1-based
     double eraddens, jrad, eamp = 0.0;
@@ -167,6 +187,7 @@ __global__ void __launch_bounds__(TRN_BLOCK, MINB) particle_advance_kernel(const
       transport11_dev(A, v, p, rng, eraddens, eamp, jrad, evelo, ierr);
       if (p.itype != 1) {
         nsw_p++;
+        p.lumped = 0;
         if (A.dogrdtally) atomicAdd(&A.methodswap[icold - 1], 1);
       }
       if (!A.noampfact && eamp != 0.0) atomicAdd(&A.eamp[icold - 1], eamp);
@@ -178,12 +199,9 @@ __global__ void __launch_bounds__(TRN_BLOCK, MINB) particle_advance_kernel(const
         if (A.dogrdtally) atomicAdd(&A.methodswap[icold - 1], 1);
       }
     }
-    {
-      // ndist histogram: one shared-memory add per distinct bin in the warp
-      const int di = 9 + (p.idist > -3 ? p.idist : -3) + 3;
-      const unsigned grp = __match_any_sync(__activemask(), di);
-      if (lane == __ffs(grp) - 1) atomicAdd(&s_cnt[di], (unsigned long long)__popc(grp));
-    }
+    // ndist histogram: eight-bit counts of the particle's last events
+    nd8 += 1ull << (8 * ndist_slot(p.idist));
+    if ((istep & 127) == 0) ndist_flush(s_cnt + 9, nd8);
     if (icold != t_ic) {
       if (t_ic > 0 && t_acc != 0.0) atomicAdd(&A.tally[t_ic - 1], t_acc);
       t_ic = icold;
@@ -205,7 +223,8 @@ __global__ void __launch_bounds__(TRN_BLOCK, MINB) particle_advance_kernel(const
       h = fnv_mix(h, p.stat);
     }
     if (p.itype == 1 && p.stat == 0) {
-      if (p.x > A.xarr[vxo + p.ix] || p.x < A.xarr[vxo + p.ix - 1] || p.x != p.x) {
+      const TrnCell& R = A.T.cell[vco + p.ix - 1];
+      if (p.x > R.xb || p.x < R.xa || p.x != p.x) {
         if (ierr == 0) ierr = -99;
       }
     }
@@ -220,6 +239,7 @@ __global__ void __launch_bounds__(TRN_BLOCK, MINB) particle_advance_kernel(const
     }
     if (p.stat != 0) {
       // ---- particle end, particle_advance.f90:271-292
+      ndist_flush(s_cnt + 9, nd8);
       atomicMax(&s_cnt[5], (unsigned long long)istep);
       atomicAdd(&s_cnt[2], (unsigned long long)(istep - nd_p));
       atomicAdd(&s_cnt[3], (unsigned long long)nd_p);
@@ -355,8 +375,13 @@ int launch_mix_rate_tables(cudaStream_t st, int nc, const int4* cellmap, const T
 constexpr int kMixedVariants = 4;
 
 // Transport kernel variants (register budget / resident blocks), see MINB.
+// v < 0 (nobody chose): the one without spills for one model (variants 0 / 1 / 2
+// / 3: 86 / 91 / 102 / 105 ms at 256 shells x 2000 groups, 4e5 particles; 48 /
+// 51 / 54 / 57 ms at 64 x 100, 1e6 particles), five blocks per SM for several,
+// whose kernel holds more state (2.04 / 1.80 / 2.11 / 2.42 s, 64 models).
 constexpr int kTransportVariants = 4;
 int launch_transport_variant(int v, bool trace, int num_sms, long long npart, cudaStream_t st, const TrnArgs& A) {
+  if (v < 0) v = A.nmodel > 1 ? 1 : 0;
   if (A.nmodel > 1) {  // several models: no per-event trace
     switch (v) {
       case 1: return launch_one<false, 5, true>(num_sms, npart, st, A);
@@ -427,14 +452,14 @@ __global__ void mix_cell_kernel(int nc, const int4* __restrict__ cellmap, const 
 }
 
 // FP32 copies of the four running-sum tables (n entries each).
-__global__ void cdf32_kernel(size_t n, const double* __restrict__ a0, const double* __restrict__ a1,
-                             const double* __restrict__ a2, const double* __restrict__ a3, float* __restrict__ b0,
+__global__ void cdf32_kernel(size_t n, const CdfEntry* __restrict__ a0, const CdfEntry* __restrict__ a1,
+                             const CdfEntry* __restrict__ a2, const CdfEntry* __restrict__ a3, float* __restrict__ b0,
                              float* __restrict__ b1, float* __restrict__ b2, float* __restrict__ b3) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    b0[i] = (float)a0[i];
-    b1[i] = (float)a1[i];
-    b2[i] = (float)a2[i];
-    b3[i] = (float)a3[i];
+    b0[i] = (float)a0[i].sum;
+    b1[i] = (float)a1[i].sum;
+    b2[i] = (float)a2[i].sum;
+    b3[i] = (float)a3[i].sum;
   }
 }
 
