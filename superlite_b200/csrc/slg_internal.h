@@ -205,11 +205,10 @@ struct slg_ctx {
   uint64_t* trace_hash = nullptr;
   int32_t* trace_nstep = nullptr;
   // transport kernel variants until slg_autotune_transport or
-  // slg_set_transport_variant choose: the ones measured fastest.  FP64 (-1):
-  // variant 0 for one model, 1 for several (launch_transport_variant); mixed:
-  // whole steps of the batched 128-model workload at full particle budgets
+  // slg_set_transport_variant choose (-1: by the rules of
+  // launch_transport_variant and launch_transport_mixed)
   int trn_variant = -1;
-  int mix_variant = 3;  // mixed-precision variant (see launch_transport_mixed)
+  int mix_variant = -1;
   // transport_out of a queued slg_dev_particle_advance, completed by slg_sync
   slg_transport_out* pending_out = nullptr;
   // models (one for slg_set_grid): host descriptors, device copies, and the

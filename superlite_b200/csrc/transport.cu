@@ -371,7 +371,7 @@ int launch_one(int num_sms, long long npart, cudaStream_t st, const TrnArgs& A) 
 
 int launch_transport_mixed(int variant, int num_sms, long long npart, cudaStream_t st, const TrnArgs& A);
 int launch_mix_rate_tables(cudaStream_t st, int nc, const int4* cellmap, const TrnArgs& A, float4* mrate,
-                           float* emit32, int16_t* eguide);
+                           float* emit32, short2* eguide);
 constexpr int kMixedVariants = 4;
 
 // Transport kernel variants (register budget / resident blocks), see MINB.
@@ -494,7 +494,7 @@ int build_mix_cells(slg_ctx* ctx, const slg_transport_in* in, TrnArgs& A) {
   // per (cell, group) DDMC rates and per-cell emission CDFs (scratch slots 81-83)
   auto* mrate = (float4*)scratch(ctx, 81, sizeof(float4) * n);
   auto* emit32 = (float*)scratch(ctx, 82, sizeof(float) * n);
-  auto* eguide = (int16_t*)scratch(ctx, 83, sizeof(int16_t) * (size_t)nc * (T.guide_m + 1));
+  auto* eguide = (short2*)scratch(ctx, 83, sizeof(short2) * (size_t)nc * T.fine_m);
   if (!mrate || !emit32 || !eguide) return SLG_ERR_OOM;
   A.mrate = mrate;
   A.emit32 = emit32;

@@ -40,11 +40,11 @@ struct TrnArgs {
   // mixed-precision kernel: per (cell, group) DDMC branch rates of an unlumped
   // group, {doplump, opacleak(1), opacleak(2), (1 - emitlump) caplump}, with
   // sentinels and neighbour flags (see mix_rate_kernel); per cell the emission
-  // CDF over groups divided by capgrey, and its guide table (T.guide_m + 1
-  // entries per cell)
+  // CDF over groups divided by capgrey, and its guide table (T.fine_m ranges per
+  // cell)
   const float4* mrate = nullptr;
   const float* emit32 = nullptr;
-  const int16_t* eguide = nullptr;
+  const short2* eguide = nullptr;
 };
 
 struct Ptcl {
