@@ -51,7 +51,7 @@ void* scratch(slg_ctx* ctx, int slot, size_t bytes) {
   return b.p;
 }
 
-int opacity_flags(slg_ctx* ctx, int32_t* sanity, int32_t* binning);
+int opacity_flags(slg_ctx* ctx, int32_t* sanity);
 int sourcetally_error(slg_ctx* ctx, int* err);
 int finish_particle_advance_acc(const TransportAcc& a, slg_transport_out* out);
 void host_sourceenergy(int nx, const double* xarr, const double* radtemp, double L_bol, double* emit,
@@ -257,7 +257,7 @@ void slg_destroy(slg_ctx* ctx) {
   free_dev(ctx->d_gff); free_dev(ctx->d_acc);
   free_dev(ctx->d_totals); free_dev(ctx->d_epoch); free_dev(ctx->d_models); free_dev(ctx->d_cellmap);
   free_dev(ctx->d_eos_ni); free_dev(ctx->d_eos_e); free_dev(ctx->d_eos_q); free_dev(ctx->d_eos_g1);
-  free_dev(ctx->d_amass); free_dev(ctx->d_lrow_of_slot); free_dev(ctx->d_slot_of_lrow);
+  free_dev(ctx->d_amass); free_dev(ctx->d_lrow_of_slot);
   if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
   if (ctx->h_acc) cudaFreeHost(ctx->h_acc);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -376,6 +376,7 @@ int slg_set_groups(slg_ctx* ctx, int32_t ng, const double* grp_wl) {
   ctx->nep = (int)lround(std::sqrt((double)ng));                 // gridmod.f:121
   ctx->nepg = (int)std::ceil(ng / (ctx->nep + 1.0));              // gridmod.f:122
   ctx->tables.nx = ctx->tables.ng = 0;
+  ctx->plan_edges = ctx->plan_bb = ctx->plan_bf = false;
   return SLG_OK;
 }
 
@@ -403,6 +404,7 @@ int slg_set_atomic_data(slg_ctx* ctx, int32_t nelem, int32_t nstage, const int32
       return set_error(ctx, SLG_ERR_ARG, "slg_set_atomic_data: line %lld has ion (%d,%d) outside the tables",
                        (long long)l, bb_xs[l].iz, bb_xs[l].ii);
   cudaSetDevice(ctx->device);
+  ctx->plan_bb = ctx->plan_bf = false;
   free_dev(ctx->d_ion_ni); free_dev(ctx->d_bb); free_dev(ctx->d_ph1); free_dev(ctx->d_ph2); free_dev(ctx->d_gff);
   ctx->d_ion_ni = nullptr; ctx->d_bb = nullptr; ctx->d_ph1 = ctx->d_ph2 = nullptr; ctx->d_gff = nullptr;
   int rc = cuda_check(ctx, cudaMalloc(&ctx->d_ion_ni, sizeof(int32_t) * nelem), "alloc ion_ni");
@@ -421,10 +423,11 @@ int slg_set_atomic_data(slg_ctx* ctx, int32_t nelem, int32_t nstage, const int32
     rc = cuda_check(ctx, cudaMalloc(&ctx->d_gff, sizeof(double) * 81 * 41), "alloc gff");
     if (!rc) rc = cuda_check(ctx, cudaMemcpy(ctx->d_gff, ff_gff, sizeof(double) * 81 * 41, cudaMemcpyHostToDevice), "gff");
   }
-  // the population rows the lines reference (the opacity adjoint accumulates
-  // d cap / d population for those rows only)
+  // the population rows the lines reference (the opacity plan orders a
+  // sub-group's lines by them)
   const int nslot = nelem * nstage;
-  std::vector<int16_t> row_of(nslot, (int16_t)-1), slot_of;
+  std::vector<int16_t> row_of(nslot, (int16_t)-1);
+  int nrow = 0;
   // the largest lower-level energy: the opacity kernels skip the range check
   // of their exp for a shell with hc/kT * chimax <= 700 (infinite when a
   // value is negative or NaN: every term is then checked)
@@ -436,25 +439,19 @@ int slg_set_atomic_data(slg_ctx* ctx, int32_t nelem, int32_t nstage, const int32
   for (int64_t l = 0; l < nline; ++l) {
     const int sl = (bb_xs[l].iz - 1) * nstage + (bb_xs[l].ii - 1);
     if (row_of[sl] < 0) {
-      row_of[sl] = (int16_t)slot_of.size();
-      slot_of.push_back((int16_t)sl);
+      row_of[sl] = (int16_t)nrow++;
     }
   }
-  free_dev(ctx->d_lrow_of_slot); free_dev(ctx->d_slot_of_lrow);
-  ctx->d_lrow_of_slot = ctx->d_slot_of_lrow = nullptr;
+  free_dev(ctx->d_lrow_of_slot);
+  ctx->d_lrow_of_slot = nullptr;
   if (!rc) rc = cuda_check(ctx, cudaMalloc(&ctx->d_lrow_of_slot, sizeof(int16_t) * nslot), "alloc row map");
   if (!rc) rc = cuda_check(ctx, cudaMemcpy(ctx->d_lrow_of_slot, row_of.data(), sizeof(int16_t) * nslot,
                                           cudaMemcpyHostToDevice), "row map");
-  if (!rc && !slot_of.empty()) {
-    rc = cuda_check(ctx, cudaMalloc(&ctx->d_slot_of_lrow, sizeof(int16_t) * slot_of.size()), "alloc slot map");
-    if (!rc) rc = cuda_check(ctx, cudaMemcpy(ctx->d_slot_of_lrow, slot_of.data(), sizeof(int16_t) * slot_of.size(),
-                                            cudaMemcpyHostToDevice), "slot map");
-  }
   if (rc) return rc;
   ctx->nelem = nelem;
   ctx->nstage = nstage;
   ctx->nline = nline;
-  ctx->nlrow = (int)slot_of.size();
+  ctx->nlrow = nrow;
   ctx->line_chimax = chimax;
   ctx->h_ion_ni.assign(ion_ni, ion_ni + nelem);
   return SLG_OK;
@@ -565,10 +562,8 @@ int slg_physical_opacity(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_fla
   if (cap64) down(ctx, cap64, dc64, nc * ng, &rc);
   rc = finish(ctx, rc);
   if (!rc) {
-    int32_t s = 0, b = 0;
-    rc = opacity_flags(ctx, &s, &b);
-    if (!rc && (b & 1)) rc = set_error(ctx, SLG_ERR_UNSORTED, "bb line list not sorted by wl0");
-    if (!rc && (b & 2)) rc = set_error(ctx, SLG_ERR_CUDA, "line binning: shared-memory staging timed out");
+    int32_t s = 0;
+    rc = opacity_flags(ctx, &s);
     if (sanity) *sanity = s;
   }
   return rc;

@@ -7,16 +7,16 @@
 // GAS/opacity_rossmean.f:17-21.
 //
 // Design (one B200):
-//  * bin_lines: lines (sorted by wl0) are binned to sub-groups by a
-//    warp-cooperative kernel: the sub-group edges are staged into shared memory
-//    with one TMA bulk copy (cp.async.bulk + mbarrier), each thread binary-
-//    searches its lines there, and a shared-memory histogram of lines per
-//    sub-group is flushed to global counts; a scan turns counts into ranges.
-//  * opacity_fwd: one warp per (group, 32 shells).  Every lane walks the
-//    lines of its group in file order (warp-uniform broadcast reads) and
-//    accumulates bb, then bf (ions in the reference's iz,ii order), then ff
-//    (elements in order) into one register, i.e. exactly the reference's
-//    per-(cell,sub-group) summation order.  Sub-groups are collapsed in
+//  * What depends on the line list, the bound-free fits and the group grid alone
+//    is laid out once after slg_set_groups / slg_set_atomic_data (opacity_plan):
+//    the sub-groups' line ranges, each line's 16-byte record with its
+//    sub-group's lines ordered by the population row they multiply, and the
+//    nonzero cross sections of every sub-group.
+//  * opac_cell: the shells' scalars, level populations and free-free sums.
+//  * opacity_fwd: one warp per (group, 32 FS shells).  Every lane walks the
+//    lines of its group (warp-uniform broadcast reads) and accumulates bb row
+//    by row, then bf (ions in the reference's iz,ii order), then ff (elements
+//    in order) into one register per shell.  Sub-groups are collapsed in
 //    registers, then cap and emissivity are written through a shared-memory
 //    tile so each shell's 8 groups leave as one 32-byte sector.
 //  * FP64 throughout, no FMA contraction (-fmad=false), so sums round like the
@@ -30,165 +30,34 @@ namespace slg {
 
 namespace {
 
-constexpr int OPAC_GT = 8;   // groups per block (one warp each)
-constexpr int OPAC_CT = 32;  // shells per block (one per lane)
-// forward: FS shells per lane (a block covers FS * OPAC_CT shells), 2 or 4
-// (opacity_fwd_kernel<FS>; launch_fwd picks it)
+constexpr int kMaxLineSubgroups = 18770;  // sub-groups that the line binning accepts
+constexpr int OPAC_CT = 32;  // lanes of a warp, each with one or more shells
 
-// ------------------------------------------------------------ TMA bulk helpers
-__device__ inline uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ inline void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ inline void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ inline void tma_bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-// Bounded wait on phase 0 of the barrier.  Returns false on time-out.
-__device__ inline bool mbar_wait(uint64_t* bar, uint32_t parity, long max_polls) {
-  for (long it = 0; it < max_polls; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (it > 64) __nanosleep(64);
+// ------------------------------------------------------------ line ranges
+// lstart[igs] (igs = 0..nedge+1) = first line whose sub-group pointer
+// (physical_opacity.f:117-125: igs = #{k : wlsub(k) <= wl0}) is at least igs;
+// the lines are sorted by wl0 (slg_set_atomic_data), so it is the first line
+// at or above edge igs-1.
+__global__ void line_range_kernel(const slg_bbxs* __restrict__ bb, int64_t nline, const double* __restrict__ wlsub,
+                                  int nedge, int* __restrict__ lstart) {
+  const int igs = blockIdx.x * blockDim.x + threadIdx.x;
+  if (igs > nedge + 1) return;
+  int64_t lo = 0, hi = igs == 0 ? 0 : nline;
+  if (igs > nedge) lo = nline;
+  const double edge = igs >= 1 && igs <= nedge ? wlsub[igs - 1] : 0.0;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if ((double)bb[mid].wl0 * pc_ang >= edge) hi = mid;
+    else lo = mid + 1;
   }
-  return false;
-}
-
-// ------------------------------------------------------------ line binning
-// counts[igs] (igs = 0..ngsub+1) = number of lines whose sub-group pointer is
-// igs (physical_opacity.f:117-125): igs = #{k : wlsub(k) <= wl0}.
-__global__ void __launch_bounds__(256) bin_lines_kernel(const slg_bbxs* __restrict__ bb, int64_t nline,
-                                                        const double* __restrict__ wlsub_pad,
-                                                        int nedge, int nedge_pad,
-                                                        unsigned int* __restrict__ counts,
-                                                        int* __restrict__ flags) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
-  double* edges = reinterpret_cast<double*>(smem + 16);
-  unsigned int* hist = reinterpret_cast<unsigned int*>(smem + 16 + sizeof(double) * nedge_pad);
-  const int nbins = nedge + 1;  // 0..ngsub+1
-  if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    mbar_expect_tx(bar, (uint32_t)(sizeof(double) * nedge_pad));
-    tma_bulk_g2s(edges, wlsub_pad, (uint32_t)(sizeof(double) * nedge_pad), bar);
-  }
-  for (int k = threadIdx.x; k < nbins; k += blockDim.x) hist[k] = 0u;
-  __syncthreads();
-  if (!mbar_wait(bar, 0, 1L << 24)) {
-    if (threadIdx.x == 0) atomicOr(flags + 1, 2);
-    // keep waiting (bounded) for the copy in flight before leaving
-    mbar_wait(bar, 0, 1L << 24);
-    return;
-  }
-  const int64_t per_block = (int64_t)blockDim.x * 8;
-  const int64_t l0 = (int64_t)blockIdx.x * per_block;
-  for (int it = 0; it < 8; ++it) {
-    const int64_t l = l0 + (int64_t)it * blockDim.x + threadIdx.x;
-    if (l >= nline) break;
-    const float w = bb[l].wl0;
-    if (l + 1 < nline && !(w <= bb[l + 1].wl0)) atomicOr(flags + 1, 1);
-    const double wl0 = (double)w * pc_ang;
-    // upper bound: number of edges <= wl0
-    int lo = 0, hi = nedge;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (edges[mid] <= wl0) lo = mid + 1;
-      else hi = mid;
-    }
-    atomicAdd(&hist[lo], 1u);
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < nbins; k += blockDim.x)
-    if (hist[k]) atomicAdd(&counts[k], hist[k]);
-}
-
-// exclusive scan of counts (n <= a few 1e4) in one block
-__global__ void __launch_bounds__(1024) scan_counts_kernel(const unsigned int* __restrict__ counts, int n,
-                                                           int* __restrict__ start) {
-  __shared__ int part[1024];
-  const int per = (n + blockDim.x - 1) / blockDim.x;
-  const int b = threadIdx.x * per;
-  int s = 0;
-  for (int k = b; k < b + per && k < n; ++k) s += (int)counts[k];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int t = 0; t < (int)blockDim.x; ++t) {
-      const int v = part[t];
-      part[t] = acc;
-      acc += v;
-    }
-  }
-  __syncthreads();
-  int acc = part[threadIdx.x];
-  for (int k = b; k < b + per && k < n; ++k) {
-    start[k] = acc;
-    acc += (int)counts[k];
-  }
-  if (threadIdx.x == blockDim.x - 1) start[n] = acc;
+  lstart[igs] = (int)lo;
 }
 
 // ------------------------------------------------------------ per-cell preparation
 // hckt (physical_opacity.f:81), gas_sig (:84-89), hlparr (:203), grndlev (:95-101,
-// :165-171) and the per-(cell,element) free-free Gaunt row indices (:226-231).
-__global__ void opac_cell_prep_kernel(int nc, int nelem, int nst, const int32_t* __restrict__ ion_ni,
-                                      const double* __restrict__ temp, const double* __restrict__ natom,
-                                      const double* __restrict__ nelec, const double* __restrict__ vol,
-                                      const double* __restrict__ mass, const double* __restrict__ oc,
-                                      const double* __restrict__ ginv, int nothmson,
-                                      double* __restrict__ hckt, double* __restrict__ gas_sig,
-                                      double* __restrict__ hlparr, double* __restrict__ grndlev,
-                                      int* __restrict__ ffigg, double* __restrict__ ffdgg) {
-  // one thread per (shell i, element iz = blockIdx.y + 1)
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nc) return;
-  const double h = pc_hc / (pc_kb * temp[i]);
-  if (blockIdx.y == 0) {
-    hckt[i] = h;
-    double s = 0.0;
-    if (!nothmson) {
-      s = cthomson * nelec[i] * natom[i] / vol[i];
-      if (mass[i] <= 0.0) s = 0.0;
-    }
-    gas_sig[i] = s;
-    hlparr[i] = sq(natom[i] / vol[i]) * nelec[i];
-  }
-  {
-    const int iz = blockIdx.y + 1;
-    const int lim = min(iz, ion_ni[iz - 1] - 1);
-    for (int ii = 1; ii <= nst; ++ii) {
-      const size_t k = (size_t)(iz - 1) * nst + (ii - 1);
-      double v = 0.0;
-      if (ii <= lim && mass[i] > 0.0) v = oc[k * nc + i] * ginv[k * nc + i];
-      grndlev[k * nc + i] = v;
-    }
-    const double gg = (double)(iz * iz) * pc_rydberg * h;
-    const double rgg = 5.0 * (log10(gg) + 4.0) + 1.0;
-    // max(floor(rgg), 1) and min(., ff_ngg - 1) as :228-230; a NaN (from a NaN
-    // temperature) takes the lower bound, so the table reads stay in bounds
-    int igg = !(rgg >= 1.0) ? 1 : (rgg >= (double)(FF_NGG - 1) ? FF_NGG - 1 : (int)floor(rgg));
-    ffigg[(size_t)(iz - 1) * nc + i] = rgg > (double)FF_NGG ? -igg : igg;  // sign: gff >= 1 clamp (:238)
-    ffdgg[(size_t)(iz - 1) * nc + i] = rgg - igg;
-  }
-}
-
+// :165-171), which ion slots (iz,ii) carry any population (active, zeroed by the
+// caller), and per (cell, element) the free-free Gaunt columns (:226-231).
+//
 // Free-free, summed over elements once per shell.  For fixed table columns
 // (igg, dgg) of each element, the reference's bilinear gff (physical_opacity.f:
 // 234-237) is linear in the row weights (1 - du, du):
@@ -202,46 +71,99 @@ __global__ void opac_cell_prep_kernel(int nc, int nelem, int nst, const int32_t*
 // z^2 fr_z (G[j, igg] - G[j, igg - 1]) over the same elements (d gff / d dgg
 // is linear in the row weights too), and ffclamp_all flags every clamped
 // element whatever its fr (d cap / d fr needs them all).
-// One thread per (shell, table row j).
-__global__ void ff_sum_kernel(int nc, int nelem, const double* __restrict__ natomfr, const int* __restrict__ ffigg,
-                              const double* __restrict__ ffdgg, const double* __restrict__ G,
-                              double* __restrict__ ffsum, double* __restrict__ ffdsum, unsigned* __restrict__ ffclamp,
-                              unsigned* __restrict__ ffclamp_all) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)nc * FF_NU) return;
-  const int i = (int)(t / FF_NU), j = (int)(t % FF_NU);
-  const double* nfr = natomfr + (size_t)(nelem + 1) * i;
-  double S = 0.0, D = 0.0;
-  unsigned clamp = 0, clamp_all = 0;
-  for (int iz = 1; iz <= nelem; ++iz) {
-    const double fr = nfr[iz];
-    const int igg = ffigg[(size_t)(iz - 1) * nc + i];
-    if (igg < 0) {
-      clamp_all |= 1u << (iz - 1);
-      if (fr != 0.0) clamp |= 1u << (iz - 1);
-      continue;
+//
+// A block takes CELLS shells: first the populations, shells fastest, then a warp
+// per shell: a lane per element finds its columns, the elements that enter the
+// sums are compacted into shared memory, and the lanes take the 81 table rows.
+// (As one thread per (shell, row) that walked all elements the sums alone took
+// 17-20 us whatever the grid, besides 9 us for the rest; now 15 us in all at 32 and
+// at 256 shells, 20 us at 4096.)
+constexpr int CELLS = 8;
+constexpr int kRun = 64;  // most shells of a warp: the population rows are padded to whole warps' shells
+__global__ void __launch_bounds__(CELLS * 32) opac_cell_kernel(
+    int nc, int nelem, int nst, const int32_t* __restrict__ ion_ni, const double* __restrict__ temp,
+    const double* __restrict__ natom, const double* __restrict__ nelec, const double* __restrict__ vol,
+    const double* __restrict__ mass, const double* __restrict__ oc, const double* __restrict__ ginv, int nothmson,
+    const double* __restrict__ natomfr, const double* __restrict__ G, double* __restrict__ hckt,
+    double* __restrict__ gas_sig, double* __restrict__ hlparr, int ld, double* __restrict__ grndlev,
+    double* __restrict__ ocp, int* __restrict__ active, int* __restrict__ ffigg, double* __restrict__ ffdgg, double* __restrict__ ffsum,
+    double* __restrict__ ffdsum, unsigned* __restrict__ ffclamp, unsigned* __restrict__ ffclamp_all) {
+  __shared__ double s_w[CELLS][32], s_dgg[CELLS][32];
+  __shared__ int s_igg[CELLS][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nslot = nelem * nst;
+  for (int t = threadIdx.x; t < nslot * CELLS; t += CELLS * 32) {  // a multiple of CELLS per slot
+    const int k = t / CELLS, i = blockIdx.x * CELLS + t % CELLS;
+    double o = 0.0, v = 0.0;
+    if (i < nc) {
+      const int iz = k / nst + 1, ii = k % nst + 1;
+      o = oc[(size_t)k * nc + i];
+      if (ii <= min(iz, ion_ni[iz - 1] - 1) && mass[i] > 0.0) v = o * ginv[(size_t)k * nc + i];
     }
-    if (fr == 0.0) continue;
-    const double dgg = ffdgg[(size_t)(iz - 1) * nc + i];
-    const double g0 = G[j + FF_NU * (igg - 1)], g1 = G[j + FF_NU * igg];
-    const double gz = (1.0 - dgg) * g0 + dgg * g1;
-    const double w = (double)(iz * iz) * fr;
-    S = S + w * gz;
-    D = D + w * (g1 - g0);
+    if (i < ld) {
+      grndlev[(size_t)k * ld + i] = v < 0.0 ? 0.0 : v;  // the reference skips lines with ocg <= 0
+      ocp[(size_t)k * ld + i] = o;
+    }
+    if (o != 0.0) active[k] = 1;
   }
-  ffsum[(size_t)i * FF_NU + j] = S;
-  ffdsum[(size_t)i * FF_NU + j] = D;
-  if (j == 0) {
-    ffclamp[i] = clamp;
-    ffclamp_all[i] = clamp_all;
+  const int i = blockIdx.x * CELLS + warp;
+  if (i >= nc) return;  // uniform over the warp
+  const double h = pc_hc / (pc_kb * temp[i]);
+  if (lane == 0) {
+    hckt[i] = h;
+    double s = 0.0;
+    if (!nothmson) {
+      s = cthomson * nelec[i] * natom[i] / vol[i];
+      if (mass[i] <= 0.0) s = 0.0;
+    }
+    gas_sig[i] = s;
+    hlparr[i] = sq(natom[i] / vol[i]) * nelec[i];
   }
-}
-
-// Which ion slots (iz,ii) carry any population: 1 if any cell has oc != 0.
-__global__ void ion_active_kernel(int nc, const double* __restrict__ oc, int* __restrict__ active) {
-  const int k = blockIdx.y;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x)
-    if (oc[(size_t)k * nc + i] != 0.0) { active[k] = 1; return; }
+  if (!G) return;
+  bool clamped = false, in_sum = false;
+  double fr = 0.0, dgg = 0.0;
+  int igg = 1;
+  if (lane < nelem) {
+    const int iz = lane + 1;
+    const double gg = (double)(iz * iz) * pc_rydberg * h;
+    const double rgg = 5.0 * (log10(gg) + 4.0) + 1.0;
+    // max(floor(rgg), 1) and min(., ff_ngg - 1) as :228-230; a NaN (from a NaN
+    // temperature) takes the lower bound, so the table reads stay in bounds
+    igg = !(rgg >= 1.0) ? 1 : (rgg >= (double)(FF_NGG - 1) ? FF_NGG - 1 : (int)floor(rgg));
+    dgg = rgg - igg;
+    clamped = rgg > (double)FF_NGG;
+    ffigg[(size_t)lane * nc + i] = clamped ? -igg : igg;  // sign: gff >= 1 clamp (:238)
+    ffdgg[(size_t)lane * nc + i] = dgg;
+    fr = natomfr[(size_t)(nelem + 1) * i + iz];
+    in_sum = fr != 0.0 && !clamped;
+  }
+  const unsigned m_sum = __ballot_sync(0xffffffffu, in_sum);
+  const unsigned m_all = __ballot_sync(0xffffffffu, clamped), m_fr = __ballot_sync(0xffffffffu, clamped && fr != 0.0);
+  if (in_sum) {
+    const int q = __popc(m_sum & ((1u << lane) - 1u));
+    s_w[warp][q] = (double)((lane + 1) * (lane + 1)) * fr;
+    s_dgg[warp][q] = dgg;
+    s_igg[warp][q] = igg;
+  }
+  __syncwarp();
+  const int n = __popc(m_sum);
+  for (int j = lane; j < FF_NU; j += 32) {
+    double S = 0.0, D = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < n; ++q) {
+      const double* g = G + j + FF_NU * (s_igg[warp][q] - 1);
+      const double g0 = g[0], g1 = g[FF_NU], d = s_dgg[warp][q], w = s_w[warp][q];
+      const double gz = (1.0 - d) * g0 + d * g1;
+      S = S + w * gz;
+      D = D + w * (g1 - g0);
+    }
+    ffsum[(size_t)i * FF_NU + j] = S;
+    ffdsum[(size_t)i * FF_NU + j] = D;
+  }
+  if (lane == 0) {
+    ffclamp[i] = m_fr;
+    ffclamp_all[i] = m_all;
+  }
 }
 
 // Active slots in the reference's loop order (iz ascending, ii = 1..min(iz,ni-1)),
@@ -339,49 +261,69 @@ __device__ double bfxs(const float* __restrict__ ph1, const float* __restrict__ 
   return xs;
 }
 
-// xstab[(igs-1)*nact + a] = bfxs(iz, iz-ii+1, hc/(ev*wlsub(igs))), :177-183
-__global__ void bf_table_kernel(int ngsub, int maxact, const int* __restrict__ pnact,
-                                const int16_t* __restrict__ act_slot, int nst,
+// xstab[(igs-1) nslot + slot] = bfxs(iz, iz-ii+1, hc/(ev*wlsub(igs))) * pc_mbarn,
+// :177-186 (the reference's first product), for every slot that the reference
+// visits (ii <= min(iz, ni-1)), else 0.
+__global__ void bf_table_kernel(int ngsub, int nslot, const int32_t* __restrict__ ion_ni, int nst,
                                 const double* __restrict__ wlsub, const float* __restrict__ ph1,
                                 const float* __restrict__ ph2, double* __restrict__ xstab) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)ngsub * maxact) return;
-  const int igs = (int)(t / maxact) + 1;
-  const int a = (int)(t % maxact);
-  if (a >= *pnact) return;
-  const int slot = act_slot[a];
+  if (t >= (int64_t)ngsub * nslot) return;
+  const int igs = (int)(t / nslot) + 1;
+  const int slot = (int)(t % nslot);
   const int iz = slot / nst + 1, ii = slot % nst + 1;
-  const double wl = wlsub[igs - 1];
-  const double en = pc_hc / (pc_ev * wl);
-  xstab[t] = bfxs(ph1, ph2, iz, iz - ii + 1, en) * pc_mbarn;  // physical_opacity.f:185-186: xs*pc_mbarn first
+  double x = 0.0;
+  if (ii <= min(iz, ion_ni[iz - 1] - 1)) x = bfxs(ph1, ph2, iz, iz - ii + 1, pc_hc / (pc_ev * wlsub[igs - 1])) * pc_mbarn;
+  xstab[t] = x;
 }
 
-// Per sub-group, the xstab entries with a nonzero cross section, in slot
-// order (one warp per sub-group, ballot compaction): xsc = bfxs * pc_mbarn,
-// bslot = the ion slot, bnnz = their count.  The reference skips xs == 0
-// (physical_opacity.f:184), so summing over the compacted entries adds the
-// same terms in the same order.
-__global__ void bf_compact_kernel(int ngsub, int maxact, const int* __restrict__ pnact,
-                                  const int16_t* __restrict__ act_slot, const double* __restrict__ xstab,
-                                  double* __restrict__ xsc, int* __restrict__ bslot, int* __restrict__ bnnz) {
+// One nonzero bound-free cross section of a sub-group (times pc_mbarn) and the
+// ion slot whose population it multiplies.
+struct __align__(16) BfTerm {
+  double xs;
+  int slot, pad;
+};
+
+// Per sub-group, its nonzero cross sections in slot order (the reference's loop
+// order; it skips xs == 0, physical_opacity.f:184), one warp per sub-group.
+__global__ void bf_compact_kernel(int ngsub, int nslot, const double* __restrict__ xstab, BfTerm* __restrict__ terms,
+                                  int* __restrict__ count) {
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (w >= ngsub) return;
-  const int nact = *pnact;
-  const size_t base = (size_t)w * maxact;
+  const size_t base = (size_t)w * nslot;
   int k = 0;
-  for (int a0 = 0; a0 < nact; a0 += 32) {
+  for (int a0 = 0; a0 < nslot; a0 += 32) {
     const int a = a0 + lane;
-    const double x = a < nact ? xstab[base + a] : 0.0;
-    const bool nz = x != 0.0;
-    const unsigned m = __ballot_sync(0xffffffffu, nz);
-    if (nz) {
-      const int pos = k + __popc(m & ((1u << lane) - 1u));
-      xsc[base + pos] = x;
-      bslot[base + pos] = act_slot[a];
-    }
+    const double x = a < nslot ? xstab[base + a] : 0.0;
+    const unsigned m = __ballot_sync(0xffffffffu, x != 0.0);
+    if (x != 0.0) terms[base + k + __popc(m & ((1u << lane) - 1u))] = BfTerm{x, a, 0};
     k += __popc(m);
   }
-  if (lane == 0) bnnz[w] = k;
+  if (lane == 0) count[w] = k;
+}
+
+// Of those, the terms of ions that carry any population, in the same order (a
+// term of an unpopulated ion adds +0).
+__global__ void bf_select_kernel(int ngsub, int nslot, const BfTerm* __restrict__ terms,
+                                 const int* __restrict__ count, const int* __restrict__ active,
+                                 BfTerm* __restrict__ out, int* __restrict__ nout) {
+  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (w >= ngsub) return;
+  const size_t base = (size_t)w * nslot;
+  const int n = count[w];
+  int k = 0;
+  for (int a0 = 0; a0 < n; a0 += 32) {
+    BfTerm t{0.0, 0, 0};
+    bool on = false;
+    if (a0 + lane < n) {
+      t = terms[base + a0 + lane];
+      on = active[t.slot] != 0;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (on) out[base + k + __popc(m & ((1u << lane) - 1u))] = t;
+    k += __popc(m);
+  }
+  if (lane == 0) nout[w] = k;
 }
 
 // One line's shell-independent factors, 16 bytes (one vector load per line):
@@ -392,13 +334,16 @@ __global__ void bf_compact_kernel(int ngsub, int maxact, const int* __restrict__
 // reference's bbxs type), so those bits of its FP64 value are zero: masking
 // them off gives chilw exactly, without a conversion per line.  The indices:
 // bits 0..10 the line's row among the population rows the lines reference
-// (lrow_of_slot), bits 11..26 its population slot (iz - 1) nst + (ii - 1).
+// (lrow_of_slot), bits 11..26 its population slot (iz - 1) nst + (ii - 1), bit
+// 27 set on the last line of its row in its sub-group: a sub-group's lines are
+// ordered by row, so that a sum over lines takes each population once per row.
 struct __align__(16) LineTerm {
   double pg;
   double chi_idx;
 };
 constexpr int kLineRowBits = 11;
 constexpr unsigned kLineIdxMask = 0x1fffffffu;
+constexpr unsigned kLineRowEnd = 1u << 27;
 
 struct LineVals {
   double pg, chi;
@@ -410,59 +355,91 @@ __device__ __forceinline__ LineVals load_line(const LineTerm* p) {
   const unsigned lo = (unsigned)__double2loint(v.y);
   return LineVals{v.x, __hiloint2double(__double2hiint(v.y), (int)(lo & ~kLineIdxMask)), lo & kLineIdxMask};
 }
-__device__ __forceinline__ int line_row(unsigned idx) { return (int)(idx & ((1u << kLineRowBits) - 1)); }
-__device__ __forceinline__ int line_slot(unsigned idx) { return (int)(idx >> kLineRowBits); }
+__device__ __forceinline__ int line_slot(unsigned idx) { return (int)((idx >> kLineRowBits) & 0xffffu); }
 
-// The LineTerm of each binned line of sub-groups 1..ngsub (lines outside the
-// grid get zeros and are never read).
-__global__ void decode_lines_kernel(const slg_bbxs* __restrict__ bb, int64_t nline, const int* __restrict__ lstart,
-                                    int ngsub, const double* __restrict__ wlsub, int nst,
-                                    const int16_t* __restrict__ lrow_of_slot, LineTerm* __restrict__ lt) {
-  const int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= nline) return;
-  // sub-group of line l: the largest igs with lstart[igs] <= l
-  int lo = 0, hi = ngsub + 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (lstart[mid] <= l) lo = mid;
-    else hi = mid - 1;
+// The LineTerms of sub-group w + 1, one warp each: its lines counted by row,
+// the rows' first places, then the lines written there in file order (a lane's
+// place within a round of 32 is its rank among the lanes of the same row), so
+// the layout does not depend on timing.  Dynamic shared memory: nrow ints per warp.
+constexpr int LT_WARPS = 4;
+__global__ void __launch_bounds__(LT_WARPS * 32) line_terms_kernel(const slg_bbxs* __restrict__ bb,
+                                                                   const int* __restrict__ lstart,
+                                                                   int ngsub,
+                                                                   const double* __restrict__ wlsub, int nst,
+                                                                   const int16_t* __restrict__ lrow_of_slot, int nrow,
+                                                                   LineTerm* __restrict__ lt) {
+  extern __shared__ int s_at[];
+  const int w = blockIdx.x * LT_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  int* at = s_at + (size_t)(threadIdx.x >> 5) * nrow;
+  if (w >= ngsub) return;
+  const int igs = w + 1, l0 = lstart[igs], l1 = lstart[igs + 1];
+  for (int r = lane; r < nrow; r += 32) at[r] = 0;
+  __syncwarp();
+  for (int l = l0 + lane; l < l1; l += 32) atomicAdd(&at[lrow_of_slot[(bb[l].iz - 1) * nst + (bb[l].ii - 1)]], 1);
+  __syncwarp();
+  int sum = l0;
+  for (int r0 = 0; r0 < nrow; r0 += 32) {  // exclusive scan of the counts
+    const int n = r0 + lane < nrow ? at[r0 + lane] : 0;
+    int inc = n;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    if (r0 + lane < nrow) at[r0 + lane] = sum + inc - n;
+    sum += __shfl_sync(0xffffffffu, inc, 31);
   }
-  const int igs = lo;
-  LineTerm t{0.0, 0.0};
-  if (igs >= 1 && igs <= ngsub) {
-    const slg_bbxs r = bb[l];
-    const double wa = wlsub[igs - 1], wb = wlsub[igs];
-    const double wl = 0.5 * (wa + wb);
-    const double phi = wl * wl / ((wb - wa) * pc_c);
+  __syncwarp();
+  const double wa = wlsub[igs - 1], wb = wlsub[igs];
+  const double wl = 0.5 * (wa + wb);
+  const double phi = wl * wl / ((wb - wa) * pc_c);
+  for (int c0 = l0; c0 < l1; c0 += 32) {
+    const int l = c0 + lane;
+    slg_bbxs r{0.f, 0.f, 0.f, 1, 1};
+    if (l < l1) r = bb[l];
     const int slot = (r.iz - 1) * nst + (r.ii - 1);
-    const double chi = (double)r.chilw;  // low 29 mantissa bits zero
-    const unsigned idx = ((unsigned)slot << kLineRowBits) | (unsigned)lrow_of_slot[slot];
-    t = LineTerm{phi * (double)r.gxs,
-                 __hiloint2double(__double2hiint(chi), (int)((unsigned)__double2loint(chi) | idx))};
+    const int row = l < l1 ? lrow_of_slot[slot] : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, row);
+    if (l < l1) {
+      const int pos = at[row] + __popc(same & ((1u << lane) - 1u));
+      const double chi = (double)r.chilw;  // low 29 mantissa bits zero
+      const unsigned idx = ((unsigned)slot << kLineRowBits) | (unsigned)row;
+      lt[pos] = LineTerm{phi * (double)r.gxs,
+                         __hiloint2double(__double2hiint(chi), (int)((unsigned)__double2loint(chi) | idx))};
+    }
+    __syncwarp();
+    if (l < l1 && (same & ((1u << lane) - 1u)) == 0u) at[row] += __popc(same);
+    __syncwarp();
   }
-  lt[l] = t;
+  // at[r] is now the end of row r: mark the last line of each row
+  __threadfence_block();
+  __syncwarp();
+  for (int r = lane; r < nrow; r += 32) {
+    const int end = at[r], beg = r == 0 ? l0 : at[r - 1];
+    if (end > beg) {
+      const double x = lt[end - 1].chi_idx;
+      lt[end - 1].chi_idx = __hiloint2double(__double2hiint(x), (int)((unsigned)__double2loint(x) | kLineRowEnd));
+    }
+  }
 }
 
 struct OpacArgs {
   int nc, ng, ngs, ngsub, nelem, nst, maxact;
   int nobb, nobf, noff;
-  const int* pnact;         // number of active bound-free ion slots (device)
+  const int* pnact;         // number of active bound-free ion slots (device; adjoint)
   double mix;
   const double* wlsub;
   const double* grp_wl;
-  const int* lstart;        // (ngsub+2)+1 offsets by igs
-  const slg_bbxs* bb;
-  const LineTerm* lt;       // per binned line (decode_lines_kernel)
+  const int* lstart;        // (ngsub+2)+1 line offsets by igs
+  int ld;                   // row length of grndlev and ocp: nc rounded up to kRun
+  const LineTerm* lt;       // per line, by sub-group and row (line_terms_kernel)
   double chimax;            // largest chilw of the lines (infinite: check every exp argument)
-  const int16_t* slot_of_lrow;  // line row -> slot
-  int nlrow;                // population rows the lines reference
-  int stage_rows = 0;       // forward: stage those rows of a block's shells in shared memory
-  const double* grndlev;    // [slot][cell]
+  const double* grndlev;    // [slot][ld], negative values as zero
+  const double* ocp;        // [slot][ld]
   const double* oc;         // [slot][cell]
-  const int16_t* act_slot;  // active slots, reference order
-  const double* xstab;      // [(igs-1)*maxact + a]: bfxs * pc_mbarn
-  const double* xsc;        // the nonzero entries of xstab per sub-group (bf_compact_kernel)
-  const int* bslot;         // their ion slots
+  const int* active;        // [slot]: nonzero if any cell has population there
+  const int16_t* act_slot;  // the active slots, reference order (adjoint)
+  const double* xstab;      // [(igs-1) nslot + slot]: bfxs * pc_mbarn
+  const BfTerm* bf;         // [(igs-1) nslot + k]: its nonzero entries of populated ions
   const int* bnnz;          // their count per sub-group
   const double* hckt;
   const double* hlparr;
@@ -484,89 +461,79 @@ struct OpacArgs {
   int* flags;
 };
 
-// Sum over n lines of pg * og * exp(-chi h), og the staged population of the
-// line's row for this shell (s_gl: the shell's column of the block's staged
-// rows, FC apart); four lines per round: their loads and exps are
-// independent, and the terms are added one after another in line order, each
-// by one fused multiply-add (one rounding where the reference rounds the
-// product and the sum).  INRANGE: the caller has shown -chi h in [-700, 0] for
-// every line.
-template <bool INRANGE, int FC>
-__device__ __forceinline__ double bb_sum_staged(const LineTerm* lt, int n, double h, const double* s_gl,
-                                                const double* etab) {
-  double sbb = 0.0;
-  int k = 0;
-  for (; k + 4 <= n; k += 4) {
-    LineVals t[4];
-    double og[4], e[4];
+constexpr int kOpacWarps = 4;  // most warps of a forward or adjoint block
+// N neighbouring doubles, N * 8 bytes aligned (at most 16).
+template <int N>
+__device__ __forceinline__ void load_run(const double* __restrict__ p, double* v) {
+  if (N == 1) {
+    v[0] = __ldg(p);
+  } else {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) t[q] = load_line(lt + k + q);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) og[q] = s_gl[line_row(t[q].idx) * FC];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      e[q] = INRANGE ? exp_tang_inrange(-(t[q].chi * h), etab) : exp_tang(-(t[q].chi * h), etab);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sbb = fma(t[q].pg * og[q], e[q], sbb);
+    for (int k = 0; k < N; k += 2) {
+      const double2 d = __ldg(reinterpret_cast<const double2*>(p + k));
+      v[k] = d.x;
+      v[k + 1] = d.y;
+    }
   }
-  for (; k < n; ++k) {
-    const LineVals t = load_line(lt + k);
-    const double og = s_gl[line_row(t.idx) * FC];
-    const double e = INRANGE ? exp_tang_inrange(-(t.chi * h), etab) : exp_tang(-(t.chi * h), etab);
-    sbb = fma(t.pg * og, e, sbb);
-  }
-  return sbb;
 }
 
-// bb_sum_staged for the FS shells of a lane at once (s_gl: the first shell's
-// column; the others' are OPAC_CT apart, rows FS * OPAC_CT apart): each line
-// record's load and index work serves FS terms.  NL lines per round: FS * NL
-// independent exps.
-template <bool INRANGE, int FS, int NL>
-__device__ __forceinline__ void bb_sum_staged_fs(const LineTerm* lt, int n, const double* h, const double* s_gl,
-                                                 const double* etab, double* sbb) {
-  constexpr int FC = FS * OPAC_CT;
-  double a[FS];
+// Bound-bound sums of a lane's FS neighbouring shells (pop: their first entry of
+// the population rows, ld apart; arg: their exp arguments) over the n >= 1
+// lines of a sub-group: per row sum of pg exp(-chi h), times the row's
+// population, the rows added one after another by fused multiply-adds.  The
+// next record and the next row's populations are loaded ahead.  (A loop per row:
+// as a test after each line the row's end was compiled to predicated
+// instructions that every line issued, 4 of 26 per term.)
+template <int FS>
+__device__ __forceinline__ void bb_sums(const LineTerm* __restrict__ lt, int n, const ExpArg* arg, const ExpConst& C,
+                                        const double* __restrict__ pop, int ld, const double* s_tab, uint32_t mine,
+                                        double* a) {
+  double og[FS];
+  LineVals t = load_line(lt);
+  load_run<FS>(pop + (size_t)line_slot(t.idx) * ld, og);
 #pragma unroll
   for (int s = 0; s < FS; ++s) a[s] = 0.0;
-  int k = 0;
-  for (; k + NL <= n; k += NL) {
-    LineVals t[NL];
+  const LineTerm* const end = lt + n;
+  do {
+    double acc[FS];
 #pragma unroll
-    for (int q = 0; q < NL; ++q) t[q] = load_line(lt + k + q);
+    for (int s = 0; s < FS; ++s) acc[s] = 0.0;
+#pragma unroll 1
+    for (;;) {
+      const LineVals u = load_line(lt + 1);
 #pragma unroll
-    for (int q = 0; q < NL; ++q) {
-      const double* r = s_gl + line_row(t[q].idx) * FC;
-#pragma unroll
-      for (int s = 0; s < FS; ++s) {
-        const double e = INRANGE ? exp_tang_inrange(-(t[q].chi * h[s]), etab) : exp_tang(-(t[q].chi * h[s]), etab);
-        a[s] = fma(t[q].pg * r[s * OPAC_CT], e, a[s]);
+      for (int s = 0; s < FS; ++s) acc[s] = fma(t.pg, exp_scaled(t.chi, arg[s], C, s_tab, mine), acc[s]);
+      ++lt;
+      if (t.idx & kLineRowEnd) {  // the same for the whole warp
+        t = u;
+        break;
       }
+      t = load_line(lt + 1);
+#pragma unroll
+      for (int s = 0; s < FS; ++s) acc[s] = fma(u.pg, exp_scaled(u.chi, arg[s], C, s_tab, mine), acc[s]);
+      ++lt;
+      if (u.idx & kLineRowEnd) break;
     }
-  }
-  for (; k < n; ++k) {
+#pragma unroll
+    for (int s = 0; s < FS; ++s) a[s] = fma(acc[s], og[s], a[s]);
+    load_run<FS>(pop + (size_t)line_slot(t.idx) * ld, og);  // (any row's where none follows)
+  } while (lt < end);
+}
+// The same for any arguments (a shell too cool for exp_scaled's range, or not a number).
+__device__ __noinline__ double bb_sum_any(const LineTerm* __restrict__ lt, int n, double h,
+                                          const double* __restrict__ pop, int ld) {
+  double a = 0.0;
+  for (int k = 0; k < n; ++k) {
     const LineVals t = load_line(lt + k);
-    const double* r = s_gl + line_row(t.idx) * FC;
-#pragma unroll
-    for (int s = 0; s < FS; ++s) {
-      const double e = INRANGE ? exp_tang_inrange(-(t.chi * h[s]), etab) : exp_tang(-(t.chi * h[s]), etab);
-      a[s] = fma(t.pg * r[s * OPAC_CT], e, a[s]);
-    }
+    const double og = __ldg(pop + (size_t)line_slot(t.idx) * ld);
+    if (og <= 0.0) continue;
+    a = fma(t.pg * og, exp(-(t.chi * h)), a);
   }
-#pragma unroll
-  for (int s = 0; s < FS; ++s) sbb[s] = a[s];
+  return a;
 }
 
-// Bound-free and free-free of sub-group igs for shell i (h = hc/kT), added to
-// cap in the reference's order (after the bound-bound term).
-__device__ inline double bf_ff_add(const OpacArgs& A, int i, int igs, double h, double cap) {
-  if (!A.nobf) {
-    const size_t base = (size_t)(igs - 1) * A.maxact;
-    const int n = A.bnnz[igs - 1];
-    const double* oci = A.oc + i;
-    for (int k = 0; k < n; ++k)  // bfxs * pc_mbarn (the reference's first product) * population
-      cap = cap + __ldg(A.xsc + base + k) * oci[(size_t)__ldg(A.bslot + base + k) * A.nc];
-  }
+// Free-free of sub-group igs for shell i (h = hc/kT), added to cap.
+__device__ inline double ff_add(const OpacArgs& A, int i, int igs, double h, double cap) {
   if (!A.noff) {
     const double wl = A.wlsub[igs - 1];
     const double wlinv = 1.0 / wl;
@@ -603,158 +570,129 @@ __device__ __forceinline__ double bb_expfac(const OpacArgs& A, int igs, double h
   return 1.0 - exp(-(h * wlinv));
 }
 
-// One sub-group igs for shell i: bb, bf and ff in the reference's order.
-// etab: the exp table (kExp2Tab) in shared memory; s_gl: the shell's column of
-// the block's staged population rows ([line row][FC] in shared memory), or
-// null (read grndlev).
-template <int FC>
-__device__ inline double subgroup_opacity(const OpacArgs& A, int i, const double* s_gl, int igs, bool live,
-                                          const double* etab) {
-  double cap = 0.0;
-  if (!live) return cap;
-  const double h = A.hckt[i];
-  if (!A.nobb) {
-    const int l0 = A.lstart[igs], l1 = A.lstart[igs + 1];
-    if (l1 > l0) {
-      const double expfac = bb_expfac(A, igs, h);
-      // sum over the sub-group's lines of phi gxs ocg exp(-chilw h), times the
-      // stimulated-emission factor once (the reference multiplies each term by
-      // it; the sum of positive terms differs by rounding only)
-      const LineTerm* lt = A.lt + l0;
-      const int n = l1 - l0;
-      double sbb;
-      // h * chimax <= 700: every exp argument -chi h lies in [-700, 0], where
-      // exp_tang needs no range check
-      const bool inrange = h >= 0.0 && h * A.chimax <= 700.0;
-      if (s_gl) {
-        // staged populations are clamped at zero, so a term of an unpopulated
-        // ion adds +0 (the reference skips it: the same sum)
-        sbb = inrange ? bb_sum_staged<true, FC>(lt, n, h, s_gl, etab) : bb_sum_staged<false, FC>(lt, n, h, s_gl, etab);
-      } else {
-        sbb = 0.0;
-        for (int k = 0; k < n; ++k) {
-          const LineVals t = load_line(lt + k);
-          const double ocg = A.grndlev[(size_t)line_slot(t.idx) * A.nc + i];
-          if (ocg <= 0.0) continue;
-          sbb = fma(t.pg * ocg, exp_tang(-(t.chi * h), etab), sbb);
-        }
-      }
-      cap = cap + sbb * expfac;
-    }
-  }
-  return bf_ff_add(A, i, igs, h, cap);
-}
-
-// Block: FS * OPAC_CT shells x OPAC_GT groups; warp w takes group
-// blockIdx.y * OPAC_GT + w + 1, lane l shells base + s OPAC_CT + l, s < FS.
+// Block: groups blockIdx.x * gpb + 1 .. + gpb one after another; warp w takes the
+// 32 FS shells from (blockIdx.y * warps + w) 32 FS, lane l the FS from l FS on.
+//
+// Bound by instruction issue around the FP64 pipe: 11 FP64 operations per
+// line-shell term (ten of them the exp), one shared-memory load, three integer
+// operations for the exp and a line's and a row's share of loads and tests.
+// FS shells per lane share a line record's load and index work; the warps of a
+// block walk the same lines, so they share the records in L1 and end together;
+// lines ordered by row leave one multiplication and one population load per row.
+// Seven blocks per SM (72 registers) measured best of four to eight.  4096
+// shells x 10000 groups x 2e6 lines: 9.6 -> 8.9 ms, 256 x 2000 x 5e5: 184 -> 165 us
+// (lines in file order, four shells per lane, populations staged in shared
+// memory, exp without the scaled argument and the spread table).
 template <int FS>
-__global__ void __launch_bounds__(OPAC_GT * 32, 4) opacity_fwd_kernel(const OpacArgs A) {
+__global__ void __launch_bounds__(kOpacWarps * 32, 7) opacity_fwd_kernel(const OpacArgs A, const ExpConst C, int gpb) {
   constexpr int FC = FS * OPAC_CT;
-  __shared__ float tcap[FC][OPAC_GT + 1];
-  __shared__ float tem[FC][OPAC_GT + 1];
-  __shared__ double tcapd[FC][OPAC_GT + 1];
-  __shared__ double etab[kExpTabN];
-  extern __shared__ double s_rows[];  // [line row][FC] populations of this block's shells (A.stage_rows)
-  exp_table_load(etab);
-  const int base = blockIdx.x * FC;
-  if (A.stage_rows) {
-    for (int k = threadIdx.x; k < A.nlrow * FC; k += blockDim.x) {
-      const int ii = base + (k % FC);
-      const double v = ii < A.nc ? A.grndlev[(size_t)A.slot_of_lrow[k / FC] * A.nc + ii] : 0.0;
-      s_rows[k] = v < 0.0 ? 0.0 : v;  // the reference skips lines with ocg <= 0
-    }
-  }
+  __shared__ double etab[kExpTabN * kExpCopies];
+  exp_table_spread(etab);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ig = blockIdx.y * OPAC_GT + warp + 1;  // 1-based group
-  int ii[FS];
-  bool valid[FS], live[FS];
-  double cap[FS];
+  const uint32_t mine = exp_table_mine();
+  const int base = (blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5)) * FC, lane = threadIdx.x & 31;
+  if (base >= A.nc) return;  // uniform over the warp
+  const int i0 = base + lane * FS;  // the lane's first shell (0-based)
+  bool live[FS];
+  double h[FS];
+  ExpArg arg[FS];
+  bool inrange = true;
 #pragma unroll
   for (int s = 0; s < FS; ++s) {
-    ii[s] = base + s * OPAC_CT + lane;  // 0-based shell
-    valid[s] = ig <= A.ng && ii[s] < A.nc;
-    live[s] = valid[s] && A.mass[ii[s]] > 0.0;
-    cap[s] = 0.0;
+    live[s] = i0 + s < A.nc && A.mass[i0 + s] > 0.0;
+    // a shell that is not live runs the loops with h = 0 and is discarded
+    h[s] = live[s] ? A.hckt[i0 + s] : 0.0;
+    arg[s] = exp_arg(h[s]);
+    inrange = inrange && h[s] >= 0.0 && h[s] * A.chimax <= 700.0;
   }
-  if (A.ngs == 1 && A.stage_rows) {
-    // both shells' bound-bound sums in one pass over the group's lines
-    // (a shell that is not live runs the loop with h = 0 and is discarded)
-    double h[FS];
+  // every exp argument -chi h of the warp's shells lies in [-700, 0]
+  inrange = __all_sync(0xffffffffu, inrange);
+  for (int ig = blockIdx.x * gpb + 1; ig <= min((int)(blockIdx.x + 1) * gpb, A.ng); ++ig) {
+    double cap[FS], sp[FS], sr[FS];
 #pragma unroll
-    for (int s = 0; s < FS; ++s) h[s] = live[s] ? A.hckt[ii[s]] : 0.0;
-    const int l0 = ig <= A.ng ? A.lstart[ig] : 0, l1 = ig <= A.ng ? A.lstart[ig + 1] : 0;
-    double sbb[FS];
+    for (int s = 0; s < FS; ++s) cap[s] = sp[s] = sr[s] = 0.0;
+    for (int g = 1; g <= A.ngs; ++g) {
+      const int igs = (ig - 1) * A.ngs + g;
+      double c[FS];
 #pragma unroll
-    for (int s = 0; s < FS; ++s) sbb[s] = 0.0;
-    if (!A.nobb && l1 > l0) {
-      bool inrange = true;
+      for (int s = 0; s < FS; ++s) c[s] = 0.0;
+      if (!A.nobb) {
+        const int l0 = A.lstart[igs], n = A.lstart[igs + 1] - l0;
+        if (n > 0) {
+          // sum over the sub-group's lines of phi gxs ocg exp(-chilw h), times the
+          // stimulated-emission factor once (the reference multiplies each term
+          // by it; the sum of positive terms differs by rounding only)
+          double sbb[FS];
+          if (inrange) {
+            bb_sums<FS>(A.lt + l0, n, arg, C, A.grndlev + i0, A.ld, etab, mine, sbb);
+          } else {
 #pragma unroll
-      for (int s = 0; s < FS; ++s) inrange = inrange && h[s] >= 0.0 && h[s] * A.chimax <= 700.0;
-      constexpr int NL = FS == 2 ? 4 : 2;  // eight exps in flight
-      if (inrange)
-        bb_sum_staged_fs<true, FS, NL>(A.lt + l0, l1 - l0, h, s_rows + lane, etab, sbb);
-      else
-        bb_sum_staged_fs<false, FS, NL>(A.lt + l0, l1 - l0, h, s_rows + lane, etab, sbb);
-    }
+            for (int s = 0; s < FS; ++s)
+              sbb[s] = live[s] ? bb_sum_any(A.lt + l0, n, h[s], A.grndlev + i0 + s, A.ld) : 0.0;
+          }
 #pragma unroll
-    for (int s = 0; s < FS; ++s) {
-      if (!live[s]) continue;
-      double c = 0.0;
-      if (!A.nobb && l1 > l0) c = c + sbb[s] * bb_expfac(A, ig, h[s]);
-      cap[s] = bf_ff_add(A, ii[s], ig, h[s], c);
-    }
-  } else {
-#pragma unroll 1
-    for (int s = 0; s < FS; ++s) {
-      if (!valid[s]) continue;
-      const double* s_gl = A.stage_rows ? s_rows + s * OPAC_CT + lane : nullptr;
-      if (A.ngs == 1) {
-        cap[s] = subgroup_opacity<FC>(A, ii[s], s_gl, ig, live[s], etab);
-      } else {
-        // collapse subgridding, physical_opacity.f:252-264
-        double sp = 0.0, sr = 0.0;
-        for (int g = 1; g <= A.ngs; ++g) {
-          const double v = subgroup_opacity<FC>(A, ii[s], s_gl, (ig - 1) * A.ngs + g, live[s], etab);
-          if (v > 0.0) { sp = sp + v; sr = sr + 1.0 / v; }
+          for (int s = 0; s < FS; ++s)
+            if (live[s]) c[s] = sbb[s] * bb_expfac(A, igs, h[s]);
         }
-        const double help = 1.0 / A.ngs;
-        const double capp = sp * help;
-        double capr = sr * help;
-        if (capr > 0.0) capr = 1.0 / capr;
-        cap[s] = (1.0 - A.mix) * capp + A.mix * capr;
+      }
+      if (!A.nobf) {
+        const BfTerm* t = A.bf + (size_t)(igs - 1) * A.maxact;
+        const int n = A.bnnz[igs - 1];
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+          const double2 v = __ldg(reinterpret_cast<const double2*>(t + k));
+          double o[FS];
+          load_run<FS>(A.ocp + i0 + (size_t)__double2loint(v.y) * A.ld, o);
+#pragma unroll
+          for (int s = 0; s < FS; ++s) c[s] = fma(v.x, o[s], c[s]);
+        }
+      }
+      if (!A.noff) {
+#pragma unroll
+        for (int s = 0; s < FS; ++s)
+          if (live[s]) c[s] = ff_add(A, i0 + s, igs, h[s], c[s]);
+      }
+#pragma unroll
+      for (int s = 0; s < FS; ++s) {
+        if (A.ngs == 1) cap[s] = c[s];
+        else if (live[s] && c[s] > 0.0) { sp[s] = sp[s] + c[s]; sr[s] = sr[s] + 1.0 / c[s]; }
       }
     }
-  }
+    if (A.ngs != 1) {
+      // collapse subgridding, physical_opacity.f:252-264
+      const double help = 1.0 / A.ngs;
 #pragma unroll
-  for (int s = 0; s < FS; ++s) {
-    const int i = ii[s];
-    float c32 = (float)cap[s], e32 = 0.f;
-    if (live[s]) {
-      const double wl = 0.5 * (A.grp_wl[ig] + A.grp_wl[ig - 1]);
-      const double B_nu = (wl * wl / pc_c) * planck(wl, A.temp[i]);
-      e32 = (float)(0.0 + cap[s] * B_nu);
-      int f = 0;
-      if (c32 == 0.f) f |= 1;
-      if (c32 < 0.f) f |= 2;
-      if (c32 != c32) f |= 4;
-      if (c32 > FLT_MAX) f |= 8;
-      if (f) atomicOr(A.flags, f);
+      for (int s = 0; s < FS; ++s) {
+        double capr = sr[s] * help;
+        if (capr > 0.0) capr = 1.0 / capr;
+        cap[s] = (1.0 - A.mix) * (sp[s] * help) + A.mix * capr;
+      }
     }
-    if (valid[s] && A.cap64) A.cap64[(size_t)(ig - 1) * A.nc + i] = cap[s];
-    tcap[s * OPAC_CT + lane][warp] = c32;
-    tem[s * OPAC_CT + lane][warp] = e32;
-    if (A.capg64) tcapd[s * OPAC_CT + lane][warp] = cap[s];
-  }
-  __syncthreads();
-  // write (ng, ncell): each shell's OPAC_GT consecutive groups together
-  for (int t = threadIdx.x; t < FC * OPAC_GT; t += blockDim.x) {
-    const int ci = t / OPAC_GT, gj = t % OPAC_GT;
-    const int i2 = base + ci, g2 = blockIdx.y * OPAC_GT + gj;
-    if (i2 < A.nc && g2 < A.ng) {
-      A.cap32[(size_t)i2 * A.ng + g2] = tcap[ci][gj];
-      A.emiss32[(size_t)i2 * A.ng + g2] = tem[ci][gj];
-      if (A.capg64) A.capg64[(size_t)i2 * A.ng + g2] = tcapd[ci][gj];
+#pragma unroll
+    for (int s = 0; s < FS; ++s) {
+      const int i = i0 + s;
+      if (i >= A.nc) continue;
+      if (!live[s]) cap[s] = 0.0;
+      const float c32 = (float)cap[s];
+      float e32 = 0.f;
+      if (live[s]) {
+        const double wl = 0.5 * (A.grp_wl[ig] + A.grp_wl[ig - 1]);
+        const double B_nu = (wl * wl / pc_c) * planck(wl, A.temp[i]);
+        e32 = (float)(0.0 + cap[s] * B_nu);
+        int f = 0;
+        if (c32 == 0.f) f |= 1;
+        if (c32 < 0.f) f |= 2;
+        if (c32 != c32) f |= 4;
+        if (c32 > FLT_MAX) f |= 8;
+        if (f) atomicOr(A.flags, f);
+      }
+      // (ng, ncell): a shell's neighbouring groups are this block's next ones, so
+      // the parts of a sector meet in L2
+      const size_t o = (size_t)i * A.ng + (ig - 1);
+      A.cap32[o] = c32;
+      A.emiss32[o] = e32;
+      if (A.capg64) A.capg64[o] = cap[s];
+      if (A.cap64) A.cap64[(size_t)(ig - 1) * A.nc + i] = cap[s];
     }
   }
 }
@@ -932,187 +870,205 @@ struct OpacBwd {
   double* goc;         // [slot][cell], added to (bound-free)
   double* ghlp;        // (ncell), added to (d cap / d hlparr)
   double* gfr;         // (0:nelem, ncell), added to
-  double* W;           // [cell][81], added to: free-free table-row weights (null with noff)
+  double* W;           // [81][cell], added to: free-free table-row weights (null with noff)
 };
 
-// The bound-bound part of the adjoint for one (shell, group): adds
-// ue * d cap / d grndlev / expfac = ue * pg * exp(-chi h) of every line
-// (ue = u * expfac) to dL/d grndlev of its population row: GRED, in global
-// memory (acc_l = ggrnd + shell, entry slot * nc: one reduction without
-// return per term, coalesced over the warp's shells), else in the block's
-// shared accumulator (acc_l = s_grnd + lane, entry row * 32, atomics with
-// return).  Global reductions pay when the accumulated array is large (many
-// shells x rows: the updates spread over many addresses); on a small one they
-// queue on the same addresses, where the shared accumulator wins.  Returns
-// the sums over lines of pg exp(-chi h) og (capbb / expfac) and of the same
-// times chi (the T-derivative's weight).  Staged populations are clamped at
-// zero, so an unpopulated ion's term is +0 as the forward's skip.  Four lines
-// per round: independent loads and exps.
-template <bool INRANGE, bool GRED>
-__device__ __forceinline__ void bb_adjoint_staged(const LineTerm* lt, int n, double h, double ue,
-                                                  const double* s_gl, double* acc_l, size_t nc,
-                                                  const double* etab, double& sbb, double& schi) {
-  int k = 0;
-  for (; k + 4 <= n; k += 4) {
-    LineVals t[4];
-    int r[4];
-    double e[4], o[4];
+// The bound-bound part of the adjoint of one group for FS shells of a lane (i0,
+// i0 + 32 ...; ue: dL/dcap times the stimulated-emission factor): adds ue * pg *
+// exp(-chi h) of every line (d cap / d grndlev) to dL/d grndlev of its row, the
+// row's sum by one reduction without return (coalesced over the warp's shells),
+// and returns the sums over lines of pg exp(-chi h) og (capbb over that factor)
+// and of the same times chi (the T-derivative's weight).  FAST: exp_scaled's
+// range holds for every argument.
+template <int FS, bool FAST>
+__device__ __forceinline__ void bb_adjoint(const LineTerm* __restrict__ lt, int n, const double* h, const ExpArg* arg,
+                                           const ExpConst& C, const double* ue, const double* __restrict__ pop, int ld,
+                                           double* __restrict__ ggrnd, int nc, const double* s_tab, uint32_t mine,
+                                           double* sbb, double* schi) {
+  double og[FS];
+  auto row_begin = [&](unsigned idx) {
+    const double* g = pop + (size_t)line_slot(idx) * ld;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) t[q] = load_line(lt + k + q);
+    for (int s = 0; s < FS; ++s) og[s] = __ldg(g + s * OPAC_CT);
+  };
+  auto term = [&](const LineVals& v, double* acc, double* accc) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      r[q] = line_row(t[q].idx) << 5;
-      o[q] = s_gl[r[q]];
+    for (int s = 0; s < FS; ++s) {
+      const double e = v.pg * (FAST ? exp_scaled(v.chi, arg[s], C, s_tab, mine) : exp(-(v.chi * h[s])));
+      acc[s] = acc[s] + e;
+      accc[s] = fma(e, v.chi, accc[s]);
     }
+  };
+  LineVals t = load_line(lt);
+  row_begin(t.idx);
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      e[q] = t[q].pg * (INRANGE ? exp_tang_inrange(-(t[q].chi * h), etab) : exp_tang(-(t[q].chi * h), etab));
+  for (int s = 0; s < FS; ++s) sbb[s] = schi[s] = 0.0;
+  const LineTerm* const end = lt + n;
+  do {
+    double acc[FS], accc[FS];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      atomicAdd(acc_l + (GRED ? (size_t)line_slot(t[q].idx) * nc : (size_t)r[q]), ue * e[q]);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const double x = e[q] * o[q];
-      sbb = sbb + x;
-      schi = fma(x, t[q].chi, schi);
+    for (int s = 0; s < FS; ++s) acc[s] = accc[s] = 0.0;
+    const int slot = line_slot(t.idx);
+#pragma unroll 1
+    for (;;) {
+      const LineVals u = load_line(lt + 1);
+      term(t, acc, accc);
+      ++lt;
+      if (t.idx & kLineRowEnd) {  // the same for the whole warp
+        t = u;
+        break;
+      }
+      t = load_line(lt + 1);
+      term(u, acc, accc);
+      ++lt;
+      if (u.idx & kLineRowEnd) break;
     }
-  }
-  for (; k < n; ++k) {
-    const LineVals t = load_line(lt + k);
-    const int r = line_row(t.idx) << 5;
-    const double e = t.pg * (INRANGE ? exp_tang_inrange(-(t.chi * h), etab) : exp_tang(-(t.chi * h), etab));
-    atomicAdd(acc_l + (GRED ? (size_t)line_slot(t.idx) * nc : (size_t)r), ue * e);
-    const double x = e * s_gl[r];
-    sbb = sbb + x;
-    schi = fma(x, t.chi, schi);
-  }
+    double* g = ggrnd + (size_t)slot * nc;
+#pragma unroll
+    for (int s = 0; s < FS; ++s) {
+      if (ue[s] != 0.0) atomicAdd(g + s * OPAC_CT, ue[s] * acc[s]);
+      sbb[s] = fma(acc[s], og[s], sbb[s]);
+      schi[s] = fma(accc[s], og[s], schi[s]);
+    }
+    row_begin(t.idx);  // (any row's where none follows)
+  } while (lt < end);
 }
 
-// Adjoint of subgroup_opacity (ngs = 1): bb and ff in one pass over the lines
-// of each group (bf: bf_bwd_kernel); d/d(natomfr) sums gathered per (element,
-// shell) in shared memory, d/d(grndlev) as bb_adjoint_staged's GRED says.
-template <bool GRED>
-__global__ void __launch_bounds__(OPAC_GT * 32, 4) opacity_bwd_kernel(const OpacArgs A, const OpacBwd B) {
-  extern __shared__ double sm[];
-  const int nrow = A.nlrow;                          // population rows the lines reference
-  const int nacc = GRED ? 0 : nrow;                  // shared accumulator rows
-  double* s_W = sm;                                  // [81][32] free-free table-row weights
-  double* s_grnd = s_W + FF_NU * 32;                 // [line row][32] (not GRED)
-  double* s_fr = s_grnd + (size_t)nacc * 32;         // [nelem+1][32]
-  double* s_t = s_fr + (size_t)(A.nelem + 1) * 32;   // [warp][32]
-  double* s_h = s_t + OPAC_GT * 32;
-  double* s_g = s_h + OPAC_GT * 32;                  // [line row][32] populations of this block's shells
-  const int ntot = (FF_NU + nacc + A.nelem + 1) * 32;
-  __shared__ double etab[kExpTabN];
-  exp_table_load(etab);
-  for (int k = threadIdx.x; k < ntot; k += blockDim.x) sm[k] = 0.0;
-  for (int k = threadIdx.x; k < nrow * 32; k += blockDim.x) {
-    const int ii = blockIdx.x * OPAC_CT + (k & 31);
-    const double v = ii < A.nc ? A.grndlev[(size_t)A.slot_of_lrow[k >> 5] * A.nc + ii] : 0.0;
-    s_g[k] = v < 0.0 ? 0.0 : v;  // the forward skips lines with ocg <= 0: a zero term
+// The free-free part of the adjoint of one (shell, group): adds the group's
+// table-row weights to W and the clamped elements' d/d fr to gfr; returns dL/dT
+// and dL/d hlparr.
+__device__ inline double2 ff_adjoint(const OpacArgs& A, const OpacBwd& B, int i, int ig, double h, double u) {
+  const double T = A.temp[i];
+  const double wl = A.wlsub[ig - 1];
+  const double wlinv = 1.0 / wl;
+  const double uu = h * wlinv;
+  const double ru = 10.0 * (log10(uu) + 4.0) + 1.0;
+  const int iu = !(ru >= 1.0) ? 1 : (ru >= (double)(FF_NU - 1) ? FF_NU - 1 : (int)floor(ru));
+  const double du = ru - iu;
+  const double eu = exp(-uu);
+  const double hn = A.ffc1 * sqrt(h) * (1.0 - eu) * cube(wl);
+  const double help = hn * A.hlparr[i];
+  const double dlnhelp = -0.5 / T - eu * uu / (T * (1.0 - eu));
+  const double ln10 = 2.302585092994045684;
+  const double dru = -10.0 / (ln10 * T), drgg = -5.0 / (ln10 * T);  // table coordinates vs T
+  // this group's weights of table rows iu - 1 and iu, for d cap / d fr of
+  // the unclamped elements (ff_fr_bwd_kernel)
+  atomicAdd(&B.W[(size_t)(iu - 1) * A.nc + i], u * help * (1.0 - du));
+  atomicAdd(&B.W[(size_t)iu * A.nc + i], u * help * du);
+  // unclamped elements from the shell's sums over elements (ff_sum_kernel):
+  // S = sum z^2 fr gff, dS/dT through the table row (du) and column (dgg)
+  const double* Sv = A.ffsum + (size_t)i * FF_NU;
+  const double* Dv = A.ffdsum + (size_t)i * FF_NU;
+  const double s0 = Sv[iu - 1], s1 = Sv[iu];
+  double S = (1.0 - du) * s0 + du * s1;
+  double dS = (s1 - s0) * dru + ((1.0 - du) * Dv[iu - 1] + du * Dv[iu]) * drgg;
+  // elements under the gff >= 1 clamp, one by one
+  const double* nfr = A.natomfr + (size_t)(A.nelem + 1) * i;
+  for (unsigned m = A.ffclamp_all[i]; m; m &= m - 1) {
+    const int iz = __ffs(m);
+    const double fr = nfr[iz];
+    const int igg = -A.ffigg[(size_t)(iz - 1) * A.nc + i];
+    const double dgg = A.ffdgg[(size_t)(iz - 1) * A.nc + i];
+    const double* G = A.gff;
+    const double g00 = G[(iu - 1) + FF_NU * (igg - 1)], g10 = G[iu + FF_NU * (igg - 1)];
+    const double g01 = G[(iu - 1) + FF_NU * igg], g11 = G[iu + FF_NU * igg];
+    const double graw = (1.0 - du) * (1.0 - dgg) * g00 + du * (1.0 - dgg) * g10 + (1.0 - du) * dgg * g01 +
+                        du * dgg * g11;
+    const bool flat = graw < 1.0;
+    const double g = flat ? 1.0 : graw;
+    const double dg = flat ? 0.0
+                           : ((1.0 - dgg) * (g10 - g00) + dgg * (g11 - g01)) * dru +
+                                 ((1.0 - du) * (g01 - g00) + du * (g11 - g10)) * drgg;
+    const double w = (double)(iz * iz);
+    atomicAdd(&B.gfr[(size_t)i * (A.nelem + 1) + iz], u * help * g * w);
+    if (fr == 0.0) continue;
+    S = S + g * w * fr;
+    dS = dS + dg * w * fr;
   }
+  return make_double2(u * (help * S * dlnhelp + help * dS), u * hn * S);
+}
+
+// Adjoint of the forward's groups (ngs = 1): bb and ff in one pass over the lines
+// of each group (bf: bf_bwd_kernel).  Block: groups blockIdx.x * gpb + 1 .. + gpb
+// one after another; warp w takes the 32 FS shells from (blockIdx.y * warps + w)
+// 32 FS, lane l shells l, l + 32 ... of them.  Bound like the forward, with 13
+// FP64 operations per term; a population row's gradient leaves by one
+// reduction per (row, group) instead of one per line, whose L2 traffic held the
+// kernel at half its arithmetic's rate.
+template <int FS>
+__global__ void __launch_bounds__(kOpacWarps * 32, 4) opacity_bwd_kernel(const OpacArgs A, const OpacBwd B,
+                                                                               const ExpConst C, int gpb) {
+  __shared__ double etab[kExpTabN * kExpCopies];
+  exp_table_spread(etab);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ig = blockIdx.y * OPAC_GT + warp + 1;
-  const int i = blockIdx.x * OPAC_CT + lane;
-  const bool live = ig <= A.ng && i < A.nc && A.mass[i] > 0.0;
-  double gt = 0.0, gh = 0.0;
-  const double u = live ? B.gcap[(size_t)i * A.ng + (ig - 1)] : 0.0;
-  if (u != 0.0) {
-    const double h = A.hckt[i], T = A.temp[i];
-    if (!A.nobb) {
-      const int l0 = A.lstart[ig], l1 = A.lstart[ig + 1];
-      if (l1 > l0) {
-        const double wa = A.wlsub[ig - 1], wb = A.wlsub[ig];
-        const double wl = 0.5 * (wa + wb);
-        const double wlinv = 1.0 / wl;
-        const double eh = exp(-(h * wlinv));
-        const double expfac = 1.0 - eh;
-        double sbb = 0.0, schi = 0.0;
-        const double ue = u * expfac;
-        const bool inrange = h >= 0.0 && h * A.chimax <= 700.0;  // as in the forward
-        double* acc_l = GRED ? B.ggrnd + i : s_grnd + lane;
-        if (inrange)
-          bb_adjoint_staged<true, GRED>(A.lt + l0, l1 - l0, h, ue, s_g + lane, acc_l, A.nc, etab, sbb, schi);
-        else
-          bb_adjoint_staged<false, GRED>(A.lt + l0, l1 - l0, h, ue, s_g + lane, acc_l, A.nc, etab, sbb, schi);
-        const double capbb = sbb * expfac;
-        schi = schi * expfac;
-        // h = hc/kT: d exp(-chi h)/dT = chi h/T exp(..), d expfac/dT = -(h/T) wlinv eh
-        gt = gt + u * ((h / T) * schi - capbb * (h / T) * wlinv * eh / expfac);
-      }
+  const uint32_t mine = exp_table_mine();
+  const int base = (blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (FS * OPAC_CT), lane = threadIdx.x & 31;
+  if (base >= A.nc) return;  // uniform over the warp
+  bool live[FS];
+  int ii[FS];
+  double h[FS], gt[FS], gh[FS];
+  ExpArg arg[FS];
+  bool inrange = true;
+#pragma unroll
+  for (int s = 0; s < FS; ++s) {
+    const int i = base + s * OPAC_CT + lane;
+    ii[s] = min(i, A.nc - 1);
+    live[s] = i < A.nc && A.mass[ii[s]] > 0.0;
+    h[s] = live[s] ? A.hckt[ii[s]] : 0.0;
+    arg[s] = exp_arg(h[s]);
+    inrange = inrange && h[s] >= 0.0 && h[s] * A.chimax <= 700.0;  // as in the forward
+    gt[s] = gh[s] = 0.0;
+  }
+  inrange = __all_sync(0xffffffffu, inrange);
+  const double* const pop = A.grndlev + base + lane;
+  for (int ig = blockIdx.x * gpb + 1; ig <= min((int)(blockIdx.x + 1) * gpb, A.ng); ++ig) {
+    double u[FS];
+    bool any = false;
+#pragma unroll
+    for (int s = 0; s < FS; ++s) {
+      u[s] = live[s] ? B.gcap[(size_t)ii[s] * A.ng + (ig - 1)] : 0.0;
+      any = any || u[s] != 0.0;
     }
-    // bound-free: bf_bwd_kernel
-    if (!A.noff) {
-      const double wl = A.wlsub[ig - 1];
+    if (!__any_sync(0xffffffffu, any)) continue;
+    const int l0 = A.nobb ? 0 : A.lstart[ig], n = A.nobb ? 0 : A.lstart[ig + 1] - l0;
+    if (n > 0) {
+      const double wa = A.wlsub[ig - 1], wb = A.wlsub[ig];
+      const double wl = 0.5 * (wa + wb);
       const double wlinv = 1.0 / wl;
-      const double uu = h * wlinv;
-      const double ru = 10.0 * (log10(uu) + 4.0) + 1.0;
-      const int iu = !(ru >= 1.0) ? 1 : (ru >= (double)(FF_NU - 1) ? FF_NU - 1 : (int)floor(ru));
-      const double du = ru - iu;
-      const double eu = exp(-uu);
-      const double hn = A.ffc1 * sqrt(h) * (1.0 - eu) * cube(wl);
-      const double help = hn * A.hlparr[i];
-      const double dlnhelp = -0.5 / T - eu * uu / (T * (1.0 - eu));
-      const double ln10 = 2.302585092994045684;
-      const double dru = -10.0 / (ln10 * T), drgg = -5.0 / (ln10 * T);  // table coordinates vs T
-      // this group's weights of table rows iu - 1 and iu, for d cap / d fr of
-      // the unclamped elements (ff_fr_bwd_kernel)
-      atomicAdd(&s_W[(iu - 1) * 32 + lane], u * help * (1.0 - du));
-      atomicAdd(&s_W[iu * 32 + lane], u * help * du);
-      // unclamped elements from the shell's sums over elements (ff_sum_kernel):
-      // S = sum z^2 fr gff, dS/dT through the table row (du) and column (dgg)
-      const double* Sv = A.ffsum + (size_t)i * FF_NU;
-      const double* Dv = A.ffdsum + (size_t)i * FF_NU;
-      const double s0 = Sv[iu - 1], s1 = Sv[iu];
-      double S = (1.0 - du) * s0 + du * s1;
-      double dS = (s1 - s0) * dru + ((1.0 - du) * Dv[iu - 1] + du * Dv[iu]) * drgg;
-      // elements under the gff >= 1 clamp, one by one
-      const double* nfr = A.natomfr + (size_t)(A.nelem + 1) * i;
-      for (unsigned m = A.ffclamp_all[i]; m; m &= m - 1) {
-        const int iz = __ffs(m);
-        const double fr = nfr[iz];
-        const int igg = -A.ffigg[(size_t)(iz - 1) * A.nc + i];
-        const double dgg = A.ffdgg[(size_t)(iz - 1) * A.nc + i];
-        const double* G = A.gff;
-        const double g00 = G[(iu - 1) + FF_NU * (igg - 1)], g10 = G[iu + FF_NU * (igg - 1)];
-        const double g01 = G[(iu - 1) + FF_NU * igg], g11 = G[iu + FF_NU * igg];
-        const double graw = (1.0 - du) * (1.0 - dgg) * g00 + du * (1.0 - dgg) * g10 + (1.0 - du) * dgg * g01 +
-                            du * dgg * g11;
-        const bool flat = graw < 1.0;
-        const double g = flat ? 1.0 : graw;
-        const double dg = flat ? 0.0
-                               : ((1.0 - dgg) * (g10 - g00) + dgg * (g11 - g01)) * dru +
-                                     ((1.0 - du) * (g01 - g00) + du * (g11 - g10)) * drgg;
-        const double w = (double)(iz * iz);
-        atomicAdd(&s_fr[iz * 32 + lane], u * help * g * w);
-        if (fr == 0.0) continue;
-        S = S + g * w * fr;
-        dS = dS + dg * w * fr;
+      double eh[FS], ue[FS], sbb[FS], schi[FS];
+#pragma unroll
+      for (int s = 0; s < FS; ++s) {
+        eh[s] = exp(-(h[s] * wlinv));
+        ue[s] = u[s] != 0.0 ? u[s] * (1.0 - eh[s]) : 0.0;
       }
-      gh = gh + u * hn * S;
-      gt = gt + u * (help * S * dlnhelp + help * dS);
+      if (inrange)
+        bb_adjoint<FS, true>(A.lt + l0, n, h, arg, C, ue, pop, A.ld, B.ggrnd + ii[0], A.nc, etab, mine, sbb,
+                             schi);
+      else
+        bb_adjoint<FS, false>(A.lt + l0, n, h, arg, C, ue, pop, A.ld, B.ggrnd + ii[0], A.nc, etab, mine,
+                              sbb, schi);
+#pragma unroll
+      for (int s = 0; s < FS; ++s) {
+        if (u[s] == 0.0) continue;
+        const double expfac = 1.0 - eh[s], T = A.temp[ii[s]];
+        // h = hc/kT: d exp(-chi h)/dT = chi h/T exp(..), d expfac/dT = -(h/T) wlinv eh
+        gt[s] = gt[s] + u[s] * ((h[s] / T) * (schi[s] * expfac) - sbb[s] * expfac * (h[s] / T) * wlinv * eh[s] / expfac);
+      }
+    }
+    if (!A.noff) {
+#pragma unroll
+      for (int s = 0; s < FS; ++s) {
+        if (u[s] == 0.0) continue;
+        const double2 g = ff_adjoint(A, B, ii[s], ig, h[s], u[s]);
+        gt[s] = gt[s] + g.x;
+        gh[s] = gh[s] + g.y;
+      }
     }
   }
-  s_t[warp * 32 + lane] = gt;
-  s_h[warp * 32 + lane] = gh;
-  __syncthreads();
-  if (warp == 0 && i < A.nc) {
-    double a = 0.0, b = 0.0;
-    for (int w = 0; w < OPAC_GT; ++w) {
-      a += s_t[w * 32 + lane];
-      b += s_h[w * 32 + lane];
-    }
-    if (a != 0.0) atomicAdd(&B.gT[i], a);
-    if (b != 0.0) atomicAdd(&B.ghlp[i], b);
-  }
-  for (int k = threadIdx.x; k < ntot; k += blockDim.x) {
-    const double v = sm[k];
-    const int row = k >> 5, c = blockIdx.x * OPAC_CT + (k & 31);
-    if (v == 0.0 || c >= A.nc) continue;
-    if (row < FF_NU) atomicAdd(&B.W[(size_t)c * FF_NU + row], v);
-    else if (row < FF_NU + nacc) atomicAdd(&B.ggrnd[(size_t)A.slot_of_lrow[row - FF_NU] * A.nc + c], v);
-    else atomicAdd(&B.gfr[(size_t)c * (A.nelem + 1) + (row - FF_NU - nacc)], v);
+#pragma unroll
+  for (int s = 0; s < FS; ++s) {
+    if (gt[s] != 0.0) atomicAdd(&B.gT[ii[s]], gt[s]);
+    if (gh[s] != 0.0) atomicAdd(&B.ghlp[ii[s]], gh[s]);
   }
 }
 
@@ -1125,17 +1081,13 @@ __global__ void __launch_bounds__(OPAC_GT * 32, 4) opacity_bwd_kernel(const Opac
 // holds shell tx and slots ty, ty + 8, ty + 16, ty + 24.  Runs after
 // opacity_bwd_kernel and before opac_cell_bwd_kernel (one writer per entry).
 constexpr int BFB_T = 32;
-// shells from which the forward takes four shells per lane
-constexpr int kFwdFourShellsMin = 2048;
 // d cap(g, i) / d fr(z, i) = help(g, i) z^2 gff_z(g, i) for the elements
 // without the gff >= 1 clamp, where gff_z = (1 - du_g) Gz[iu_g - 1] + du_g
 // Gz[iu_g] is linear in the table-row weights: sum_g u_g help_g gff_z =
 // sum_j W[j] Gz[j] with W[j] the row weights of all groups, weighted by
-// u_g help_g (u = dL/dcap).  opacity_bwd_kernel gathers W per block in shared
-// memory and adds its nonzero entries (a block's eight groups touch a few rows
-// per shell), ff_fr_bwd_kernel adds
-// z^2 sum_j W[j] Gz[j] to gfr (after opacity_bwd_kernel, which adds the
-// clamped elements).
+// u_g help_g (u = dL/dcap).  opacity_bwd_kernel gathers W, ff_fr_bwd_kernel adds
+// z^2 sum_j W[j] Gz[j] to gfr (after opacity_bwd_kernel, which adds the clamped
+// elements).
 __global__ void ff_fr_bwd_kernel(const OpacArgs A, const double* __restrict__ W, double* __restrict__ gfr) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)A.nc * A.nelem) return;
@@ -1144,16 +1096,11 @@ __global__ void ff_fr_bwd_kernel(const OpacArgs A, const double* __restrict__ W,
   if (igg < 0) return;  // clamped: opacity_bwd_kernel
   const double dgg = A.ffdgg[(size_t)(iz - 1) * A.nc + i];
   const double* G = A.gff;
-  const double* w = W + (size_t)i * FF_NU;
   double acc = 0.0;
-  for (int j = 0; j < FF_NU; ++j) acc = acc + w[j] * ((1.0 - dgg) * G[j + FF_NU * (igg - 1)] + dgg * G[j + FF_NU * igg]);
+  for (int j = 0; j < FF_NU; ++j) acc = acc + W[(size_t)j * A.nc + i] * ((1.0 - dgg) * G[j + FF_NU * (igg - 1)] + dgg * G[j + FF_NU * igg]);
   gfr[(size_t)i * (A.nelem + 1) + iz] += (double)(iz * iz) * acc;
 }
 
-// population rows x shells from which the adjoint accumulates d/d(population)
-// in global memory: measured on B200, shared accumulators won at 40 rows x 256
-// shells and global reductions at 40 rows x 4096 shells
-constexpr size_t kBwdGlobalAccMin = 32768;
 __global__ void __launch_bounds__(BFB_T * 8) bf_bwd_kernel(const OpacArgs A, const OpacBwd B) {
   __shared__ double su[BFB_T][BFB_T + 1];  // [shell][group]
   __shared__ double sx[BFB_T][BFB_T + 1];  // [group][slot]
@@ -1170,7 +1117,7 @@ __global__ void __launch_bounds__(BFB_T * 8) bf_bwd_kernel(const OpacArgs A, con
     for (int k = threadIdx.x; k < BFB_T * BFB_T; k += blockDim.x) {
       const int r = k >> 5, q = k & 31;  // sx: group r, slot q
       const int gr = g0 + r, a = a0 + q;
-      const double x = (gr < A.ng && a < nact) ? A.xstab[(size_t)gr * A.maxact + a] : 0.0;
+      const double x = (gr < A.ng && a < nact) ? A.xstab[(size_t)gr * A.maxact + A.act_slot[a]] : 0.0;
       sx[r][q] = x;
       nz = nz || x != 0.0;
     }
@@ -1241,35 +1188,90 @@ __global__ void opac_cell_bwd_kernel(int nc, int nelem, int nst, const int32_t* 
 }  // namespace
 
 // ============================================================ launchers
-// One launch of opacity_fwd_kernel on the stream.  Shells per lane: 4 on large
-// grids (each line record serves four terms; measured on B200 at 4096 shells:
-// 11.2 against 11.7 ms), 2 where four would leave too few blocks for the SMs
-// (256 shells: 0.39 against 0.41 ms) or too many staged rows.  The block's
-// population rows are staged in shared memory up to 80 KB of them (beyond,
-// the kernel reads grndlev); the kernel's dynamic limit is raised on the
-// device before its first staged launch (with its static arrays a block
-// passes the default 48 KB from about 77 rows at 2 shells per lane).
+// One launch of opacity_fwd_kernel on the stream.  Two shells per lane, one where
+// that leaves lanes without a shell (measured on B200: 77 shells x 333 groups of
+// three sub-groups 16 against 19 us, 32 x 100 148 against 154 us a host call;
+// from 128 shells on two: 256 x 2000 178 against 265 us); four hold too many
+// registers for the warps they leave (256 x 2000 214 us, 4096 x 10000 9.23
+// against 8.86 ms).
 static int launch_fwd(slg_ctx* ctx, OpacArgs& A) {
-  const size_t rows4 = sizeof(double) * 4 * OPAC_CT * (size_t)A.nlrow;
-  const bool four = A.nc >= kFwdFourShellsMin && (A.nobb || A.nlrow == 0 || rows4 <= 80 * 1024);
-  const int fs = four ? 4 : 2;
-  const size_t b = sizeof(double) * fs * OPAC_CT * (size_t)A.nlrow;
-  A.stage_rows = (!A.nobb && A.nlrow > 0 && b <= 80 * 1024) ? 1 : 0;
-  const size_t shm = A.stage_rows ? b : 0;
-  static unsigned raised[2] = {0, 0};  // per device and form
-  const dim3 grid((A.nc + fs * OPAC_CT - 1) / (fs * OPAC_CT), (A.ng + OPAC_GT - 1) / OPAC_GT);
-  if (four) {
-    raise_smem_limit(raised[1], ctx->device, opacity_fwd_kernel<4>, 80 * 1024);
-    opacity_fwd_kernel<4><<<grid, OPAC_GT * 32, shm, ctx->stream>>>(A);
-  } else {
-    raise_smem_limit(raised[0], ctx->device, opacity_fwd_kernel<2>, 80 * 1024);
-    opacity_fwd_kernel<2><<<grid, OPAC_GT * 32, shm, ctx->stream>>>(A);
-  }
+  const int fs = A.nc < 128 ? 1 : 2;
+  const int tiles = (A.nc + fs * OPAC_CT - 1) / (fs * OPAC_CT), warps = tiles < kOpacWarps ? tiles : kOpacWarps;
+  const int gpb = A.nc < 1024 ? 1 : 4;
+  const dim3 grid((A.ng + gpb - 1) / gpb, (tiles + warps - 1) / warps);
+  if (fs == 2) opacity_fwd_kernel<2><<<grid, warps * 32, 0, ctx->stream>>>(A, ExpConst{}, gpb);
+  else opacity_fwd_kernel<1><<<grid, warps * 32, 0, ctx->stream>>>(A, ExpConst{}, gpb);
   return cuda_check(ctx, cudaGetLastError(), "opacity_fwd launch");
 }
 
-// Everything the opacity kernels read, queued on the stream: sub-group edges,
-// the line binning, per-cell terms (and gas_sig) and the bound-free table.
+// What the build needs of the groups, the line list and the bound-free fits
+// alone, for ngs sub-groups per group: laid out on the first call after
+// slg_set_groups or slg_set_atomic_data (or for another ngs) and kept, like the
+// atomic data, until the next.  While a graph is being captured or held the
+// layout is queued with every call, so that each graph lays out what its own
+// calls read.
+static int opacity_plan(slg_ctx* ctx, int ngs, bool need_bb, bool need_bf, OpacArgs& A) {
+  const int ngsub = ctx->ng * ngs, nslot = ctx->nelem * ctx->nstage, nst = ctx->nstage;
+  const int nedge = ngsub + 1, nedge_pad = (nedge + 1) & ~1;
+  cudaStream_t st = ctx->stream;
+  if (ctx->plan_ngs != ngs) ctx->plan_edges = ctx->plan_bb = ctx->plan_bf = false;
+  const bool keep = !ctx->capturing && !ctx->graph_exec;
+  if (!keep) ctx->plan_edges = ctx->plan_bb = ctx->plan_bf = false;
+  double* d_wlsub = (double*)scratch(ctx, 0, sizeof(double) * nedge_pad);
+  if (!d_wlsub) return SLG_ERR_OOM;
+  if (!ctx->plan_edges)
+    wlsub_kernel<<<(nedge_pad + 255) / 256, 256, 0, st>>>(ctx->ng, ngs, nedge_pad, ctx->d_wl, d_wlsub);
+  A.wlsub = d_wlsub;
+  A.lstart = nullptr;
+  A.lt = nullptr;
+  if (need_bb) {
+    if (ngsub > kMaxLineSubgroups)
+      return set_error(ctx, SLG_ERR_ARG, "too many sub-groups for line binning (%d)", ngsub);
+    int* d_lstart = (int*)scratch(ctx, 2, sizeof(int) * (nedge + 3));
+    // one record past the last is loaded ahead
+    LineTerm* d_lt = (LineTerm*)scratch(ctx, 84, sizeof(LineTerm) * ((size_t)ctx->nline + 2));
+    if (!d_lstart || !d_lt) return SLG_ERR_OOM;
+    if (!ctx->plan_bb) {
+      line_range_kernel<<<(nedge + 2 + 127) / 128, 128, 0, st>>>(ctx->d_bb, ctx->nline, d_wlsub, nedge, d_lstart);
+      // lines outside the groups, and past the last, are never used but may be loaded
+      cudaMemsetAsync(d_lt, 0, sizeof(LineTerm) * ((size_t)ctx->nline + 2), st);
+      const size_t shm = sizeof(int) * LT_WARPS * (size_t)ctx->nlrow;  // at most 30 x 64 rows: 30 KB
+      line_terms_kernel<<<(ngsub + LT_WARPS - 1) / LT_WARPS, LT_WARPS * 32, shm, st>>>(
+          ctx->d_bb, d_lstart, ngsub, d_wlsub, nst, ctx->d_lrow_of_slot, ctx->nlrow, d_lt);
+    }
+    A.lstart = d_lstart;
+    A.lt = d_lt;
+  }
+  A.xstab = nullptr;
+  A.bf = nullptr;
+  A.bnnz = nullptr;
+  if (need_bf) {
+    const size_t n = (size_t)ngsub * nslot;
+    double* d_xs = (double*)scratch(ctx, 11, sizeof(double) * n);
+    BfTerm* d_terms = (BfTerm*)scratch(ctx, 86, sizeof(BfTerm) * n);
+    int* d_cnt = (int*)scratch(ctx, 87, sizeof(int) * (size_t)ngsub);
+    if (!d_xs || !d_terms || !d_cnt) return SLG_ERR_OOM;
+    if (!ctx->plan_bf) {
+      bf_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ngsub, nslot, ctx->d_ion_ni, nst, d_wlsub,
+                                                                   ctx->d_ph1, ctx->d_ph2, d_xs);
+      bf_compact_kernel<<<(ngsub + 7) / 8, 256, 0, st>>>(ngsub, nslot, d_xs, d_terms, d_cnt);
+    }
+    A.xstab = d_xs;
+    A.bf = d_terms;
+    A.bnnz = d_cnt;
+  }
+  const int rc = cuda_check(ctx, cudaGetLastError(), "opacity plan launch");
+  if (!rc && keep) {
+    ctx->plan_ngs = ngs;
+    ctx->plan_edges = true;
+    ctx->plan_bb = ctx->plan_bb || need_bb;
+    ctx->plan_bf = ctx->plan_bf || need_bf;
+  }
+  return rc;
+}
+
+// Everything the opacity kernels read, queued on the stream: the plan, the
+// per-cell terms (and gas_sig) and the populated ions' bound-free terms.
 static int opacity_prepare(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_flags* flags, double* gas_sig,
                            OpacArgs& A) {
   const int nc = ctx->nx, ng = ctx->ng;
@@ -1279,94 +1281,51 @@ static int opacity_prepare(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_f
   const int nslot = nelem * nst;
   cudaStream_t st = ctx->stream;
   if (nelem <= 0) return set_error(ctx, SLG_ERR_STATE, "atomic data not set");
-  const int nedge = ngsub + 1, nedge_pad = (nedge + 1) & ~1;
-  double* d_wlsub = (double*)scratch(ctx, 0, sizeof(double) * nedge_pad);
-  unsigned int* d_counts = (unsigned int*)scratch(ctx, 1, sizeof(unsigned int) * (nedge + 2));
-  int* d_lstart = (int*)scratch(ctx, 2, sizeof(int) * (nedge + 3));
-  int* d_flags = (int*)scratch(ctx, 3, sizeof(int) * 4);
+  const bool do_bb = ctx->nline > 0 && !flags->nobb, do_bf = !flags->nobf;
+  const bool do_ff = !flags->noff && ctx->d_gff;
+  int rc = opacity_plan(ctx, ngs, do_bb, do_bf, A);
+  if (rc) return rc;
+  int* d_flags = (int*)scratch(ctx, 3, sizeof(int) * (4 + nslot));  // sanity word, then the active slots
   double* d_hckt = (double*)scratch(ctx, 4, sizeof(double) * nc);
   double* d_hlp = (double*)scratch(ctx, 5, sizeof(double) * nc);
-  double* d_grnd = (double*)scratch(ctx, 6, sizeof(double) * (size_t)nc * nslot);
+  const int ld = (nc + kRun - 1) / kRun * kRun;
+  double* d_grnd = (double*)scratch(ctx, 6, sizeof(double) * 2 * (size_t)ld * nslot);
+  double* d_ocp = d_grnd + (size_t)ld * nslot;
   int* d_ffigg = (int*)scratch(ctx, 7, sizeof(int) * (size_t)nc * nelem);
   double* d_ffdgg = (double*)scratch(ctx, 8, sizeof(double) * (size_t)nc * nelem);
-  int* d_active = (int*)scratch(ctx, 9, sizeof(int) * (nslot + 1));
-  int16_t* d_act = (int16_t*)scratch(ctx, 10, sizeof(int16_t) * nslot);
-  double* d_xs = (double*)scratch(ctx, 11, sizeof(double) * (size_t)ngsub * nslot);
-  if (!d_wlsub || !d_counts || !d_lstart || !d_flags || !d_hckt || !d_hlp || !d_grnd || !d_ffigg ||
-      !d_ffdgg || !d_active || !d_act || !d_xs)
-    return SLG_ERR_OOM;
-  int* d_nact = d_active + nslot;
-  cudaMemsetAsync(d_counts, 0, sizeof(unsigned int) * (nedge + 2), st);
-  cudaMemsetAsync(d_flags, 0, sizeof(int) * 4, st);
-  cudaMemsetAsync(d_active, 0, sizeof(int) * (nslot + 1), st);
-  wlsub_kernel<<<(nedge_pad + 255) / 256, 256, 0, st>>>(ng, ngs, nedge_pad, ctx->d_wl, d_wlsub);
-  const bool do_bb = ctx->nline > 0 && !flags->nobb;
-  LineTerm* d_lt = nullptr;
-  if (do_bb) {
-    const size_t shm = 16 + sizeof(double) * nedge_pad + sizeof(unsigned int) * (nedge + 1);
-    if (shm > 220 * 1024)
-      return set_error(ctx, SLG_ERR_ARG, "too many sub-groups for line binning (%d)", ngsub);
-    static unsigned raised = 0;  // per device; no attribute calls on repeated launches
-    raise_smem_limit(raised, ctx->device, bin_lines_kernel, 220 * 1024);
-    const int64_t per_block = 256 * 8;
-    const int nb = (int)((ctx->nline + per_block - 1) / per_block);
-    bin_lines_kernel<<<nb, 256, shm, st>>>(ctx->d_bb, ctx->nline, d_wlsub, nedge, nedge_pad, d_counts,
-                                           d_flags);
-    scan_counts_kernel<<<1, 1024, 0, st>>>(d_counts, nedge + 1, d_lstart);
-    d_lt = (LineTerm*)scratch(ctx, 84, sizeof(LineTerm) * (size_t)ctx->nline);
-    if (!d_lt) return SLG_ERR_OOM;
-    decode_lines_kernel<<<(unsigned)((ctx->nline + 255) / 256), 256, 0, st>>>(
-        ctx->d_bb, ctx->nline, d_lstart, ngsub, d_wlsub, nst, ctx->d_lrow_of_slot, d_lt);
-  } else {
-    cudaMemsetAsync(d_lstart, 0, sizeof(int) * (nedge + 3), st);
-  }
-  opac_cell_prep_kernel<<<dim3((nc + 127) / 128, nelem), 128, 0, st>>>(
-      nc, nelem, nst, ctx->d_ion_ni, gas->temp, gas->natom, gas->nelec, gas->vol, gas->mass, gas->oc,
-      gas->ginv, flags->nothmson, d_hckt, gas_sig, d_hlp, d_grnd, d_ffigg, d_ffdgg);
-  double *d_ffsum = nullptr, *d_ffdsum = nullptr;
-  unsigned* d_ffclamp = nullptr;
-  if (!flags->noff && ctx->d_gff) {
-    d_ffsum = (double*)scratch(ctx, 88, sizeof(double) * 2 * (size_t)nc * FF_NU);
-    d_ffclamp = (unsigned*)scratch(ctx, 89, sizeof(unsigned) * 2 * (size_t)nc);
-    if (!d_ffsum || !d_ffclamp) return SLG_ERR_OOM;
-    d_ffdsum = d_ffsum + (size_t)nc * FF_NU;
-    const int64_t nt = (int64_t)nc * FF_NU;
-    ff_sum_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(nc, nelem, gas->natomfr, d_ffigg, d_ffdgg,
-                                                                ctx->d_gff, d_ffsum, d_ffdsum, d_ffclamp,
-                                                                d_ffclamp + nc);
-  }
-  const bool do_bf = !flags->nobf;
-  double* d_xsc = nullptr;
-  int *d_bslot = nullptr, *d_bnnz = nullptr;
+  double* d_ffsum = (double*)scratch(ctx, 88, sizeof(double) * 2 * (size_t)nc * FF_NU);
+  unsigned* d_ffclamp = (unsigned*)scratch(ctx, 89, sizeof(unsigned) * 2 * (size_t)nc);
+  if (!d_flags || !d_hckt || !d_hlp || !d_grnd || !d_ffigg || !d_ffdgg || !d_ffsum || !d_ffclamp) return SLG_ERR_OOM;
+  int* d_active = d_flags + 4;
+  cudaMemsetAsync(d_flags, 0, sizeof(int) * (4 + nslot), st);
+  double* d_ffdsum = d_ffsum + (size_t)nc * FF_NU;
+  opac_cell_kernel<<<(ld + CELLS - 1) / CELLS, CELLS * 32, 0, st>>>(
+      nc, nelem, nst, ctx->d_ion_ni, gas->temp, gas->natom, gas->nelec, gas->vol, gas->mass, gas->oc, gas->ginv,
+      flags->nothmson, gas->natomfr, do_ff ? ctx->d_gff : nullptr, d_hckt, gas_sig, d_hlp, ld, d_grnd, d_ocp, d_active, d_ffigg,
+      d_ffdgg, d_ffsum, d_ffdsum, d_ffclamp, d_ffclamp + nc);
   if (do_bf) {
-    dim3 ga((nc + 255) / 256 < 8 ? (nc + 255) / 256 : 8, nslot);
-    ion_active_kernel<<<ga, 256, 0, st>>>(nc, gas->oc, d_active);
-    ion_compact_kernel<<<1, 32, 0, st>>>(nelem, nst, ctx->d_ion_ni, d_active, d_act, d_nact);
-    const int64_t nt = (int64_t)ngsub * nslot;
-    bf_table_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(ngsub, nslot, d_nact, d_act, nst, d_wlsub,
-                                                                  ctx->d_ph1, ctx->d_ph2, d_xs);
-    d_xsc = (double*)scratch(ctx, 85, sizeof(double) * (size_t)ngsub * nslot);
-    d_bslot = (int*)scratch(ctx, 86, sizeof(int) * (size_t)ngsub * nslot);
-    d_bnnz = (int*)scratch(ctx, 87, sizeof(int) * (size_t)ngsub);
-    if (!d_xsc || !d_bslot || !d_bnnz) return SLG_ERR_OOM;
-    bf_compact_kernel<<<(ngsub + 7) / 8, 256, 0, st>>>(ngsub, nslot, d_nact, d_act, d_xs, d_xsc, d_bslot, d_bnnz);
+    BfTerm* d_bf = (BfTerm*)scratch(ctx, 9, sizeof(BfTerm) * (size_t)ngsub * nslot);
+    int* d_nbf = (int*)scratch(ctx, 1, sizeof(int) * (size_t)ngsub);
+    if (!d_bf || !d_nbf) return SLG_ERR_OOM;
+    bf_select_kernel<<<(ngsub + 7) / 8, 256, 0, st>>>(ngsub, nslot, A.bf, A.bnnz, d_active, d_bf, d_nbf);
+    A.bf = d_bf;
+    A.bnnz = d_nbf;
   }
   A.nc = nc; A.ng = ng; A.ngs = ngs; A.ngsub = ngsub; A.nelem = nelem; A.nst = nst; A.maxact = nslot;
-  A.pnact = d_nact;
+  A.pnact = nullptr;
   A.nobb = !do_bb; A.nobf = !do_bf; A.noff = flags->noff;
   A.mix = flags->opacmixrossel;
-  A.wlsub = d_wlsub; A.grp_wl = ctx->d_wl; A.lstart = d_lstart; A.bb = ctx->d_bb;
-  A.lt = d_lt; A.chimax = ctx->line_chimax; A.slot_of_lrow = ctx->d_slot_of_lrow; A.nlrow = ctx->nlrow;
-  A.grndlev = d_grnd; A.oc = gas->oc; A.act_slot = d_act; A.xstab = d_xs;
-  A.xsc = d_xsc; A.bslot = d_bslot; A.bnnz = d_bnnz;
+  A.grp_wl = ctx->d_wl;
+  A.chimax = ctx->line_chimax;
+  A.ld = ld; A.ocp = d_ocp;
+  A.grndlev = d_grnd; A.oc = gas->oc; A.active = d_active; A.act_slot = nullptr;
   A.hckt = d_hckt; A.hlparr = d_hlp; A.mass = gas->mass; A.natomfr = gas->natomfr; A.temp = gas->temp;
   A.ffigg = d_ffigg; A.ffdgg = d_ffdgg; A.gff = ctx->d_gff;
-  A.ffsum = d_ffsum; A.ffdsum = d_ffdsum; A.ffclamp = d_ffclamp;
-  A.ffclamp_all = d_ffclamp ? d_ffclamp + nc : nullptr;
+  A.ffsum = d_ffsum; A.ffdsum = d_ffdsum; A.ffclamp = d_ffclamp; A.ffclamp_all = d_ffclamp + nc;
   A.ffc1 = ff_c1a * sqrt(ff_c1b);
   A.cap32 = nullptr; A.emiss32 = nullptr; A.cap64 = nullptr; A.capg64 = nullptr; A.flags = d_flags;
   if (!ctx->d_gff && !A.noff) return set_error(ctx, SLG_ERR_STATE, "free-free table not set");
-  return SLG_OK;
+  return cuda_check(ctx, cudaGetLastError(), "opacity preparation launch");
 }
 
 int launch_physical_opacity(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_flags* flags,
@@ -1422,28 +1381,27 @@ int launch_opacity_bwd(slg_ctx* ctx, const slg_gas* gas, const double* gcap, con
   cudaMemsetAsync(gfr, 0, sizeof(double) * (size_t)nc * (A.nelem + 1), st);
   double* W = nullptr;
   if (!A.noff) {
-    W = (double*)scratch(ctx, 90, sizeof(double) * ((size_t)nc * FF_NU + 1));
+    W = (double*)scratch(ctx, 90, sizeof(double) * (size_t)nc * FF_NU);
     if (!W) return SLG_ERR_OOM;
-    cudaMemsetAsync(W, 0, sizeof(double) * ((size_t)nc * FF_NU + 1), st);
+    cudaMemsetAsync(W, 0, sizeof(double) * (size_t)nc * FF_NU, st);
   }
   OpacBwd B{gcap, gT, ggrnd, goc, ghlp, gfr, W};
-  // d/d(population) accumulated in global memory when that array (rows x
-  // shells) is large, in shared memory otherwise (bb_adjoint_staged)
-  // (and where the shared accumulators would not fit in a block's shared memory)
-  auto bwd_smem = [&](bool g) {
-    return sizeof(double) * ((size_t)(FF_NU + (g ? 1 : 2) * A.nlrow + A.nelem + 1) * 32 + 2 * OPAC_GT * 32);
-  };
-  const bool gred = (size_t)A.nlrow * nc >= kBwdGlobalAccMin || bwd_smem(false) > 200 * 1024;
-  const size_t shm = bwd_smem(gred);
-  if (shm > 200 * 1024) return set_error(ctx, SLG_ERR_ARG, "opacity adjoint: too many ion slots (%d)", A.nlrow);
-  static unsigned raised[2] = {0, 0};  // per device and form (with the static table, before 48 KB)
-  if (gred) raise_smem_limit(raised[1], ctx->device, opacity_bwd_kernel<true>, 200 * 1024);
-  else raise_smem_limit(raised[0], ctx->device, opacity_bwd_kernel<false>, 200 * 1024);
-  dim3 grid((nc + OPAC_CT - 1) / OPAC_CT, (A.ng + OPAC_GT - 1) / OPAC_GT);
-  if (gred)
-    opacity_bwd_kernel<true><<<grid, OPAC_GT * 32, shm, st>>>(A, B);
-  else
-    opacity_bwd_kernel<false><<<grid, OPAC_GT * 32, shm, st>>>(A, B);
+  // the active slots, for the bound-free product
+  int16_t* d_act = (int16_t*)scratch(ctx, 10, sizeof(int16_t) * (size_t)nslot);
+  int* d_nact = (int*)scratch(ctx, 85, sizeof(int));
+  if (!d_act || !d_nact) return SLG_ERR_OOM;
+  ion_compact_kernel<<<1, 32, 0, st>>>(A.nelem, A.nst, ctx->d_ion_ni, A.active, d_act, d_nact);
+  A.act_slot = d_act;
+  A.pnact = d_nact;
+  // two shells per lane and several groups per block where that leaves blocks
+  // enough (whole adjoint calls on B200: 4096 x 10000 17.2 ms with two, 18.0 with
+  // one; 256 x 2000 0.57 ms with one shell and one group, 0.59 with two shells,
+  // 0.62 with four groups)
+  const int fs = nc < 1024 ? 1 : 2, gpb = nc < 1024 ? 1 : 8;
+  const int tiles = (nc + fs * OPAC_CT - 1) / (fs * OPAC_CT), warps = tiles < kOpacWarps ? tiles : kOpacWarps;
+  const dim3 grid((A.ng + gpb - 1) / gpb, (tiles + warps - 1) / warps);
+  if (fs == 2) opacity_bwd_kernel<2><<<grid, warps * 32, 0, st>>>(A, B, ExpConst{}, gpb);
+  else opacity_bwd_kernel<1><<<grid, warps * 32, 0, st>>>(A, B, ExpConst{}, gpb);
   if (!A.noff) {
     const int64_t nf = (int64_t)nc * A.nelem;
     ff_fr_bwd_kernel<<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(A, W, gfr);
@@ -1458,17 +1416,15 @@ int launch_opacity_bwd(slg_ctx* ctx, const slg_gas* gas, const double* gcap, con
   return cuda_check(ctx, cudaGetLastError(), "opacity adjoint launch");
 }
 
-// Sanity bitmask of physical_opacity.f:282-291 (word 0) and line-binning
-// errors (word 1: 1 unsorted lines, 2 shared-memory staging time-out).
-int opacity_flags(slg_ctx* ctx, int32_t* sanity, int32_t* binning) {
+// Sanity bitmask of physical_opacity.f:282-291.
+int opacity_flags(slg_ctx* ctx, int32_t* sanity) {
   int* d_flags = (int*)scratch(ctx, 3, sizeof(int) * 4);
-  int h[2] = {0, 0};
-  int rc = cuda_check(ctx, cudaMemcpyAsync(h, d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream),
+  int h = 0;
+  int rc = cuda_check(ctx, cudaMemcpyAsync(&h, d_flags, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream),
                       "flags download");
   if (rc) return rc;
   if ((rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "flags sync"))) return rc;
-  if (sanity) *sanity = h[0];
-  if (binning) *binning = h[1];
+  if (sanity) *sanity = h;
   return SLG_OK;
 }
 

@@ -10,7 +10,7 @@
 // The host entry point times one launch with CUDA events on a private stream.
 //
 // slg_exp_eval evaluates the opacity kernels' table-driven FP64 exp
-// (exp_tang, slg_device.cuh) on given arguments, for accuracy tests.
+// (exp_scaled, slg_device.cuh) on given arguments, for accuracy tests.
 #include <cuda_runtime.h>
 #include <cstdint>
 #include "slg.h"
@@ -79,12 +79,14 @@ __global__ void __launch_bounds__(PK_BLOCK) imad_kernel(int iters, uint32_t a, u
   out[(size_t)blockIdx.x * blockDim.x + threadIdx.x] = (double)s;
 }
 
-__global__ void exp_eval_kernel(int64_t n, const double* __restrict__ x, double* __restrict__ y) {
-  __shared__ double tab[slg::kExpTabN];
-  slg::exp_table_load(tab);
+__global__ void exp_eval_kernel(int64_t n, const double* __restrict__ x, double* __restrict__ y,
+                                const slg::ExpConst C) {
+  __shared__ double tab[slg::kExpTabN * slg::kExpCopies];
+  slg::exp_table_spread(tab);
   __syncthreads();
+  const uint32_t mine = slg::exp_table_mine();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = slg::exp_tang(x[i], tab);
+    y[i] = fabs(x[i]) <= 700.0 ? slg::exp_scaled(1.0, slg::exp_arg(-x[i]), C, tab, mine) : exp(x[i]);  // also NaN
 }
 
 }  // namespace
@@ -114,7 +116,7 @@ extern "C" int slg_exp_eval(int device, int64_t n, const double* x, double* y) {
   if (cudaMemcpy(d, x, sizeof(double) * n, cudaMemcpyHostToDevice) != cudaSuccess) rc = SLG_ERR_CUDA;
   if (!rc) {
     const int64_t nb = (n + 255) / 256;
-    exp_eval_kernel<<<(unsigned)(nb < 4096 ? nb : 4096), 256>>>(n, d, d + n);
+    exp_eval_kernel<<<(unsigned)(nb < 4096 ? nb : 4096), 256>>>(n, d, d + n, slg::ExpConst{});
     if (cudaGetLastError() != cudaSuccess ||
         cudaMemcpy(y, d + n, sizeof(double) * n, cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = SLG_ERR_CUDA;

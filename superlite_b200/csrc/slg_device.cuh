@@ -41,22 +41,19 @@ constexpr double c2c = pc_c * pc_c;
 constexpr double c4c = c2c * c2c;
 constexpr double cthomson = 8.0 * pc_pi * e4c / (3.0 * (pc_me * pc_me) * c4c);  // physical_opacity.f:51
 
-// ---- exp(x) by Tang's table-driven method (P. T. P. Tang, "Table-driven
+// ---- exp by Tang's table-driven method (P. T. P. Tang, "Table-driven
 // implementation of the exponential function in IEEE floating-point
 // arithmetic", ACM TOMS 15 (1989) 144-157), for the opacity build's inner
 // loops, whose one exp per line-shell term is their binding work:
-//   x = (64 m + j) ln2/64 + r,  |r| <= ln2/128,  exp(x) = 2^m 2^(j/64) e^r,
-// with ln2/64 split in a 36-bit head (so that n * head is exact for |n| <
-// 2^17) and its remainder, e^r - 1 by its Taylor polynomial of degree 5
-// (truncation below 4e-17 relative), 2^(j/64) from a 64-entry table and 2^m
-// added to the exponent field.  Arguments outside [-700, 700] go to exp().
-// The constants and the table are the output of csrc/exp_table.py.  (A
-// 256-entry table with a degree-4 polynomial saves one FMA per exp but was
-// slower in the opacity kernels: its shared-memory lookups conflict more.)
+//   x = (64 m + j + f) ln2/64,  |f| <= 1/2,  exp(x) = 2^m 2^(j/64) 2^(f/64),
+// 2^(j/64) from a 64-entry table and 2^(f/64) - 1 by its Taylor polynomial of
+// degree 5 (truncation below 4e-17 relative), in the form exp(-chi h) with one h
+// for many chi, chi in single precision.  The constants and the table are the
+// output of csrc/exp_table.py.  (A 256-entry table with a degree-4 polynomial
+// saves one FMA per exp but was slower in the opacity kernels.)
 constexpr int kExpTabN = 64;
-constexpr double kExpInvL = 92.33248261689366;        // 64 / ln 2
-constexpr double kExpL1 = 0.010830424696223417;       // ln2/64, 36 significant bits
-constexpr double kExpL2 = 2.572804622327669e-14;      // ln2/64 - kExpL1
+constexpr double kExpInvL = 92.33248261689366;           // 64 / ln 2
+constexpr double kExpInvLLo = 1.3027375194195861e-15;    // 64 / ln 2 - kExpInvL
 // 2^(j/64), j = 0..63, correctly rounded
 static __constant__ double kExp2Tab[kExpTabN] = {
     1.0, 1.0108892860517005, 1.0218971486541166, 1.0330248790212284,
@@ -77,37 +74,59 @@ static __constant__ double kExp2Tab[kExpTabN] = {
     1.9152065613971474, 1.9360617934922943, 1.9571441241754002, 1.978456026387951,
 };
 
-// Copies kExp2Tab into a block's shared array of kExpTabN doubles (call from
-// every thread, then __syncthreads()).
-__device__ inline void exp_table_load(double* s_tab) {
-  for (int k = threadIdx.x; k < kExpTabN; k += blockDim.x) s_tab[k] = kExp2Tab[k];
+// The division of chi h by ln2/64 is made once per h, in two parts (ExpArg), so
+// that n = 64 m + j (the nearest integer of -chi h 64/ln2, by adding and taking
+// off 1.5 2^52: the low 32 bits of that sum are n) and f come from one fused
+// multiply-add each and f's second part from another.  The
+// table is spread over kExpCopies interleaved copies, one per bank pair of a
+// half warp, so that no lookup conflicts (random lookups of one copy took about
+// six wavefronts), with j << 14 taken off entry j's high word: adding n << 14 to
+// it then scales by 2^m and takes the entry's j off again, in one integer
+// operation.  The constants come as a kernel argument (ExpConst), which FP64
+// instructions read as an operand; as literals they cost moves in the loop.
+// Eleven FP64 operations with the caller's multiply-add.  Valid for chi h in
+// [-700, 700] (not checked).
+struct ExpArg {
+  double hi, lo;  // -h 64/ln2
+};
+constexpr int kExpCopies = 16;                         // one per bank pair of a half warp
+struct ExpConst {
+  double round = 6755399441055744.0;  // 1.5 * 2^52
+  // (ln2/64)^k / k!
+  double c1 = 0.010830424696249145, c2 = 5.86490495505617e-05, c3 = 2.1173137155464776e-07,
+         c4 = 5.732851688640402e-10, c5 = 1.2417843701716925e-12;
+};
+__device__ __forceinline__ ExpArg exp_arg(double h) {
+  const double hi = -h * kExpInvL;
+  return ExpArg{hi, fma(-h, kExpInvLLo, fma(-h, kExpInvL, -hi))};
 }
-
-// tab: kExp2Tab in shared memory.  n = nearest integer of x 64/ln2 by the
-// add-and-subtract of 1.5 2^52 (|x 64/ln2| < 2^31, so the sum's low 32 bits
-// are n in two's complement and the difference is n exactly).  This form
-// requires x in [-700, 700] and does not check it: the result's exponent
-// field is formed by an integer add, valid for normal results only.
-__device__ __forceinline__ double exp_tang_inrange(double x, const double* tab) {
-  constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
-  const double big = fma(x, kExpInvL, kRound);
-  const int ni = (int)__double2loint(big);
-  const double n = big - kRound;
-  double r = fma(-n, kExpL1, x);
-  r = fma(-n, kExpL2, r);
-  double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
-  p = fma(r, p, 1.0 / 6.0);
-  p = fma(r, p, 0.5);
-  p = fma(r, p, 1.0);
-  p = p * r;  // e^r - 1
-  const double s = tab[ni & (kExpTabN - 1)];
-  const double v = fma(s, p, s);  // in [0.99, 2): adding m to the exponent field stays normal
-  return __hiloint2double(__double2hiint(v) + (ni >> 6) * (1 << 20), __double2loint(v));
+// mine: the byte offset (exp_table_mine) of the caller's copy in s_tab.
+__device__ __forceinline__ double exp_scaled(double chi, const ExpArg& a, const ExpConst& C, const double* s_tab,
+                                             uint32_t mine) {
+  const double big = fma(chi, a.hi, C.round);
+  const uint32_t ni = (uint32_t)__double2loint(big);
+  const double n = big - C.round;
+  const double f = fma(chi, a.lo, fma(chi, a.hi, -n));
+  double p = fma(f, C.c5, C.c4);
+  p = fma(f, p, C.c3);
+  p = fma(f, p, C.c2);
+  p = fma(f, p, C.c1);
+  p = p * f;
+  constexpr uint32_t kMask = 8u * kExpCopies * (kExpTabN - 1);
+  const double t = *reinterpret_cast<const double*>(reinterpret_cast<const char*>(s_tab) +
+                                                    (((ni * (8u * kExpCopies)) & kMask) | mine));
+  const double s = __hiloint2double((int)((uint32_t)__double2hiint(t) + (ni << 14)), __double2loint(t));
+  return fma(s, p, s);
 }
-// Any x: outside [-700, 700], and for NaN, CUDA's exp.
-__device__ inline double exp_tang(double x, const double* tab) {
-  if (!(fabs(x) <= 700.0)) return exp(x);  // also NaN
-  return exp_tang_inrange(x, tab);
+__device__ __forceinline__ uint32_t exp_table_mine() { return (threadIdx.x & (kExpCopies - 1)) * 8u; }
+// Fills a block's spread table (kExpTabN * kExpCopies doubles; call from every
+// thread, then __syncthreads()).
+__device__ inline void exp_table_spread(double* s_tab) {
+  for (int k = threadIdx.x; k < kExpTabN * kExpCopies; k += blockDim.x) {
+    const int j = k / kExpCopies;
+    const double t = kExp2Tab[j];
+    s_tab[k] = __hiloint2double(__double2hiint(t) - (j << 14), __double2loint(t));
+  }
 }
 constexpr double ff_c1a = 4.0 * e6c / (3.0 * pc_h * pc_me * c4c);              // physical_opacity.f:32
 constexpr double ff_c1b = pc_pi2 / (3.0 * pc_me * pc_h * pc_c);                 // argument of its sqrt

@@ -178,11 +178,10 @@ struct slg_ctx {
   std::vector<int32_t> h_ion_ni;
   slg_bbxs* d_bb = nullptr;
   // population rows (slot = (iz-1) nstage + ii-1) that the lines reference:
-  // d_lrow_of_slot[slot] = compact row or -1, d_slot_of_lrow[row] = slot
+  // d_lrow_of_slot[slot] = compact row or -1
   int nlrow = 0;
   double line_chimax = 0.0;  // largest chilw of the lines (infinite if any is negative or NaN)
   int16_t* d_lrow_of_slot = nullptr;
-  int16_t* d_slot_of_lrow = nullptr;
   float* d_ph1 = nullptr;
   float* d_ph2 = nullptr;
   double* d_gff = nullptr;
@@ -199,6 +198,9 @@ struct slg_ctx {
   // derived per-call scratch
   slg::DevBuf scratch[128];
   slg::CellTables tables;
+  // opacity_plan's layouts that are in place (for plan_ngs sub-groups)
+  int plan_ngs = 0;
+  bool plan_edges = false, plan_bb = false, plan_bf = false;
   slg::TransportAcc* d_acc = nullptr;
   slg::TransportAcc* h_acc = nullptr;  // pinned
   // optional trace (host arrays) for the next particle_advance call
