@@ -66,158 +66,151 @@ __device__ inline LeakArgsT<CT> leak_view(LeakArgsT<CT> A, int c, int* i) {
   return A;
 }
 
-// leakage_opacity11.f90:30-171, one block per cell.  Sums are fixed-shape
-// tree reductions (the reference sums sequentially).
-template <class CT>
-__global__ void __launch_bounds__(GB) leakage_kernel(const LeakArgsT<CT> A0) {
-  __shared__ double sh[GB];
-  __shared__ double shv[GB];
-  __shared__ int shi[GB];
+// leakage_opacity11.f90:30-171, TPC threads per cell.  One pass over the groups:
+// one Planck weight per group and one division per face, the factors that the
+// terms of a sum share (speclump, x^2 / vterm, divv / 3c) taken out of it.  The sums
+// are fixed-shape tree reductions (the reference sums sequentially).  In four
+// passes that each formed the weight anew, with eight block-wide reductions and
+// a block per cell: 341 us at 28800 cells x 100 groups (now 72), 988 us at 4096 x 10000
+// in FP64 (640).
+template <class CT, int TPC>
+__global__ void __launch_bounds__(GB) leakage_kernel(const LeakArgsT<CT> A0, int nc) {
+  __shared__ double sh[6 * (GB / 32)];
+  __shared__ double shv[GB / 32];
+  __shared__ int shi[GB / 32];
+  const int cell = blockIdx.x * (GB / TPC) + threadIdx.x / TPC, t = threadIdx.x % TPC;
+  if (cell >= nc) return;  // uniform over the cell's threads
   int i0;
-  const LeakArgsT<CT> A = leak_view(A0, blockIdx.x, &i0);
+  const LeakArgsT<CT> A = leak_view(A0, cell, &i0);
   const int i = i0;  // 1-based cell
   const int l = i, ng = A.ng;
-  const double* X = A.xarr - 1;  // 1-based view
-  auto dx = [&](int k) { return A.xarr[k] - A.xarr[k - 1]; };
+  const double Xa = A.xarr[i - 1], Xb = A.xarr[i];
   const CT* capl = A.cap + (size_t)(l - 1) * ng;
   const double sigl = A.sig[l - 1];
-  const double dist = dx(i);
+  const double dist = Xb - Xa;
   const double tinv = A.tempinv[l - 1];
   const double hct = hck * tinv;
   const double divv = A.divv[l - 1];
-  const int icnb1 = max(i - 1, 1), icnb2 = min(i + 1, A.nx);
-  auto lumpable = [&](int ig) {
-    const double c = (double)capl[ig - 1];
-    return c * dist >= A.taulump && (sigl + c) * dist >= A.tauddmc;
-  };
-  // speclump
-  double s = 0.0;
-  for (int ig = threadIdx.x + 1; ig <= ng; ig += GB)
-    if (lumpable(ig)) s = s + specintv_elem(hct, A.wlinv, ig - 1);
-  double speclump = block_sum(s, sh);
-  speclump = speclump > 0.0 ? 1.0 / speclump : 0.0;
-  // caplump, capemitlump, igemitmax (first strict maximum over loop 1 then loop 2)
-  double cl = 0.0, cel = 0.0, bestv = 0.0;
+  const bool in = i > 1, out = i < A.nx;  // a neighbour inside, outside
+  const CT* cap1 = in ? capl - ng : capl;
+  const CT* cap2 = out ? capl + ng : capl;
+  const double sig1 = in ? A.sig[l - 2] : 0.0, sig2 = out ? A.sig[l] : 0.0;
+  const double dx1 = in ? Xa - A.xarr[i - 2] : 0.0, dx2 = out ? A.xarr[i + 1] - Xb : 0.0;
+  // sums: speclump, caplump, capemitlump, leakage left and right, doplump
+  double a[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  double bestv = 0.0;
   int besto = 0x7fffffff;
-  for (int ig = threadIdx.x + 1; ig <= ng; ig += GB) {
-    if (!lumpable(ig)) continue;
-    const double sv = specintv_elem(hct, A.wlinv, ig - 1);
-    const double h1 = sv * (double)capl[ig - 1];
-    cl = cl + h1;
-    if (h1 > bestv || (h1 == bestv && h1 > 0.0 && ig < besto)) { bestv = h1; besto = ig; }
-    const double h2 = A.capemit ? sv * (double)A.capemit[(size_t)(l - 1) * ng + ig - 1] : 0.0;
-    cel = cel + h2;
-    if (h2 > bestv) { bestv = h2; besto = ng + ig; }
-  }
-  const double caplump = block_sum(cl, sh);
-  const double capemitlump = block_sum(cel, sh);
-  shv[threadIdx.x] = bestv;
-  shi[threadIdx.x] = besto;
-  __syncthreads();
-  for (int w = GB / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      const double v2 = shv[threadIdx.x + w];
-      const int o2 = shi[threadIdx.x + w];
-      if (v2 > shv[threadIdx.x] || (v2 == shv[threadIdx.x] && o2 < shi[threadIdx.x])) {
-        shv[threadIdx.x] = v2;
-        shi[threadIdx.x] = o2;
+  for (int ig = t + 1; ig <= ng; ig += TPC) {
+    const double c = (double)capl[ig - 1];
+    const double tau = (sigl + c) * dist;
+    if (c * dist >= A.taulump && tau >= A.tauddmc) {
+      const double sv = specintv_elem(hct, A.wlinv, ig - 1);
+      a[0] = a[0] + sv;
+      // caplump, capemitlump, igemitmax (first strict maximum over loop 1 then loop 2)
+      const double h1 = sv * c;
+      a[1] = a[1] + h1;
+      if (h1 > bestv || (h1 == bestv && h1 > 0.0 && ig < besto)) { bestv = h1; besto = ig; }
+      const double h2 = A.capemit ? sv * (double)A.capemit[(size_t)(l - 1) * ng + ig - 1] : 0.0;
+      a[2] = a[2] + h2;
+      if (h2 > bestv) { bestv = h2; besto = ng + ig; }
+      // leakage: 1.5 * 4 / (3 tau + 6 dext) at a face to IMC, 2 / (tau + tau') inside
+      const double tau1 = in ? ((double)cap1[ig - 1] + sig1) * dx1 : 0.0;
+      const bool imc1 = !in || tau1 < A.tauddmc;
+      a[3] = a[3] + sv * ((imc1 ? 6.0 : 2.0) / (imc1 ? 3.0 * tau + 6.0 * pc_dext : tau + tau1));
+      const double tau2 = out ? ((double)cap2[ig - 1] + sig2) * dx2 : 0.0;
+      const bool imc2 = !out || tau2 < A.tauddmc;
+      a[4] = a[4] + sv * ((imc2 ? 6.0 : 2.0) / (imc2 ? 3.0 * tau + 6.0 * pc_dext : tau + tau2));
+    }
+    // doplump: a thick group whose next one (previous, for divv < 0) is not
+    if (!(c * dist < A.taulump) && !(tau < A.tauddmc)) {
+      if (divv >= 0.0) {
+        if (ig < ng && !((double)capl[ig] * dist >= A.taulump)) a[5] = a[5] + dopspeccalc(tinv, A.wlinv, ig);
+      } else {
+        if (ig > 1 && !((double)capl[ig - 2] * dist >= A.taulump)) a[5] = a[5] - dopspeccalc(tinv, A.wlinv, ig - 1);
       }
     }
+  }
+  cell_sum<TPC, 6>(a, sh);
+  auto better = [](double v2, int o2, double& v, int& o) {
+    if (v2 > v || (v2 == v && o2 < o)) {
+      v = v2;
+      o = o2;
+    }
+  };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    better(__shfl_xor_sync(0xffffffffu, bestv, o), __shfl_xor_sync(0xffffffffu, besto, o), bestv, besto);
+  if (TPC > 32) {
+    if ((threadIdx.x & 31) == 0) {
+      shv[threadIdx.x >> 5] = bestv;
+      shi[threadIdx.x >> 5] = besto;
+    }
     __syncthreads();
+    if (t == 0)
+      for (int w = 1; w < GB / 32; ++w) better(shv[w], shi[w], bestv, besto);
   }
-  int igemitmax = 0;
-  if (shv[0] > 0.0) igemitmax = shi[0] > ng ? shi[0] - ng : shi[0];
-  __syncthreads();
-  // doplump
-  double dl = 0.0;
-  if (divv >= 0.0) {
-    for (int ig = threadIdx.x + 1; ig <= ng - 1; ig += GB) {
-      if ((double)capl[ig - 1] * dist < A.taulump) continue;
-      if ((double)capl[ig] * dist >= A.taulump) continue;
-      if ((sigl + (double)capl[ig - 1]) * dist < A.tauddmc) continue;
-      dl = dl + dopspeccalc(tinv, A.wlinv, ig) * divv / (3.0 * pc_c);
-    }
-  } else {
-    for (int ig = threadIdx.x + 2; ig <= ng; ig += GB) {
-      if ((double)capl[ig - 1] * dist < A.taulump) continue;
-      if ((double)capl[ig - 2] * dist >= A.taulump) continue;
-      if ((sigl + (double)capl[ig - 1]) * dist < A.tauddmc) continue;
-      dl = dl - dopspeccalc(tinv, A.wlinv, ig - 1) * divv / (3.0 * pc_c);
-    }
-  }
-  const double doplump = block_sum(dl, sh);
-  // leakage opacities
-  const double vterm = 3.0 * A.vol[l - 1] / pc_pi4;
-  double o1 = 0.0, o2 = 0.0;
-  for (int ig = threadIdx.x + 1; ig <= ng; ig += GB) {
-    if (!lumpable(ig)) continue;
-    const double specval = specintv_elem(hct, A.wlinv, ig - 1);
-    const double cap_l = (double)capl[ig - 1];
-    bool lhelp;
-    if (i == 1) lhelp = true;
-    else lhelp = ((double)A.cap[(size_t)(icnb1 - 1) * ng + ig - 1] + A.sig[icnb1 - 1]) * dx(i - 1) < A.tauddmc;
-    if (lhelp) {
-      const double help = (cap_l + sigl) * dx(i);
-      const double ppl = 4.0 / (3.0 * help + 6.0 * pc_dext);
-      o1 = o1 + (specval * speclump) * 1.5 * ppl * sq(X[i]) / vterm;
-    } else {
-      const double help = (sigl + cap_l) * dx(i) +
-                          (A.sig[icnb1 - 1] + (double)A.cap[(size_t)(icnb1 - 1) * ng + ig - 1]) * dx(i - 1);
-      o1 = o1 + (specval * speclump) * 2.0 * sq(X[i]) / (help * 3.0 * A.vol[l - 1] / pc_pi4);
-    }
-    if (i == A.nx) lhelp = true;
-    else lhelp = ((double)A.cap[(size_t)(icnb2 - 1) * ng + ig - 1] + A.sig[icnb2 - 1]) * dx(i + 1) < A.tauddmc;
-    if (lhelp) {
-      const double help = (cap_l + sigl) * dx(i);
-      const double ppr = 4.0 / (3.0 * help + 6.0 * pc_dext);
-      o2 = o2 + (specval * speclump) * 1.5 * ppr * sq(X[i + 1]) / vterm;
-    } else {
-      const double help = (sigl + cap_l) * dx(i) +
-                          (A.sig[icnb2 - 1] + (double)A.cap[(size_t)(icnb2 - 1) * ng + ig - 1]) * dx(i + 1);
-      o2 = o2 + (specval * speclump) * 2.0 * sq(X[i + 1]) / (help * 3.0 * A.vol[l - 1] / pc_pi4);
-    }
-  }
-  const double ol1 = block_sum(o1, sh);
-  const double ol2 = block_sum(o2, sh);
-  if (threadIdx.x == 0) {
+  if (t == 0) {
+    const double speclump = a[0] > 0.0 ? 1.0 / a[0] : 0.0;
+    const double vterm = 3.0 * A.vol[l - 1] / pc_pi4;
+    int igemitmax = 0;
+    if (bestv > 0.0) igemitmax = besto > ng ? besto - ng : besto;
     double* ol = A.opaclump + (size_t)11 * (l - 1);
-    ol[0] = ol1;
-    ol[1] = ol2;
+    ol[0] = a[3] * speclump * (sq(Xa) / vterm);
+    ol[1] = a[4] * speclump * (sq(Xb) / vterm);
     ol[2] = 0.0; ol[3] = 0.0; ol[4] = 0.0; ol[5] = 0.0;
     ol[6] = speclump;
-    ol[7] = caplump;
-    ol[8] = capemitlump;
+    ol[7] = a[1];
+    ol[8] = a[2];
     ol[9] = (double)igemitmax;
-    ol[10] = doplump;
+    ol[10] = a[5] * divv / (3.0 * pc_c);
   }
 }
 
 // emission_probability.f90:40-63: bin sums are sequential within a bin (one
-// thread per bin) and the running sum over bins is sequential (thread 0), as in
-// the reference.
-__global__ void __launch_bounds__(GB) emitprob_kernel(int ng, int nep, int nepg, const double* __restrict__ tempinv,
+// thread per bin) and the running sum over bins is sequential (one thread), as
+// in the reference.  The terms are formed by all TPC threads of a cell first,
+// bins_per_tile whole bins at a time, in shared memory (tile doubles per cell,
+// then nep for the bin sums); with a thread per bin forming its own terms most
+// of a block idled: 91 us at 28800 cells x 100 groups (now 25), 55 us at 1001 x 4003
+// (35).
+template <int TPC>
+__global__ void __launch_bounds__(GB) emitprob_kernel(int nc, int ng, int nep, int nepg, int bins_per_tile,
+                                                      const double* __restrict__ tempinv,
                                                       const float* __restrict__ cap,
                                                       const double* __restrict__ capgrey,
                                                       const double* __restrict__ wlinv,
                                                       double* __restrict__ emitprob) {
-  extern __shared__ double binsum[];
-  const int l = blockIdx.x;
+  extern __shared__ double s_dyn[];
+  const int tile = bins_per_tile * nepg;
+  double* const term = s_dyn + (size_t)(threadIdx.x / TPC) * (tile + nep);
+  double* const binsum = term + tile;
+  const int l = blockIdx.x * (GB / TPC) + threadIdx.x / TPC, t = threadIdx.x % TPC;
+  if (l >= nc) return;  // uniform over the cell's threads
   double* ep = emitprob + (size_t)nep * l;
   if (ng == 1) {
-    if (threadIdx.x == 0) ep[0] = capgrey[l];
+    if (t == 0) ep[0] = capgrey[l];
     return;
   }
+  auto sync = [] {
+    if (TPC == 32) __syncwarp();
+    else __syncthreads();
+  };
   const double hct = hck * tempinv[l];
   const float* capl = cap + (size_t)l * ng;
-  for (int iep = threadIdx.x + 1; iep <= nep - 1; iep += blockDim.x) {
-    const int ig = (iep - 1) * nepg + 1;
-    const int top = min(iep * nepg, ng);
-    double s = 0.0;
-    for (int g = ig; g <= top; ++g) s = s + specintv_elem(hct, wlinv, g - 1) * (double)capl[g - 1];
-    binsum[iep - 1] = s;
+  for (int b0 = 0; b0 < nep - 1; b0 += bins_per_tile) {
+    const int g0 = b0 * nepg, n = min(min(b0 + bins_per_tile, nep - 1) * nepg, ng) - g0;
+    sync();
+    for (int k = t; k < n; k += TPC) term[k] = specintv_elem(hct, wlinv, g0 + k) * (double)capl[g0 + k];
+    sync();
+    for (int b = b0 + t; b < min(b0 + bins_per_tile, nep - 1); b += TPC) {
+      double s = 0.0;
+      const int top = min((b + 1) * nepg, ng) - g0;
+      for (int k = b * nepg - g0; k < top; ++k) s = s + term[k];
+      binsum[b] = s;
+    }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  sync();
+  if (t == 0) {
     double help = 0.0;
     for (int iep = 1; iep <= nep - 1; ++iep) {
       help = help + binsum[iep - 1];
@@ -227,17 +220,22 @@ __global__ void __launch_bounds__(GB) emitprob_kernel(int ng, int nep, int nepg,
   }
 }
 
-// d/dT of specintv_elem and dopspeccalc (groupmod.f:123-143, :189-198) at
-// temperature T: x = hc/(lambda k T) scales as 1/T; zero where x is clamped.
-__device__ inline double dspec_dT(double hct, double T, const double* __restrict__ wlinv, int g0) {
+// specintv_elem and its d/dT, from one exp, and the d/dT of dopspeccalc
+// (groupmod.f:123-143, :189-198) at temperature T: x = hc/(lambda k T) scales as
+// 1/T; zero derivative where x is clamped.
+__device__ inline double spec_dT(double hct, double Tinv, const double* __restrict__ wlinv, int g0, double& dT) {
   const double x1 = hct * wlinv[g0], x2 = hct * wlinv[g0 + 1];
   const double xm = 0.5 * (x2 + x1), ax = fabs(x2 - x1);
-  double dfp = 0.0;
-  if (xm < 300.0) {
-    const double ex = exp(xm), d = ex - 1.0;
-    dfp = 3.0 * sq(xm) / d - cube(xm) * ex / sq(d);
+  double fp, dfp = 0.0;
+  if (xm >= 300.0) {
+    fp = fplanck(xm);
+  } else {
+    const double ex = exp(xm), dinv = 1.0 / (ex - 1.0);
+    fp = cube(xm) * dinv;
+    dfp = (3.0 * sq(xm) - fp * ex) * dinv;
   }
-  return -(ftpi4 * ax * (fplanck(xm) + xm * dfp)) / T;
+  dT = -(ftpi4 * ax * (fp + xm * dfp)) * Tinv;
+  return ftpi4 * ax * fp;
 }
 __device__ inline double ddop_dT(double tinv, const double* __restrict__ wlinv, int ig) {
   const double x = hck * tinv * wlinv[ig];
@@ -259,7 +257,7 @@ __global__ void __launch_bounds__(GB, 4) leakage_bwd_kernel(const LeakArgsT<doub
   const double* capl = A.cap + (size_t)(i - 1) * ng;
   const double sigl = A.sig[i - 1];
   const double dist = dx(i);
-  const double tinv = A.tempinv[i - 1], T = 1.0 / tinv;
+  const double tinv = A.tempinv[i - 1];
   const double hct = hck * tinv;
   const double divv = A.divv[i - 1];
   const double* ol = A.opaclump + (size_t)11 * (i - 1);
@@ -271,7 +269,8 @@ __global__ void __launch_bounds__(GB, 4) leakage_bwd_kernel(const LeakArgsT<doub
   for (int ig = threadIdx.x + 1; ig <= ng; ig += GB) {
     const double cg = capl[ig - 1];
     if (!(cg * dist >= A.taulump && (sigl + cg) * dist >= A.tauddmc)) continue;
-    const double sv = specintv_elem(hct, A.wlinv, ig - 1);
+    double dsv;
+    const double sv = spec_dT(hct, tinv, A.wlinv, ig - 1, dsv);
     // left leakage term a and d a / d(opacity sum) of this cell (da) and the left one (dal)
     double a, da, dal = 0.0;
     const bool lint = i != 1 && (A.cap[(size_t)(i - 2) * ng + ig - 1] + A.sig[i - 2]) * dx(i - 1) >= A.tauddmc;
@@ -300,7 +299,7 @@ __global__ void __launch_bounds__(GB, 4) leakage_bwd_kernel(const LeakArgsT<doub
     // ol1 = sum w_g a_g with w_g = sv_g speclump and speclump = 1/sum sv: d ol1/d sv_g = speclump (a_g - ol1)
     const double ua = u1 * sv * speclump, ub = u2 * sv * speclump;
     const double us = u1 * speclump * (a - ol1) + u2 * speclump * (b - ol2) - u7 * speclump * speclump + u8 * cg;
-    gt += us * dspec_dT(hct, T, A.wlinv, ig - 1);
+    gt += us * dsv;
     atomicAdd(&gcap[(size_t)c * ng + ig - 1], u8 * sv + ua * da + ub * db);
     gs += ua * da + ub * db;
     if (lint) {
@@ -637,15 +636,19 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
     }
   }
   if (A.fp64 && A.T.fine) {
+    // a thread per limit k / fm (exact: fm is a power of two): the number of
+    // entries not above it is the end of range k - 1 and the start of range k
     const int fm = A.T.fine_m;
     short2* fd = A.T.fine + (size_t)(ic - 1) * kFineTables * fm;
+    auto limit = [&](int t, int k, int n) {
+      if (k < fm) fd[t * fm + k].x = (short)n;
+      if (k > 0) fd[t * fm + k - 1].y = (short)n;
+    };
     if (nlump > 0) {
       for (int t = 0; t < 4; ++t) {
         const CdfEntry* a = t == 0 ? cdop : (t == 1 ? cleft : (t == 2 ? cright : cscat));
-        const int n = t == 1 && ix == 1 ? 0 : (t == 3 ? ng - nlump : nlump);
-        for (int k = threadIdx.x; k < fm; k += blockDim.x)  // k / fm is exact: fm is a power of two
-          fd[t * fm + k] = make_short2((short)count_le(a, n, (double)k / (double)fm),
-                                       (short)count_le(a, n, (double)(k + 1) / (double)fm));
+        const int n = t == 1 && ix == 1 ? 0 : (t == 3 ? ng - nlump : nlump);  // no left leak from the first shell
+        for (int k = threadIdx.x; k <= fm; k += blockDim.x) limit(t, k, count_le(a, n, (double)k / (double)fm));
       }
     }
     // the emission thresholds against (k / fine_m) capgrey, rounded as a draw's
@@ -653,20 +656,15 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
     const int n = emit_last_group(A.nep, A.nepg, ng) - 1;
     const double cg = A.capgrey[ic - 1];
     const int one = emit_only_group(A.nep, A.nepg, ng, cg != cg);
-    for (int k = threadIdx.x; k < fm; k += blockDim.x) {
-      int r[2];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const double v = ((double)(k + j) / (double)fm) * cg;
-        int lo = 0, hi = n;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (ecum[mid] > v) hi = mid;
-          else lo = mid + 1;
-        }
-        r[j] = one ? one - 1 : lo;
+    for (int k = threadIdx.x; k <= fm; k += blockDim.x) {
+      const double v = ((double)k / (double)fm) * cg;
+      int lo = 0, hi = n;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (ecum[mid] > v) hi = mid;
+        else lo = mid + 1;
       }
-      fd[4 * fm + k] = make_short2((short)r[0], (short)r[1]);
+      limit(4, k, one ? one - 1 : lo);
     }
   }
 }
@@ -783,11 +781,20 @@ __global__ void __launch_bounds__(256) ddmc_rate_kernel(const TabArgs A0, int nc
 
 }  // namespace
 
+template <class CT>
+static void launch_leakage_kernel(slg_ctx* ctx, const LeakArgsT<CT>& A) {
+  const int nc = ctx->nx;
+  if (ctx->ng <= kWarpCellGroups)
+    leakage_kernel<CT, 32><<<(nc + GB / 32 - 1) / (GB / 32), GB, 0, ctx->stream>>>(A, nc);
+  else
+    leakage_kernel<CT, GB><<<nc, GB, 0, ctx->stream>>>(A, nc);
+}
+
 int launch_leakage(slg_ctx* ctx, const double* tempinv, const double* sig, const float* cap,
                    const float* capemit, double tauddmc, double taulump, double* opaclump) {
   LeakArgs A{ctx->nx, ctx->ng, ctx->d_xarr, ctx->d_vol, ctx->d_divv, tempinv, sig, ctx->d_wlinv,
              cap, capemit, tauddmc, taulump, opaclump, ctx->nmodel > 1 ? ctx->d_cellmap : nullptr};
-  leakage_kernel<float><<<ctx->nx, GB, 0, ctx->stream>>>(A);
+  launch_leakage_kernel(ctx, A);
   return cuda_check(ctx, cudaGetLastError(), "leakage launch");
 }
 
@@ -796,7 +803,7 @@ int launch_leakage64(slg_ctx* ctx, const double* tempinv, const double* sig, con
                      double taulump, double* opaclump) {
   LeakArgsT<double> A{ctx->nx, ctx->ng, ctx->d_xarr, ctx->d_vol, ctx->d_divv, tempinv, sig, ctx->d_wlinv,
                       cap, nullptr, tauddmc, taulump, opaclump, ctx->nmodel > 1 ? ctx->d_cellmap : nullptr};
-  leakage_kernel<double><<<ctx->nx, GB, 0, ctx->stream>>>(A);
+  launch_leakage_kernel(ctx, A);
   return cuda_check(ctx, cudaGetLastError(), "leakage64 launch");
 }
 
@@ -816,9 +823,18 @@ int launch_leakage64_bwd(slg_ctx* ctx, const double* tempinv, const double* sig,
 
 int launch_emitprob(slg_ctx* ctx, const double* tempinv, const float* cap, const double* capgrey,
                     double* emitprob) {
-  const size_t shm = sizeof(double) * (ctx->nep > 0 ? ctx->nep : 1);
-  emitprob_kernel<<<ctx->nx, 128, shm, ctx->stream>>>(ctx->ng, ctx->nep, ctx->nepg, tempinv, cap, capgrey,
-                                                      ctx->d_wlinv, emitprob);
+  // a tile: all bins of a cell where a warp takes it, else up to 4096 groups
+  // (nepg is at most 181 for the largest group count)
+  const int nc = ctx->nx, ng = ctx->ng, nep = ctx->nep, nepg = ctx->nepg;
+  const bool warp = ng <= kWarpCellGroups;
+  const int cells = warp ? GB / 32 : 1, bins = warp ? nep : (4096 / nepg < nep ? 4096 / nepg : nep);
+  const size_t shm = sizeof(double) * cells * ((size_t)bins * nepg + nep);  // at most 36 KB
+  if (warp)
+    emitprob_kernel<32><<<(nc + cells - 1) / cells, GB, shm, ctx->stream>>>(nc, ng, nep, nepg, bins, tempinv, cap,
+                                                                           capgrey, ctx->d_wlinv, emitprob);
+  else
+    emitprob_kernel<GB><<<nc, GB, shm, ctx->stream>>>(nc, ng, nep, nepg, bins, tempinv, cap, capgrey, ctx->d_wlinv,
+                                                     emitprob);
   return cuda_check(ctx, cudaGetLastError(), "emission_probability launch");
 }
 

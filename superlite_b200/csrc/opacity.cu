@@ -721,37 +721,36 @@ __global__ void analytic_opacity_kernel(int nc, int ng, const double* __restrict
 }
 
 // ------------------------------------------------------------ Planck / Rosseland means
-// One block per shell; a fixed-shape tree reduction over groups.
+// TPC threads per shell, both integrals' weights from one exp, a fixed-shape tree
+// reduction over groups.  CT: float (gas_cap) or double (the FP64 opacity of the
+// differentiable path), (ng, ncell).  With a block per shell, two exps per group
+// and a reduction
+// through nine block-wide steps: 103 us at 28800 shells x 100 groups (now 28), 303 us
+// at 4096 x 10000 in FP64 (227).
+template <class CT, int TPC>
 __global__ void __launch_bounds__(256) opacity_means_kernel(int nc, int ng, const double* __restrict__ wlinv,
                                                             const double* __restrict__ temp,
                                                             const double* __restrict__ sig,
-                                                            const float* __restrict__ cap,
-                                                            double* __restrict__ capgrey,
+                                                            const CT* __restrict__ cap, double* __restrict__ capgrey,
                                                             double* __restrict__ capross) {
-  __shared__ double sp[256], sr[256];
-  const int i = blockIdx.x;
+  __shared__ double sh[2 * 8];
+  const int i = blockIdx.x * (256 / TPC) + threadIdx.x / TPC, t = threadIdx.x % TPC;
+  if (i >= nc) return;  // uniform over the cell's threads
   const double tinv = 1.0 / temp[i];
   const double hct = hck * tinv;
   const double s = sig ? sig[i] : 0.0;
-  double ap = 0.0, ar = 0.0;
-  for (int g = threadIdx.x; g < ng; g += blockDim.x) {
+  double a[2] = {0.0, 0.0};
+  for (int g = t; g < ng; g += TPC) {
     const double c = (double)cap[(size_t)i * ng + g];
-    ap = ap + c * specintv_elem(hct, wlinv, g);
-    ar = ar + (1.0 / (s + c)) * spectintv_elem(hct, wlinv, g);
+    double w, wr;
+    spec_weights(hct, wlinv, g, w, wr);
+    a[0] = a[0] + c * w;
+    a[1] = a[1] + (1.0 / (s + c)) * wr;
   }
-  sp[threadIdx.x] = ap;
-  sr[threadIdx.x] = ar;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      sp[threadIdx.x] = sp[threadIdx.x] + sp[threadIdx.x + w];
-      sr[threadIdx.x] = sr[threadIdx.x] + sr[threadIdx.x + w];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    capgrey[i] = sp[0];
-    if (capross) capross[i] = 1.0 / sr[0];
+  cell_sum<TPC, 2>(a, sh);
+  if (t == 0) {
+    capgrey[i] = a[0];
+    if (capross) capross[i] = 1.0 / a[1];
   }
 }
 
@@ -787,40 +786,7 @@ __device__ inline void spec_weights_dT(double hct, double T, const double* __res
   dwr = bad ? 0.0 : -(ftpi4r * ax * (fr + xm * dfr)) / T;
 }
 
-// opacity_planckmean / opacity_rossmean on the FP64 opacity in (ng, ncell) layout.
-__global__ void __launch_bounds__(256) opacity_means64_kernel(int nc, int ng, const double* __restrict__ wlinv,
-                                                              const double* __restrict__ temp,
-                                                              const double* __restrict__ sig,
-                                                              const double* __restrict__ cap,
-                                                              double* __restrict__ capgrey,
-                                                              double* __restrict__ capross) {
-  __shared__ double sp[256], sr[256];
-  const int i = blockIdx.x;
-  const double hct = hck * (1.0 / temp[i]);
-  const double s = sig ? sig[i] : 0.0;
-  double ap = 0.0, ar = 0.0;
-  for (int g = threadIdx.x; g < ng; g += blockDim.x) {
-    const double c = cap[(size_t)i * ng + g];
-    ap = ap + c * specintv_elem(hct, wlinv, g);
-    ar = ar + (1.0 / (s + c)) * spectintv_elem(hct, wlinv, g);
-  }
-  sp[threadIdx.x] = ap;
-  sr[threadIdx.x] = ar;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      sp[threadIdx.x] = sp[threadIdx.x] + sp[threadIdx.x + w];
-      sr[threadIdx.x] = sr[threadIdx.x] + sr[threadIdx.x + w];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    capgrey[i] = sp[0];
-    capross[i] = 1.0 / sr[0];
-  }
-}
-
-// Adjoint of opacity_means64_kernel: adds to gcap (ng, ncell), gsig and gT.
+// Adjoint of opacity_means_kernel<double>: adds to gcap (ng, ncell), gsig and gT.
 __global__ void __launch_bounds__(256) means_bwd_kernel(int nc, int ng, const double* __restrict__ wlinv,
                                                         const double* __restrict__ temp,
                                                         const double* __restrict__ sig,
@@ -1078,8 +1044,12 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 4) opacity_bwd_kernel(const O
 // -- a product of the (shell, group) gradient with the (group, slot) table.
 // Tiled like a matrix product: a block computes 32 shells x 32 slots, staging
 // 32 groups of both operands in shared memory per round; thread (tx, ty)
-// holds shell tx and slots ty, ty + 8, ty + 16, ty + 24.  Runs after
-// opacity_bwd_kernel and before opac_cell_bwd_kernel (one writer per entry).
+// holds shell tx and slots ty, ty + 8, ty + 16, ty + 24.  The groups are split
+// over gridDim.z blocks, whose parts are added by atomics: on small grids a
+// block per (32 shells, 32 slots) left most SMs idle (256 x 2000: 72 blocks, 165
+// us; split
+// 21 us; 4096 x 10000: 737 -> 415 us).  Runs after opacity_bwd_kernel and before
+// opac_cell_bwd_kernel.
 constexpr int BFB_T = 32;
 // d cap(g, i) / d fr(z, i) = help(g, i) z^2 gff_z(g, i) for the elements
 // without the gff >= 1 clamp, where gff_z = (1 - du_g) Gz[iu_g - 1] + du_g
@@ -1091,7 +1061,7 @@ constexpr int BFB_T = 32;
 __global__ void ff_fr_bwd_kernel(const OpacArgs A, const double* __restrict__ W, double* __restrict__ gfr) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)A.nc * A.nelem) return;
-  const int i = (int)(t / A.nelem), iz = (int)(t % A.nelem) + 1;
+  const int i = (int)(t % A.nc), iz = (int)(t / A.nc) + 1;
   const int igg = A.ffigg[(size_t)(iz - 1) * A.nc + i];
   if (igg < 0) return;  // clamped: opacity_bwd_kernel
   const double dgg = A.ffdgg[(size_t)(iz - 1) * A.nc + i];
@@ -1110,7 +1080,9 @@ __global__ void __launch_bounds__(BFB_T * 8) bf_bwd_kernel(const OpacArgs A, con
   const int i0 = blockIdx.x * BFB_T;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int g0 = 0; g0 < A.ng; g0 += BFB_T) {
+  const int ntile = (A.ng + BFB_T - 1) / BFB_T;
+  const int t0 = (int)((long long)ntile * blockIdx.z / gridDim.z), t1 = (int)((long long)ntile * (blockIdx.z + 1) / gridDim.z);
+  for (int g0 = t0 * BFB_T; g0 < t1 * BFB_T; g0 += BFB_T) {
     // the cross sections first: most (group, slot) tiles lie beyond the slots'
     // ionisation edges, all zero, and are skipped (the forward skips xs = 0)
     bool nz = false;
@@ -1141,7 +1113,7 @@ __global__ void __launch_bounds__(BFB_T * 8) bf_bwd_kernel(const OpacArgs A, con
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int a = a0 + ty + 8 * j;
-    if (a < nact && acc[j] != 0.0) B.goc[(size_t)A.act_slot[a] * A.nc + i] += acc[j];  // xstab holds * pc_mbarn
+    if (a < nact && acc[j] != 0.0) atomicAdd(&B.goc[(size_t)A.act_slot[a] * A.nc + i], acc[j]);  // xstab holds * pc_mbarn
   }
 }
 
@@ -1349,10 +1321,20 @@ int launch_physical_opacity64(slg_ctx* ctx, const slg_gas* gas, double* gas_sig,
   return launch_fwd(ctx, A);
 }
 
+template <class CT>
+static void launch_means(slg_ctx* ctx, const double* temp, const double* sig, const CT* cap, double* capgrey,
+                         double* capross) {
+  const int nc = ctx->nx, ng = ctx->ng;
+  if (ng <= kWarpCellGroups)
+    opacity_means_kernel<CT, 32><<<(nc + 7) / 8, 256, 0, ctx->stream>>>(nc, ng, ctx->d_wlinv, temp, sig, cap, capgrey,
+                                                                       capross);
+  else
+    opacity_means_kernel<CT, 256><<<nc, 256, 0, ctx->stream>>>(nc, ng, ctx->d_wlinv, temp, sig, cap, capgrey, capross);
+}
+
 int launch_opacity_means64(slg_ctx* ctx, const double* temp, const double* sig, const double* cap,
                            double* capgrey, double* capross) {
-  opacity_means64_kernel<<<ctx->nx, 256, 0, ctx->stream>>>(ctx->nx, ctx->ng, ctx->d_wlinv, temp, sig, cap,
-                                                          capgrey, capross);
+  launch_means(ctx, temp, sig, cap, capgrey, capross);
   return cuda_check(ctx, cudaGetLastError(), "opacity_means64 launch");
 }
 
@@ -1407,7 +1389,12 @@ int launch_opacity_bwd(slg_ctx* ctx, const slg_gas* gas, const double* gcap, con
     ff_fr_bwd_kernel<<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(A, W, gfr);
   }
   if (!A.nobf) {
-    const dim3 bgrid((nc + BFB_T - 1) / BFB_T, (A.maxact + BFB_T - 1) / BFB_T);
+    // about four blocks per SM over the slot tiles that a third of the slots fill
+    // (the populated ones are known on the device only), of four tiles at least
+    const int bx = (nc + BFB_T - 1) / BFB_T, by = (A.maxact + BFB_T - 1) / BFB_T;
+    const int want = (4 * ctx->num_sms + bx * ((by + 2) / 3) - 1) / (bx * ((by + 2) / 3));
+    const int most = (A.ng + 4 * BFB_T - 1) / (4 * BFB_T);
+    const dim3 bgrid(bx, by, want < 1 ? 1 : want > most ? most : want);
     bf_bwd_kernel<<<bgrid, BFB_T * 8, 0, st>>>(A, B);
   }
   opac_cell_bwd_kernel<<<dim3((nc + 127) / 128, A.nelem), 128, 0, st>>>(nc, A.nelem, A.nst, ctx->d_ion_ni, gas->natom, gas->nelec,
@@ -1439,8 +1426,7 @@ int launch_analytic_opacity(slg_ctx* ctx, const double* temp, const double* rho,
 
 int launch_opacity_means(slg_ctx* ctx, const double* temp, const double* sig, const float* cap,
                          double* capgrey, double* capross) {
-  opacity_means_kernel<<<ctx->nx, 256, 0, ctx->stream>>>(ctx->nx, ctx->ng, ctx->d_wlinv, temp, sig, cap,
-                                                        capgrey, capross);
+  launch_means(ctx, temp, sig, cap, capgrey, capross);
   return cuda_check(ctx, cudaGetLastError(), "opacity_means launch");
 }
 

@@ -218,6 +218,46 @@ __device__ inline double spectintv_elem(double hct, const double* __restrict__ w
   return s != s ? 0.0 : s;  // groupmod.f:390-392
 }
 
+// specintv_elem and spectintv_elem of one group (the same values) from one exp.
+__device__ inline void spec_weights(double hct, const double* __restrict__ wlinv, int g0, double& w, double& wr) {
+  const double x1 = hct * wlinv[g0], x2 = hct * wlinv[g0 + 1];
+  const double xm = 0.5 * (x2 + x1), ax = fabs(x2 - x1);
+  double fp, fr;
+  if (xm >= 300.0) {
+    fp = fplanck(xm);
+    fr = fross(xm);
+  } else {
+    const double ex = exp(xm), d = ex - 1.0;
+    fp = cube(xm) / d;
+    fr = (pow4(xm) * ex) / sq(d);
+  }
+  w = ftpi4 * ax * fp;
+  const double s = ftpi4r * ax * fr;
+  wr = s != s ? 0.0 : s;  // groupmod.f:390-392
+}
+
+// Sums over the TPC threads (32: a warp; else the whole block) that share a
+// cell; every thread gets them.  sh: N * TPC / 32 doubles of the block (TPC > 32).
+template <int TPC, int N>
+__device__ inline void cell_sum(double* v, double* sh) {
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] = v[k] + __shfl_xor_sync(0xffffffffu, v[k], o);
+  if (TPC == 32) return;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < N; ++k) sh[k * (TPC / 32) + (threadIdx.x >> 5)] = v[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    v[k] = sh[k * (TPC / 32)];
+#pragma unroll
+    for (int w = 1; w < TPC / 32; ++w) v[k] = v[k] + sh[k * (TPC / 32) + w];
+  }
+}
+
 // physconstmod.f:79-93
 __device__ inline double planck(double wl, double temp) {
   double b = 1.0 / (wl * temp);

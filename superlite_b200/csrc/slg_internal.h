@@ -252,6 +252,11 @@ int set_error(slg_ctx* ctx, int code, const char* fmt, ...);
 int cuda_check(slg_ctx* ctx, cudaError_t e, const char* what);
 void* scratch(slg_ctx* ctx, int slot, size_t bytes);  // nullptr on failure (error set)
 
+// Threads that share a cell in the kernels that sum over a cell's groups: a warp
+// up to this many groups (eight cells per block, no block-wide steps), else a
+// block of 256.
+constexpr int kWarpCellGroups = 512;
+
 // kernels launch wrappers (return SLG_OK or error)
 int launch_physical_opacity(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_flags* flags,
                             double* gas_sig, float* gas_cap, float* gas_emiss, double* cap64);
