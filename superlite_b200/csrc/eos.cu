@@ -39,6 +39,14 @@ struct EosArgs {
   int* flags;      // bit 1: a cell where the reference stops (invalid sum, nelec <= 0)
 };
 
+// Sum of v over the lanes z < nelem in element order.
+__device__ inline double element_sum(double v, int nelem) {
+  double s = 0.0;
+#pragma unroll 6
+  for (int z = 0; z < nelem; ++z) s = s + __shfl_sync(0xffffffffu, v, z);
+  return s;
+}
+
 __global__ void __launch_bounds__(EOS_BLOCK) saha_eos_kernel(const EosArgs A) {
   const int lane = threadIdx.x & 31;
   const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -53,7 +61,11 @@ __global__ void __launch_bounds__(EOS_BLOCK) saha_eos_kernel(const EosArgs A) {
   const double ndens = A.natom[i] / A.vol[i];
   const double kti = 1.0 / (pc_kb * T);
   const double sahac = pow(pc_pi2 * pc_me * pc_kb * T / (pc_h * pc_h), 1.5);
-  double n[EOS_MAXST];
+  // exp(-e/kT) of every stage, once: the iterations share them (evaluated in
+  // each: 95 us at 4096 cells; 78 us so, bound by the FP64 divisions and the
+  // chain of stages)
+  double n[EOS_MAXST], ex[EOS_MAXST];
+  for (int ii = 0; ii < nion - 1; ++ii) ex[ii] = exp(-kti * e[ii]);
   double nel = A.nelec[i];
   double nec_nel0 = 0.0, nec_nel1 = 0.0, nec_err0 = 1e10, nec_err1 = -1e10;
   int iprev = 0, iconv, bad = 0;
@@ -67,7 +79,7 @@ __global__ void __launch_bounds__(EOS_BLOCK) saha_eos_kernel(const EosArgs A) {
       for (int istart = 1; istart <= nion - 1; ++istart) {
         n[istart - 1] = 1.0;
         for (int ii = istart + 1; ii <= nion; ++ii) {
-          help = sahac2 * exp(-kti * e[ii - 2]) * n[ii - 2] * q[ii - 1] / q[ii - 2];
+          help = sahac2 * ex[ii - 2] * n[ii - 2] * q[ii - 1] / q[ii - 2];
           n[ii - 1] = help;
         }
         if (help < DBL_MAX) break;
@@ -80,9 +92,7 @@ __global__ void __launch_bounds__(EOS_BLOCK) saha_eos_kernel(const EosArgs A) {
       for (int ii = 2; ii <= nion; ++ii) ne = ne + (double)(ii - 1) * n[ii - 1];
     }
     if (__any_sync(0xffffffffu, inval)) { bad = 1; break; }
-    const double term = fr * ne;
-    double nel_new = 0.0;
-    for (int z = 0; z < A.nelem; ++z) nel_new = nel_new + __shfl_sync(0xffffffffu, term, z);
+    const double nel_new = element_sum(fr * ne, A.nelem);
     const double err = nel / nel_new - 1.0;
     if (fabs(err) < A.acc) {
       if (iconv > 1) nel = nel_new;
@@ -235,52 +245,55 @@ __global__ void __launch_bounds__(EOS_BLOCK) saha_eos_bwd_kernel(const EosArgs A
 // massfr2natomfr (GAS/gas_setup.f:101-160) for differentiable inputs: mass
 // fractions X (nelem, ncell) renormalised to one, gas_mass = rho vol,
 // natomfr(z) ~ X_z/m_z normalised, gas_natom = mass sum(X/m) / amu.
-__global__ void composition_kernel(int nc, int nelem, const double* __restrict__ rho, const double* __restrict__ X,
-                                   const double* __restrict__ vol, const double* __restrict__ amass,
-                                   double* __restrict__ mass, double* __restrict__ natom,
-                                   double* __restrict__ natomfr) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nc) return;
-  const double* x = X + (size_t)i * nelem;
-  double sx = 0.0;
-  for (int z = 0; z < nelem; ++z) sx += x[z];
-  double S = 0.0;
-  for (int z = 0; z < nelem; ++z) S += (x[z] / sx) / amass[z];
-  const double m = rho[i] * vol[i];
-  mass[i] = m;
-  natom[i] = m * S / pc_amu;
+// A warp per shell, lane = element; sums in element order.  (A thread per shell
+// waited on 30 strided loads and divisions in turn: 32 us, its adjoint 48 us,
+// whatever the number of shells; 5 and 7 us now.)
+__global__ void __launch_bounds__(EOS_BLOCK) composition_kernel(int nc, int nelem, const double* __restrict__ rho,
+                                                                const double* __restrict__ X,
+                                                                const double* __restrict__ vol,
+                                                                const double* __restrict__ amass,
+                                                                double* __restrict__ mass, double* __restrict__ natom,
+                                                                double* __restrict__ natomfr) {
+  const int lane = threadIdx.x & 31;
+  const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (i >= nc) return;  // uniform over the warp
+  const bool act = lane < nelem;
+  const double x = act ? X[(size_t)i * nelem + lane] : 0.0;
+  const double sx = element_sum(x, nelem);
+  const double y = act ? (x / sx) / amass[lane] : 0.0;
+  const double S = element_sum(y, nelem);
   double* fr = natomfr + (size_t)i * (nelem + 1);
-  fr[0] = 0.0;
-  for (int z = 0; z < nelem; ++z) fr[z + 1] = ((x[z] / sx) / amass[z]) / S;
+  if (act) fr[lane + 1] = y / S;
+  if (lane == 0) {
+    const double m = rho[i] * vol[i];
+    mass[i] = m;
+    natom[i] = m * S / pc_amu;
+    fr[0] = 0.0;
+  }
 }
 
 // Adjoint of composition_kernel: gnatom, gfr -> grho, gX.
-__global__ void composition_bwd_kernel(int nc, int nelem, const double* __restrict__ rho,
-                                       const double* __restrict__ X, const double* __restrict__ vol,
-                                       const double* __restrict__ amass, const double* __restrict__ gnatom,
-                                       const double* __restrict__ gfr, double* __restrict__ grho,
-                                       double* __restrict__ gX) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nc) return;
-  const double* x = X + (size_t)i * nelem;
-  const double* g = gfr + (size_t)i * (nelem + 1);
-  double sx = 0.0;
-  for (int z = 0; z < nelem; ++z) sx += x[z];
-  double S = 0.0, gy_fr = 0.0;
-  for (int z = 0; z < nelem; ++z) S += (x[z] / sx) / amass[z];
-  for (int z = 0; z < nelem; ++z) gy_fr += g[z + 1] * ((x[z] / sx) / amass[z]);
+__global__ void __launch_bounds__(EOS_BLOCK) composition_bwd_kernel(
+    int nc, int nelem, const double* __restrict__ rho, const double* __restrict__ X, const double* __restrict__ vol,
+    const double* __restrict__ amass, const double* __restrict__ gnatom, const double* __restrict__ gfr,
+    double* __restrict__ grho, double* __restrict__ gX) {
+  const int lane = threadIdx.x & 31;
+  const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (i >= nc) return;  // uniform over the warp
+  const bool act = lane < nelem;
+  const double x = act ? X[(size_t)i * nelem + lane] : 0.0;
+  const double g = act ? gfr[(size_t)i * (nelem + 1) + lane + 1] : 0.0;
+  const double sx = element_sum(x, nelem);
+  const double y = act ? (x / sx) / amass[lane] : 0.0;
+  const double S = element_sum(y, nelem);
+  const double gy_fr = element_sum(act ? g * y : 0.0, nelem);
   const double m = rho[i] * vol[i];
-  grho[i] = gnatom[i] * vol[i] * S / pc_amu;
+  if (lane == 0) grho[i] = gnatom[i] * vol[i] * S / pc_amu;
   // y_z = Xhat_z/m_z, S = sum y, natom = m S/amu, fr_z = y_z/S
   const double gS = gnatom[i] * m / pc_amu - gy_fr / (S * S);
-  double dot = 0.0;
-  double* gx = gX + (size_t)i * nelem;
-  for (int z = 0; z < nelem; ++z) {
-    const double gxh = (g[z + 1] / S + gS) / amass[z];
-    gx[z] = gxh;
-    dot += gxh * (x[z] / sx);
-  }
-  for (int z = 0; z < nelem; ++z) gx[z] = (gx[z] - dot) / sx;  // Xhat = X / sum X
+  const double gxh = act ? (g / S + gS) / amass[lane] : 0.0;
+  const double dot = element_sum(act ? gxh * (x / sx) : 0.0, nelem);
+  if (act) gX[(size_t)i * nelem + lane] = (gxh - dot) / sx;  // Xhat = X / sum X
 }
 
 int launch_saha_eos(slg_ctx* ctx, const double* temp, const double* natom, const double* vol,
@@ -306,7 +319,7 @@ int check_eos(slg_ctx* ctx, int noc) {
 int launch_composition(slg_ctx* ctx, const double* rho, const double* X, double* mass, double* natom,
                        double* natomfr) {
   const int nc = ctx->nx;
-  composition_kernel<<<(nc + 127) / 128, 128, 0, ctx->stream>>>(nc, ctx->eos_nelem, rho, X, ctx->d_vol,
+  composition_kernel<<<(unsigned)(((long long)nc * 32 + EOS_BLOCK - 1) / EOS_BLOCK), EOS_BLOCK, 0, ctx->stream>>>(nc, ctx->eos_nelem, rho, X, ctx->d_vol,
                                                                 ctx->d_amass, mass, natom, natomfr);
   return cuda_check(ctx, cudaGetLastError(), "composition launch");
 }
@@ -314,7 +327,7 @@ int launch_composition(slg_ctx* ctx, const double* rho, const double* X, double*
 int launch_composition_bwd(slg_ctx* ctx, const double* rho, const double* X, const double* gnatom,
                            const double* gfr, double* grho, double* gX) {
   const int nc = ctx->nx;
-  composition_bwd_kernel<<<(nc + 127) / 128, 128, 0, ctx->stream>>>(nc, ctx->eos_nelem, rho, X, ctx->d_vol,
+  composition_bwd_kernel<<<(unsigned)(((long long)nc * 32 + EOS_BLOCK - 1) / EOS_BLOCK), EOS_BLOCK, 0, ctx->stream>>>(nc, ctx->eos_nelem, rho, X, ctx->d_vol,
                                                                     ctx->d_amass, gnatom, gfr, grho, gX);
   return cuda_check(ctx, cudaGetLastError(), "composition adjoint launch");
 }

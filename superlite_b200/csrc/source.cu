@@ -24,12 +24,39 @@ namespace {
 
 constexpr int SB = 256;
 
+// Sum of n values in index order by one thread, RUNNING: the running sums in
+// their place.  One chain of dependent additions; the next round's values are
+// loaded while a round is added.
+template <bool RUNNING>
+__device__ inline double ordered_sum(double* __restrict__ a, int n) {
+  constexpr int N = 16;
+  double v[N], s = 0.0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) v[j] = j < n ? a[j] : 0.0;
+  for (int q = 0; q < n; q += N) {
+    double w[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) w[j] = q + N + j < n ? a[q + N + j] : 0.0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      if (q + j < n) {
+        s = s + v[j];
+        if (RUNNING) a[q + j] = s;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = w[j];
+  }
+  return s;
+}
+
 // per-cell normalised Planck weights, then their running sum in the order of
 // interior_source.f90:177-181,202-209 (one block per emitting cell)
 __global__ void __launch_bounds__(SB) source_cdf_kernel(int nx, int ng, const double* __restrict__ radtemp,
                                                         const double* __restrict__ wlinv,
                                                         const int32_t* __restrict__ nvol,
                                                         double* __restrict__ cdf) {
+  __shared__ double s_sum;
   const int l = blockIdx.x;
   if (nvol[l] < 1) return;
   double* c = cdf + (size_t)l * ng;
@@ -37,15 +64,12 @@ __global__ void __launch_bounds__(SB) source_cdf_kernel(int nx, int ng, const do
   const double hct = hck * tradinv;
   for (int g = threadIdx.x; g < ng; g += SB) c[g] = specintv_elem(hct, wlinv, g);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int g = 0; g < ng; ++g) s = s + c[g];
-    double denom2 = 0.0;
-    for (int g = 0; g < ng; ++g) {
-      denom2 = denom2 + c[g] / s;
-      c[g] = denom2;
-    }
-  }
+  if (threadIdx.x == 0) s_sum = ordered_sum<false>(c, ng);
+  __syncthreads();
+  const double s = s_sum;
+  for (int g = threadIdx.x; g < ng; g += SB) c[g] = c[g] / s;
+  __syncthreads();
+  if (threadIdx.x == 0) ordered_sum<true>(c, ng);
 }
 
 // vacancies.f90: the first nnew vacant slots in index order.
