@@ -278,16 +278,19 @@ __global__ void bf_table_kernel(int ngsub, int nslot, const int32_t* __restrict_
 }
 
 // One nonzero bound-free cross section of a sub-group (times pc_mbarn) and the
-// ion slot whose population it multiplies.
+// ion slot whose population it multiplies: one vector load.
 struct __align__(16) BfTerm {
   double xs;
   int slot, pad;
 };
 
-// Per sub-group, its nonzero cross sections in slot order (the reference's loop
-// order; it skips xs == 0, physical_opacity.f:184), one warp per sub-group.
-__global__ void bf_compact_kernel(int ngsub, int nslot, const double* __restrict__ xstab, BfTerm* __restrict__ terms,
-                                  int* __restrict__ count) {
+// Per sub-group, its nonzero cross sections whose ion carries any population, in
+// slot order (the reference's loop order; it skips xs == 0,
+// physical_opacity.f:184, and a term of an unpopulated ion adds +0), one warp
+// per sub-group.
+__global__ void bf_select_kernel(int ngsub, int nslot, const double* __restrict__ xstab,
+                                 const int* __restrict__ active, BfTerm* __restrict__ terms,
+                                 int* __restrict__ count) {
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (w >= ngsub) return;
   const size_t base = (size_t)w * nslot;
@@ -295,35 +298,12 @@ __global__ void bf_compact_kernel(int ngsub, int nslot, const double* __restrict
   for (int a0 = 0; a0 < nslot; a0 += 32) {
     const int a = a0 + lane;
     const double x = a < nslot ? xstab[base + a] : 0.0;
-    const unsigned m = __ballot_sync(0xffffffffu, x != 0.0);
-    if (x != 0.0) terms[base + k + __popc(m & ((1u << lane) - 1u))] = BfTerm{x, a, 0};
+    const bool on = x != 0.0 && active[a] != 0;
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (on) terms[base + k + __popc(m & ((1u << lane) - 1u))] = BfTerm{x, a, 0};
     k += __popc(m);
   }
   if (lane == 0) count[w] = k;
-}
-
-// Of those, the terms of ions that carry any population, in the same order (a
-// term of an unpopulated ion adds +0).
-__global__ void bf_select_kernel(int ngsub, int nslot, const BfTerm* __restrict__ terms,
-                                 const int* __restrict__ count, const int* __restrict__ active,
-                                 BfTerm* __restrict__ out, int* __restrict__ nout) {
-  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (w >= ngsub) return;
-  const size_t base = (size_t)w * nslot;
-  const int n = count[w];
-  int k = 0;
-  for (int a0 = 0; a0 < n; a0 += 32) {
-    BfTerm t{0.0, 0, 0};
-    bool on = false;
-    if (a0 + lane < n) {
-      t = terms[base + a0 + lane];
-      on = active[t.slot] != 0;
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, on);
-    if (on) out[base + k + __popc(m & ((1u << lane) - 1u))] = t;
-    k += __popc(m);
-  }
-  if (lane == 0) nout[w] = k;
 }
 
 // One line's shell-independent factors, 16 bytes (one vector load per line):
@@ -1215,22 +1195,14 @@ static int opacity_plan(slg_ctx* ctx, int ngs, bool need_bb, bool need_bf, OpacA
     A.lt = d_lt;
   }
   A.xstab = nullptr;
-  A.bf = nullptr;
-  A.bnnz = nullptr;
   if (need_bf) {
     const size_t n = (size_t)ngsub * nslot;
     double* d_xs = (double*)scratch(ctx, 11, sizeof(double) * n);
-    BfTerm* d_terms = (BfTerm*)scratch(ctx, 86, sizeof(BfTerm) * n);
-    int* d_cnt = (int*)scratch(ctx, 87, sizeof(int) * (size_t)ngsub);
-    if (!d_xs || !d_terms || !d_cnt) return SLG_ERR_OOM;
-    if (!ctx->plan_bf) {
+    if (!d_xs) return SLG_ERR_OOM;
+    if (!ctx->plan_bf)
       bf_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ngsub, nslot, ctx->d_ion_ni, nst, d_wlsub,
                                                                    ctx->d_ph1, ctx->d_ph2, d_xs);
-      bf_compact_kernel<<<(ngsub + 7) / 8, 256, 0, st>>>(ngsub, nslot, d_xs, d_terms, d_cnt);
-    }
     A.xstab = d_xs;
-    A.bf = d_terms;
-    A.bnnz = d_cnt;
   }
   const int rc = cuda_check(ctx, cudaGetLastError(), "opacity plan launch");
   if (!rc && keep) {
@@ -1276,12 +1248,12 @@ static int opacity_prepare(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_f
       flags->nothmson, gas->natomfr, do_ff ? ctx->d_gff : nullptr, d_hckt, gas_sig, d_hlp, ld, d_grnd, d_ocp, d_active, d_ffigg,
       d_ffdgg, d_ffsum, d_ffdsum, d_ffclamp, d_ffclamp + nc);
   if (do_bf) {
-    BfTerm* d_bf = (BfTerm*)scratch(ctx, 9, sizeof(BfTerm) * (size_t)ngsub * nslot);
-    int* d_nbf = (int*)scratch(ctx, 1, sizeof(int) * (size_t)ngsub);
-    if (!d_bf || !d_nbf) return SLG_ERR_OOM;
-    bf_select_kernel<<<(ngsub + 7) / 8, 256, 0, st>>>(ngsub, nslot, A.bf, A.bnnz, d_active, d_bf, d_nbf);
+    BfTerm* d_bf = (BfTerm*)scratch(ctx, 86, sizeof(BfTerm) * (size_t)ngsub * nslot);
+    int* d_bnnz = (int*)scratch(ctx, 87, sizeof(int) * (size_t)ngsub);
+    if (!d_bf || !d_bnnz) return SLG_ERR_OOM;
+    bf_select_kernel<<<(ngsub + 7) / 8, 256, 0, st>>>(ngsub, nslot, A.xstab, d_active, d_bf, d_bnnz);
     A.bf = d_bf;
-    A.bnnz = d_nbf;
+    A.bnnz = d_bnnz;
   }
   A.nc = nc; A.ng = ng; A.ngs = ngs; A.ngsub = ngsub; A.nelem = nelem; A.nst = nst; A.maxact = nslot;
   A.pnact = nullptr;
