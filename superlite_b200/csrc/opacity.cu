@@ -816,7 +816,6 @@ struct OpacBwd {
   double* goc;         // [slot][cell], added to (bound-free)
   double* ghlp;        // (ncell), added to (d cap / d hlparr)
   double* gfr;         // (0:nelem, ncell), added to
-  double* W;           // [81][cell], added to: free-free table-row weights (null with noff)
 };
 
 // The bound-bound part of the adjoint of one group for FS shells of a lane (i0,
@@ -880,69 +879,15 @@ __device__ __forceinline__ void bb_adjoint(const LineTerm* __restrict__ lt, int 
   } while (lt < end);
 }
 
-// The free-free part of the adjoint of one (shell, group): adds the group's
-// table-row weights to W and the clamped elements' d/d fr to gfr; returns dL/dT
-// and dL/d hlparr.
-__device__ inline double2 ff_adjoint(const OpacArgs& A, const OpacBwd& B, int i, int ig, double h, double u) {
-  const double T = A.temp[i];
-  const double wl = A.wlsub[ig - 1];
-  const double wlinv = 1.0 / wl;
-  const double uu = h * wlinv;
-  const double ru = 10.0 * (log10(uu) + 4.0) + 1.0;
-  const int iu = !(ru >= 1.0) ? 1 : (ru >= (double)(FF_NU - 1) ? FF_NU - 1 : (int)floor(ru));
-  const double du = ru - iu;
-  const double eu = exp(-uu);
-  const double hn = A.ffc1 * sqrt(h) * (1.0 - eu) * cube(wl);
-  const double help = hn * A.hlparr[i];
-  const double dlnhelp = -0.5 / T - eu * uu / (T * (1.0 - eu));
-  const double ln10 = 2.302585092994045684;
-  const double dru = -10.0 / (ln10 * T), drgg = -5.0 / (ln10 * T);  // table coordinates vs T
-  // this group's weights of table rows iu - 1 and iu, for d cap / d fr of
-  // the unclamped elements (ff_fr_bwd_kernel)
-  atomicAdd(&B.W[(size_t)(iu - 1) * A.nc + i], u * help * (1.0 - du));
-  atomicAdd(&B.W[(size_t)iu * A.nc + i], u * help * du);
-  // unclamped elements from the shell's sums over elements (ff_sum_kernel):
-  // S = sum z^2 fr gff, dS/dT through the table row (du) and column (dgg)
-  const double* Sv = A.ffsum + (size_t)i * FF_NU;
-  const double* Dv = A.ffdsum + (size_t)i * FF_NU;
-  const double s0 = Sv[iu - 1], s1 = Sv[iu];
-  double S = (1.0 - du) * s0 + du * s1;
-  double dS = (s1 - s0) * dru + ((1.0 - du) * Dv[iu - 1] + du * Dv[iu]) * drgg;
-  // elements under the gff >= 1 clamp, one by one
-  const double* nfr = A.natomfr + (size_t)(A.nelem + 1) * i;
-  for (unsigned m = A.ffclamp_all[i]; m; m &= m - 1) {
-    const int iz = __ffs(m);
-    const double fr = nfr[iz];
-    const int igg = -A.ffigg[(size_t)(iz - 1) * A.nc + i];
-    const double dgg = A.ffdgg[(size_t)(iz - 1) * A.nc + i];
-    const double* G = A.gff;
-    const double g00 = G[(iu - 1) + FF_NU * (igg - 1)], g10 = G[iu + FF_NU * (igg - 1)];
-    const double g01 = G[(iu - 1) + FF_NU * igg], g11 = G[iu + FF_NU * igg];
-    const double graw = (1.0 - du) * (1.0 - dgg) * g00 + du * (1.0 - dgg) * g10 + (1.0 - du) * dgg * g01 +
-                        du * dgg * g11;
-    const bool flat = graw < 1.0;
-    const double g = flat ? 1.0 : graw;
-    const double dg = flat ? 0.0
-                           : ((1.0 - dgg) * (g10 - g00) + dgg * (g11 - g01)) * dru +
-                                 ((1.0 - du) * (g01 - g00) + du * (g11 - g10)) * drgg;
-    const double w = (double)(iz * iz);
-    atomicAdd(&B.gfr[(size_t)i * (A.nelem + 1) + iz], u * help * g * w);
-    if (fr == 0.0) continue;
-    S = S + g * w * fr;
-    dS = dS + dg * w * fr;
-  }
-  return make_double2(u * (help * S * dlnhelp + help * dS), u * hn * S);
-}
-
-// Adjoint of the forward's groups (ngs = 1): bb and ff in one pass over the lines
-// of each group (bf: bf_bwd_kernel).  Block: groups blockIdx.x * gpb + 1 .. + gpb
+// Adjoint of the forward's groups (ngs = 1), bound-bound part: one pass over the
+// lines of each group (bf: bf_bwd_kernel, ff: ff_bwd_kernel).  Block: groups blockIdx.x * gpb + 1 .. + gpb
 // one after another; warp w takes the 32 FS shells from (blockIdx.y * warps + w)
 // 32 FS, lane l shells l, l + 32 ... of them.  Bound like the forward, with 13
 // FP64 operations per term; a population row's gradient leaves by one
 // reduction per (row, group) instead of one per line, whose L2 traffic held the
 // kernel at half its arithmetic's rate.
 template <int FS>
-__global__ void __launch_bounds__(kOpacWarps * 32, 4) opacity_bwd_kernel(const OpacArgs A, const OpacBwd B,
+__global__ void __launch_bounds__(kOpacWarps * 32, 5) opacity_bwd_kernel(const OpacArgs A, const OpacBwd B,
                                                                                const ExpConst C, int gpb) {
   __shared__ double etab[kExpTabN * kExpCopies];
   exp_table_spread(etab);
@@ -952,7 +897,7 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 4) opacity_bwd_kernel(const O
   if (base >= A.nc) return;  // uniform over the warp
   bool live[FS];
   int ii[FS];
-  double h[FS], gt[FS], gh[FS];
+  double h[FS], gt[FS];
   ExpArg arg[FS];
   bool inrange = true;
 #pragma unroll
@@ -963,7 +908,7 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 4) opacity_bwd_kernel(const O
     h[s] = live[s] ? A.hckt[ii[s]] : 0.0;
     arg[s] = exp_arg(h[s]);
     inrange = inrange && h[s] >= 0.0 && h[s] * A.chimax <= 700.0;  // as in the forward
-    gt[s] = gh[s] = 0.0;
+    gt[s] = 0.0;
   }
   inrange = __all_sync(0xffffffffu, inrange);
   const double* const pop = A.grndlev + base + lane;
@@ -976,45 +921,193 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 4) opacity_bwd_kernel(const O
       any = any || u[s] != 0.0;
     }
     if (!__any_sync(0xffffffffu, any)) continue;
-    const int l0 = A.nobb ? 0 : A.lstart[ig], n = A.nobb ? 0 : A.lstart[ig + 1] - l0;
-    if (n > 0) {
-      const double wa = A.wlsub[ig - 1], wb = A.wlsub[ig];
-      const double wl = 0.5 * (wa + wb);
-      const double wlinv = 1.0 / wl;
-      double eh[FS], ue[FS], sbb[FS], schi[FS];
+    const int l0 = A.lstart[ig], n = A.lstart[ig + 1] - l0;
+    if (n <= 0) continue;
+    const double wa = A.wlsub[ig - 1], wb = A.wlsub[ig];
+    const double wl = 0.5 * (wa + wb);
+    const double wlinv = 1.0 / wl;
+    double eh[FS], ue[FS], sbb[FS], schi[FS];
 #pragma unroll
-      for (int s = 0; s < FS; ++s) {
-        eh[s] = exp(-(h[s] * wlinv));
-        ue[s] = u[s] != 0.0 ? u[s] * (1.0 - eh[s]) : 0.0;
-      }
-      if (inrange)
-        bb_adjoint<FS, true>(A.lt + l0, n, h, arg, C, ue, pop, A.ld, B.ggrnd + ii[0], A.nc, etab, mine, sbb,
-                             schi);
-      else
-        bb_adjoint<FS, false>(A.lt + l0, n, h, arg, C, ue, pop, A.ld, B.ggrnd + ii[0], A.nc, etab, mine,
-                              sbb, schi);
-#pragma unroll
-      for (int s = 0; s < FS; ++s) {
-        if (u[s] == 0.0) continue;
-        const double expfac = 1.0 - eh[s], T = A.temp[ii[s]];
-        // h = hc/kT: d exp(-chi h)/dT = chi h/T exp(..), d expfac/dT = -(h/T) wlinv eh
-        gt[s] = gt[s] + u[s] * ((h[s] / T) * (schi[s] * expfac) - sbb[s] * expfac * (h[s] / T) * wlinv * eh[s] / expfac);
-      }
+    for (int s = 0; s < FS; ++s) {
+      eh[s] = exp(-(h[s] * wlinv));
+      ue[s] = u[s] != 0.0 ? u[s] * (1.0 - eh[s]) : 0.0;
     }
-    if (!A.noff) {
+    if (inrange)
+      bb_adjoint<FS, true>(A.lt + l0, n, h, arg, C, ue, pop, A.ld, B.ggrnd + ii[0], A.nc, etab, mine, sbb,
+                           schi);
+    else
+      bb_adjoint<FS, false>(A.lt + l0, n, h, arg, C, ue, pop, A.ld, B.ggrnd + ii[0], A.nc, etab, mine,
+                            sbb, schi);
 #pragma unroll
-      for (int s = 0; s < FS; ++s) {
-        if (u[s] == 0.0) continue;
-        const double2 g = ff_adjoint(A, B, ii[s], ig, h[s], u[s]);
-        gt[s] = gt[s] + g.x;
-        gh[s] = gh[s] + g.y;
-      }
+    for (int s = 0; s < FS; ++s) {
+      if (u[s] == 0.0) continue;
+      const double expfac = 1.0 - eh[s], T = A.temp[ii[s]];
+      // h = hc/kT: d exp(-chi h)/dT = chi h/T exp(..), d expfac/dT = -(h/T) wlinv eh
+      gt[s] = gt[s] + u[s] * ((h[s] / T) * (schi[s] * expfac) - sbb[s] * expfac * (h[s] / T) * wlinv * eh[s] / expfac);
     }
   }
 #pragma unroll
-  for (int s = 0; s < FS; ++s) {
+  for (int s = 0; s < FS; ++s)
     if (gt[s] != 0.0) atomicAdd(&B.gT[ii[s]], gt[s]);
-    if (gh[s] != 0.0) atomicAdd(&B.ghlp[ii[s]], gh[s]);
+}
+
+// Free-free part of the adjoint (physical_opacity.f:197-247, ngs = 1).  The
+// shell's opacity at a group is hn hlparr sum_z z^2 fr_z gff_z, gff_z linear in
+// two rows of the table (the group's iu, du) between two columns (the shell's
+// igg, dgg of the element).  A block takes one shell, a warp 64 consecutive
+// groups at a time, a lane two of them:
+// - elements without the gff >= 1 clamp: d cap / d fr(z) = help z^2 gff_z, so
+//   sum_g u_g help_g gff_z = sum_j W[j] Gz[j] with W[j] the groups' row weights
+//   times u help (u = dL/dcap).  Neighbouring groups share their row (a decade of
+//   wavelengths is ten rows), so a warp adds one pair of sums per distinct row
+//   to W; dL/dT from the shell's sums over elements (opac_cell_kernel);
+// - clamped elements, the same for the whole block: one by one, a sum over the
+//   warp each.
+// All that depends on the shell, and nearly always the table's row, is the same
+// for the whole warp, and gcap is read along the groups.  With a shell per lane
+// at the end of each of opacity_bwd_kernel's groups, it read the table and gcap
+// with a sector per lane, added to W in memory twice per (shell, group) and held
+// registers that the line loop wanted: 4.1 of the adjoint's 16.4 ms at 4096 x 10000
+// (now 1.0), and another 25 us in a kernel for the products with W.  Bound by FP64
+// issue (log10, exp, three divisions and the clamped elements per pair).  One or four
+// groups a lane, or blocks of four warps: 0.05 to 0.2 ms more.
+constexpr int kFfK = 2, kFfWarps = 8;
+__global__ void __launch_bounds__(kFfWarps * 32) ff_bwd_kernel(const OpacArgs A, const OpacBwd B) {
+  __shared__ double sW[kFfWarps][FF_NU];
+  __shared__ double sfr[kFfWarps][32];
+  __shared__ double sg[2][kFfWarps];
+  const int i = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+  if (!(A.mass[i] > 0.0)) return;  // uniform over the block
+  for (int j = lane; j < FF_NU; j += 32) sW[warp][j] = 0.0;
+  sfr[warp][lane] = 0.0;
+  __syncwarp();
+  const double T = A.temp[i], h = A.hckt[i], hl = A.hlparr[i];
+  const double ln10 = 2.302585092994045684;
+  const double dru = -10.0 / (ln10 * T), drgg = -5.0 / (ln10 * T);  // table coordinates vs T
+  const double* Sv = A.ffsum + (size_t)i * FF_NU;
+  const double* Dv = A.ffdsum + (size_t)i * FF_NU;
+  const double* nfr = A.natomfr + (size_t)(A.nelem + 1) * i;
+  const double* G = A.gff;
+  const unsigned clamped = A.ffclamp_all[i];
+  double a[2] = {0.0, 0.0};  // dL/dT, dL/d hlparr
+  for (int g0 = (blockIdx.y * nwarp + warp) * (32 * kFfK); g0 < A.ng; g0 += gridDim.y * nwarp * (32 * kFfK)) {
+    int iu[kFfK];  // 0: nothing to do
+    double u[kFfK], hn[kFfK], du[kFfK], dlnhelp[kFfK], S[kFfK], dS[kFfK];
+#pragma unroll
+    for (int k = 0; k < kFfK; ++k) {
+      const int ig = g0 + 32 * k + lane;
+      iu[k] = 0;
+      u[k] = ig < A.ng ? B.gcap[(size_t)i * A.ng + ig] : 0.0;
+      if (u[k] == 0.0) continue;
+      const double wl = A.wlsub[ig];
+      const double wlinv = 1.0 / wl;
+      const double uu = h * wlinv;
+      const double ru = 10.0 * (log10(uu) + 4.0) + 1.0;
+      iu[k] = !(ru >= 1.0) ? 1 : (ru >= (double)(FF_NU - 1) ? FF_NU - 1 : (int)floor(ru));
+      du[k] = ru - iu[k];
+      const double eu = exp(-uu);
+      hn[k] = A.ffc1 * sqrt(h) * (1.0 - eu) * cube(wl);
+      dlnhelp[k] = -0.5 / T - eu * uu / (T * (1.0 - eu));
+      // unclamped elements: S = sum z^2 fr gff, dS/dT through the table row (du) and
+      // column (dgg)
+      const double s0 = Sv[iu[k] - 1], s1 = Sv[iu[k]];
+      S[k] = (1.0 - du[k]) * s0 + du[k] * s1;
+      dS[k] = (s1 - s0) * dru + ((1.0 - du[k]) * Dv[iu[k] - 1] + du[k] * Dv[iu[k]]) * drgg;
+    }
+    // elements under the gff >= 1 clamp
+    for (unsigned m = clamped; m; m &= m - 1) {
+      const int iz = __ffs(m);
+      const double fr = nfr[iz];
+      const int igg = -A.ffigg[(size_t)(iz - 1) * A.nc + i];
+      const double dgg = A.ffdgg[(size_t)(iz - 1) * A.nc + i];
+      const double w = (double)(iz * iz);
+      double v[1] = {0.0};
+#pragma unroll
+      for (int k = 0; k < kFfK; ++k) {
+        if (iu[k] == 0) continue;
+        // the table's rows iu - 1 and iu at the element's column, and their slopes over it
+        const double* q = G + (iu[k] - 1) + FF_NU * (igg - 1);
+        const double g00 = q[0], g10 = q[1], c0 = q[FF_NU] - g00, c1 = q[FF_NU + 1] - g10;
+        const double r0 = g00 + dgg * c0, dr = (g10 + dgg * c1) - r0;
+        const double graw = r0 + du[k] * dr;
+        const bool flat = graw < 1.0;
+        const double g = flat ? 1.0 : graw;
+        const double dg = flat ? 0.0 : dr * dru + (c0 + du[k] * (c1 - c0)) * drgg;
+        v[0] = v[0] + u[k] * (hn[k] * hl) * g * w;
+        if (fr == 0.0) continue;
+        S[k] = S[k] + g * w * fr;
+        dS[k] = dS[k] + dg * w * fr;
+      }
+      cell_sum<32, 1>(v, nullptr);
+      if (lane == 0) sfr[warp][iz - 1] = sfr[warp][iz - 1] + v[0];
+    }
+#pragma unroll
+    for (int k = 0; k < kFfK; ++k) {
+      if (iu[k] == 0) continue;
+      const double help = hn[k] * hl;
+      a[0] = a[0] + u[k] * (help * S[k] * dlnhelp[k] + help * dS[k]);
+      a[1] = a[1] + u[k] * hn[k] * S[k];
+      u[k] = u[k] * help;
+    }
+    // the unclamped elements' row weights
+    for (;;) {
+      int j = FF_NU;
+#pragma unroll
+      for (int k = 0; k < kFfK; ++k)
+        if (iu[k] != 0) j = min(j, iu[k]);
+      j = __reduce_min_sync(0xffffffffu, j);
+      if (j == FF_NU) break;  // iu < FF_NU
+      double v[2] = {0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < kFfK; ++k) {
+        if (iu[k] != j) continue;
+        v[0] = v[0] + u[k] * (1.0 - du[k]);
+        v[1] = v[1] + u[k] * du[k];
+        iu[k] = 0;
+      }
+      cell_sum<32, 2>(v, nullptr);
+      if (lane == 0) {
+        sW[warp][j - 1] = sW[warp][j - 1] + v[0];
+        sW[warp][j] = sW[warp][j] + v[1];
+      }
+    }
+  }
+  cell_sum<32, 2>(a, nullptr);
+  if (lane == 0) {
+    sg[0][warp] = a[0];
+    sg[1][warp] = a[1];
+  }
+  // the block's sums, and the product of W with the elements' columns, eight
+  // lanes an element
+  __syncthreads();
+  for (int j = threadIdx.x; j < FF_NU; j += blockDim.x) {
+    double w = sW[0][j];
+    for (int k = 1; k < nwarp; ++k) w = w + sW[k][j];
+    sW[0][j] = w;
+  }
+  if (threadIdx.x < 2) {
+    double w = sg[threadIdx.x][0];
+    for (int k = 1; k < nwarp; ++k) w = w + sg[threadIdx.x][k];
+    if (w != 0.0) atomicAdd((threadIdx.x ? B.ghlp : B.gT) + i, w);
+  }
+  __syncthreads();
+  for (int z0 = 0; z0 < A.nelem; z0 += blockDim.x >> 3) {
+    const int z = z0 + (threadIdx.x >> 3), t = threadIdx.x & 7;  // element z + 1
+    const bool some = z < A.nelem;
+    double acc = 0.0;
+    if (some && (clamped >> z & 1u)) {
+      for (int k = t; k < nwarp; k += 8) acc = acc + sfr[k][z];
+    } else if (some) {
+      const int igg = A.ffigg[(size_t)z * A.nc + i];
+      const double dgg = A.ffdgg[(size_t)z * A.nc + i];
+      for (int j = t; j < FF_NU; j += 8)
+        if (sW[0][j] != 0.0)  // (most rows lie outside the groups' range)
+          acc = acc + sW[0][j] * ((1.0 - dgg) * G[j + FF_NU * (igg - 1)] + dgg * G[j + FF_NU * igg]);
+      acc = (double)((z + 1) * (z + 1)) * acc;
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, o);
+    if (some && t == 0) atomicAdd(&B.gfr[(size_t)i * (A.nelem + 1) + z + 1], acc);
   }
 }
 
@@ -1031,26 +1124,6 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 4) opacity_bwd_kernel(const O
 // 21 us; 4096 x 10000: 737 -> 415 us).  Runs after opacity_bwd_kernel and before
 // opac_cell_bwd_kernel.
 constexpr int BFB_T = 32;
-// d cap(g, i) / d fr(z, i) = help(g, i) z^2 gff_z(g, i) for the elements
-// without the gff >= 1 clamp, where gff_z = (1 - du_g) Gz[iu_g - 1] + du_g
-// Gz[iu_g] is linear in the table-row weights: sum_g u_g help_g gff_z =
-// sum_j W[j] Gz[j] with W[j] the row weights of all groups, weighted by
-// u_g help_g (u = dL/dcap).  opacity_bwd_kernel gathers W, ff_fr_bwd_kernel adds
-// z^2 sum_j W[j] Gz[j] to gfr (after opacity_bwd_kernel, which adds the clamped
-// elements).
-__global__ void ff_fr_bwd_kernel(const OpacArgs A, const double* __restrict__ W, double* __restrict__ gfr) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)A.nc * A.nelem) return;
-  const int i = (int)(t % A.nc), iz = (int)(t / A.nc) + 1;
-  const int igg = A.ffigg[(size_t)(iz - 1) * A.nc + i];
-  if (igg < 0) return;  // clamped: opacity_bwd_kernel
-  const double dgg = A.ffdgg[(size_t)(iz - 1) * A.nc + i];
-  const double* G = A.gff;
-  double acc = 0.0;
-  for (int j = 0; j < FF_NU; ++j) acc = acc + W[(size_t)j * A.nc + i] * ((1.0 - dgg) * G[j + FF_NU * (igg - 1)] + dgg * G[j + FF_NU * igg]);
-  gfr[(size_t)i * (A.nelem + 1) + iz] += (double)(iz * iz) * acc;
-}
-
 __global__ void __launch_bounds__(BFB_T * 8) bf_bwd_kernel(const OpacArgs A, const OpacBwd B) {
   __shared__ double su[BFB_T][BFB_T + 1];  // [shell][group]
   __shared__ double sx[BFB_T][BFB_T + 1];  // [group][slot]
@@ -1333,13 +1406,7 @@ int launch_opacity_bwd(slg_ctx* ctx, const slg_gas* gas, const double* gcap, con
   cudaMemsetAsync(ggrnd, 0, sizeof(double) * ((size_t)nslot * nc + nc), st);
   cudaMemsetAsync(goc, 0, sizeof(double) * (size_t)nslot * nc, st);
   cudaMemsetAsync(gfr, 0, sizeof(double) * (size_t)nc * (A.nelem + 1), st);
-  double* W = nullptr;
-  if (!A.noff) {
-    W = (double*)scratch(ctx, 90, sizeof(double) * (size_t)nc * FF_NU);
-    if (!W) return SLG_ERR_OOM;
-    cudaMemsetAsync(W, 0, sizeof(double) * (size_t)nc * FF_NU, st);
-  }
-  OpacBwd B{gcap, gT, ggrnd, goc, ghlp, gfr, W};
+  OpacBwd B{gcap, gT, ggrnd, goc, ghlp, gfr};
   // the active slots, for the bound-free product
   int16_t* d_act = (int16_t*)scratch(ctx, 10, sizeof(int16_t) * (size_t)nslot);
   int* d_nact = (int*)scratch(ctx, 85, sizeof(int));
@@ -1347,18 +1414,24 @@ int launch_opacity_bwd(slg_ctx* ctx, const slg_gas* gas, const double* gcap, con
   ion_compact_kernel<<<1, 32, 0, st>>>(A.nelem, A.nst, ctx->d_ion_ni, A.active, d_act, d_nact);
   A.act_slot = d_act;
   A.pnact = d_nact;
-  // two shells per lane and several groups per block where that leaves blocks
-  // enough (whole adjoint calls on B200: 4096 x 10000 17.2 ms with two, 18.0 with
-  // one; 256 x 2000 0.57 ms with one shell and one group, 0.59 with two shells,
-  // 0.62 with four groups)
-  const int fs = nc < 1024 ? 1 : 2, gpb = nc < 1024 ? 1 : 8;
+  // two shells per lane where there are two warps of them, several groups per block
+  // where that leaves blocks enough (whole adjoint calls on B200: 4096 x 10000 13.7 ms
+  // with two, 15.9 with one, 13.4 with one group; 256 x 2000 0.384 ms with two
+  // shells and one group, 0.442 with one shell, 0.42 with two or four groups)
+  const int fs = nc <= OPAC_CT ? 1 : 2, gpb = nc < 1024 ? 1 : 8;
   const int tiles = (nc + fs * OPAC_CT - 1) / (fs * OPAC_CT), warps = tiles < kOpacWarps ? tiles : kOpacWarps;
   const dim3 grid((A.ng + gpb - 1) / gpb, (tiles + warps - 1) / warps);
-  if (fs == 2) opacity_bwd_kernel<2><<<grid, warps * 32, 0, st>>>(A, B, ExpConst{}, gpb);
-  else opacity_bwd_kernel<1><<<grid, warps * 32, 0, st>>>(A, B, ExpConst{}, gpb);
-  if (!A.noff) {
-    const int64_t nf = (int64_t)nc * A.nelem;
-    ff_fr_bwd_kernel<<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(A, W, gfr);
+  if (A.nobb) {  // no lines set
+  } else if (fs == 2) {
+    opacity_bwd_kernel<2><<<grid, warps * 32, 0, st>>>(A, B, ExpConst{}, gpb);
+  } else {
+    opacity_bwd_kernel<1><<<grid, warps * 32, 0, st>>>(A, B, ExpConst{}, gpb);
+  }
+  {
+    // a block per shell, its groups split where that leaves less than four blocks an SM
+    const int parts = (A.ng + 32 * kFfK - 1) / (32 * kFfK), fw = parts < kFfWarps ? parts : kFfWarps;
+    const int want = (4 * ctx->num_sms + nc - 1) / nc, most = (parts + fw - 1) / fw;
+    ff_bwd_kernel<<<dim3(nc, want < most ? want : most), fw * 32, 0, st>>>(A, B);
   }
   if (!A.nobf) {
     // about four blocks per SM over the slot tiles that a third of the slots fill
