@@ -735,12 +735,12 @@ __global__ void __launch_bounds__(256) opacity_means_kernel(int nc, int ng, cons
 }
 
 // ------------------------------------------------------------ adjoint (no reference counterpart)
-// specintv_elem and spectintv_elem of group g0 and their d/dT at temperature T
-// (hct = hck/T), from one exp of the group's x: the expressions of fplanck and
-// fross (so the same values) and of their derivatives in x, which are zero
-// where the reference clamps x at 300; spectintv's NaN guard
-// (groupmod.f:390-392) gives zero for both.
-__device__ inline void spec_weights_dT(double hct, double T, const double* __restrict__ wlinv, int g0, double& w,
+// specintv_elem and spectintv_elem of group g0 and their d/dT at temperature
+// 1 / tinv (hct = hck tinv), from one exp and two divisions of the group's x:
+// fplanck and fross and their derivatives in x, which are zero where the
+// reference clamps x at 300; spectintv's NaN guard (groupmod.f:390-392) gives
+// zero for both.  (Eight divisions: 526 us of means_bwd_kernel at 4096 x 10000, now 372.)
+__device__ inline void spec_weights_dT(double hct, double tinv, const double* __restrict__ wlinv, int g0, double& w,
                                        double& wr, double& dw, double& dwr) {
   const double x1 = hct * wlinv[g0], x2 = hct * wlinv[g0 + 1];
   const double xm = 0.5 * (x2 + x1), ax = fabs(x2 - x1);
@@ -751,19 +751,19 @@ __device__ inline void spec_weights_dT(double hct, double T, const double* __res
     dfp = 0.0;
     dfr = 0.0;
   } else {
-    const double ex = exp(xm), d = ex - 1.0;
-    fp = cube(xm) / d;
-    fr = (pow4(xm) * ex) / sq(d);
-    dfp = 3.0 * sq(xm) / d - cube(xm) * ex / sq(d);
-    const double v = fr * (4.0 / xm + 1.0 - 2.0 * ex / d);
+    const double ex = exp(xm), d = 1.0 / (ex - 1.0), exd = ex * d;
+    fp = cube(xm) * d;
+    fr = (pow4(xm) * d) * exd;
+    dfp = (3.0 * sq(xm) - cube(xm) * exd) * d;
+    const double v = fr * (4.0 / xm + 1.0 - 2.0 * exd);
     dfr = v != v ? 0.0 : v;
   }
   w = ftpi4 * ax * fp;
-  dw = -(ftpi4 * ax * (fp + xm * dfp)) / T;
+  dw = -(ftpi4 * ax * (fp + xm * dfp)) * tinv;
   const double sr = ftpi4r * ax * fr;
   const bool bad = sr != sr;  // groupmod.f:390-392
   wr = bad ? 0.0 : sr;
-  dwr = bad ? 0.0 : -(ftpi4r * ax * (fr + xm * dfr)) / T;
+  dwr = bad ? 0.0 : -(ftpi4r * ax * (fr + xm * dfr)) * tinv;
 }
 
 // Adjoint of opacity_means_kernel<double>: adds to gcap (ng, ncell), gsig and gT.
@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(256) means_bwd_kernel(int nc, int ng, const do
                                                         double* __restrict__ gsig, double* __restrict__ gT) {
   __shared__ double s1[256], s2[256];
   const int i = blockIdx.x;
-  const double T = temp[i], hct = hck * (1.0 / T);
+  const double tinv = 1.0 / temp[i], hct = hck * tinv;
   const double s = sig[i];
   const double ug = ggrey ? ggrey[i] : 0.0;
   const double cr = capross[i];
@@ -786,7 +786,7 @@ __global__ void __launch_bounds__(256) means_bwd_kernel(int nc, int ng, const do
   for (int g = threadIdx.x; g < ng; g += blockDim.x) {
     const double c = cap[(size_t)i * ng + g];
     double w, wr, dw, dwr;
-    spec_weights_dT(hct, T, wlinv, g, w, wr, dw, dwr);
+    spec_weights_dT(hct, tinv, wlinv, g, w, wr, dw, dwr);
     const double inv = 1.0 / (s + c);
     const double dr = wr * inv * inv;  // -dR/dc
     gcap[(size_t)i * ng + g] += ug * w + ur * dr;
@@ -968,7 +968,7 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 5) opacity_bwd_kernel(const O
 // at the end of each of opacity_bwd_kernel's groups, it read the table and gcap
 // with a sector per lane, added to W in memory twice per (shell, group) and held
 // registers that the line loop wanted: 4.1 of the adjoint's 16.4 ms at 4096 x 10000
-// (now 1.0), and another 25 us in a kernel for the products with W.  Bound by FP64
+// (now 1.4), and another 25 us in a kernel for the products with W.  Bound by FP64
 // issue (log10, exp, three divisions and the clamped elements per pair).  One or four
 // groups a lane, or blocks of four warps: 0.05 to 0.2 ms more.
 constexpr int kFfK = 2, kFfWarps = 8;
