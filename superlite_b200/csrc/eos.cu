@@ -47,6 +47,19 @@ __device__ inline double element_sum(double v, int nelem) {
   return s;
 }
 
+// a / b, correctly rounded, from y = 1 / b: two of Markstein's corrections
+// (Computation of elementary functions on the IBM RISC System/6000, 1990).  The
+// quotient's first estimate is off by less than two units in the last place,
+// the first correction leaves less than one, and the second, whose remainder is
+// exact, rounds it.  Next to the ends of the range a remainder may not be
+// representable: plain division there.
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+  double c = a * y;
+  if ((unsigned)__double2hiint(c) - 0x08000000u >= 0x70000000u) return a / b;  // not in 2^[-895, 897)
+  c = fma(fma(-b, c, a), y, c);
+  return fma(fma(-b, c, a), y, c);
+}
+
 __global__ void __launch_bounds__(EOS_BLOCK) saha_eos_kernel(const EosArgs A) {
   const int lane = threadIdx.x & 31;
   const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -61,11 +74,16 @@ __global__ void __launch_bounds__(EOS_BLOCK) saha_eos_kernel(const EosArgs A) {
   const double ndens = A.natom[i] / A.vol[i];
   const double kti = 1.0 / (pc_kb * T);
   const double sahac = pow(pc_pi2 * pc_me * pc_kb * T / (pc_h * pc_h), 1.5);
-  // exp(-e/kT) of every stage, once: the iterations share them (evaluated in
-  // each: 95 us at 4096 cells; 78 us so, bound by the FP64 divisions and the
-  // chain of stages)
-  double n[EOS_MAXST], ex[EOS_MAXST];
-  for (int ii = 0; ii < nion - 1; ++ii) ex[ii] = exp(-kti * e[ii]);
+  // exp(-e/kT) and 1/q of every stage, once: the iterations share them.  Bound by
+  // FP64 issue over the stages, on small grids by their chain; a call at 4096
+  // cells took 119 us with the exps in each iteration, 98 with a division per
+  // stage and iteration, 92 so
+  double n[EOS_MAXST], ex[EOS_MAXST], qi[EOS_MAXST];
+  for (int ii = 0; ii < nion - 1; ++ii) {
+    ex[ii] = exp(-kti * e[ii]);
+    qi[ii] = 1.0 / q[ii];
+  }
+  double norm = 0.0;  // the stage fractions are n norm
   double nel = A.nelec[i];
   double nec_nel0 = 0.0, nec_nel1 = 0.0, nec_err0 = 1e10, nec_err1 = -1e10;
   int iprev = 0, iconv, bad = 0;
@@ -75,21 +93,25 @@ __global__ void __launch_bounds__(EOS_BLOCK) saha_eos_kernel(const EosArgs A) {
     double ne = 0.0;
     int inval = 0;
     if (act) {
-      double help = 0.0;
+      double help = 0.0, nsum = 0.0;
       for (int istart = 1; istart <= nion - 1; ++istart) {
-        n[istart - 1] = 1.0;
-        for (int ii = istart + 1; ii <= nion; ++ii) {
-          help = sahac2 * ex[ii - 2] * n[ii - 2] * q[ii - 1] / q[ii - 2];
-          n[ii - 1] = help;
+        double prev = 1.0;
+        n[istart - 1] = prev;
+        nsum = 0.0;
+        for (int ii = 0; ii < istart; ++ii) nsum = nsum + n[ii];
+#pragma unroll 2
+        for (int ii = istart; ii < nion; ++ii) {
+          help = quotient(sahac2 * ex[ii - 1] * prev * q[ii], q[ii - 1], qi[ii - 1]);
+          n[ii] = help;
+          nsum = nsum + help;
+          prev = help;
         }
         if (help < DBL_MAX) break;
       }
-      double nsum = 0.0;
-      for (int ii = 0; ii < nion; ++ii) nsum = nsum + n[ii];
       if (nsum != nsum || nsum > DBL_MAX || nsum < DBL_MIN) inval = 1;
-      nsum = 1.0 / nsum;
-      for (int ii = 0; ii < nion; ++ii) n[ii] = n[ii] * nsum;
-      for (int ii = 2; ii <= nion; ++ii) ne = ne + (double)(ii - 1) * n[ii - 1];
+      norm = 1.0 / nsum;
+#pragma unroll 2
+      for (int ii = 1; ii < nion; ++ii) ne = ne + (double)ii * (n[ii] * norm);
     }
     if (__any_sync(0xffffffffu, inval)) { bad = 1; break; }
     const double nel_new = element_sum(fr * ne, A.nelem);
@@ -134,7 +156,7 @@ __global__ void __launch_bounds__(EOS_BLOCK) saha_eos_kernel(const EosArgs A) {
     const size_t o = (size_t)i + (size_t)A.nc * ((size_t)ii + (size_t)A.noc * lane);
     if (ii < nion) {
       A.ginv[o] = 1.0 / g1[ii];
-      A.oc[o] = na * fr * g1[ii] * n[ii] / (q[ii] * v);
+      A.oc[o] = na * fr * g1[ii] * (n[ii] * norm) / (q[ii] * v);
     } else {
       A.ginv[o] = 1.0;
       A.oc[o] = 0.0;
