@@ -522,7 +522,7 @@ __device__ inline double ff_add(const OpacArgs& A, int i, int igs, double h, dou
     const int iu = !(ru >= 1.0) ? 1 : (ru >= (double)(FF_NU - 1) ? FF_NU - 1 : (int)floor(ru));
     const double du = ru - iu;
     const double help = A.ffc1 * sqrt(h) * (1.0 - exp(-u)) * cube(wl) * A.hlparr[i];
-    // sum over elements of z^2 fr gff (ff_sum_kernel), the clamped ones here
+    // sum over elements of z^2 fr gff (opac_cell_kernel), the clamped ones here
     const double* S = A.ffsum + (size_t)i * FF_NU;
     double sg = (1.0 - du) * __ldg(S + iu - 1) + du * __ldg(S + iu);
     for (unsigned m = __ldg(A.ffclamp + i); m; m &= m - 1) {
@@ -1170,7 +1170,7 @@ __global__ void __launch_bounds__(BFB_T * 8) bf_bwd_kernel(const OpacArgs A, con
   }
 }
 
-// Adjoint of opac_cell_prep_kernel: grndlev = oc ginv, hlparr = (natom/vol)^2
+// Adjoint of opac_cell_kernel: grndlev = oc ginv, hlparr = (natom/vol)^2
 // nelec, gas_sig = cthomson nelec natom / vol.
 __global__ void opac_cell_bwd_kernel(int nc, int nelem, int nst, const int32_t* __restrict__ ion_ni,
                                      const double* __restrict__ natom, const double* __restrict__ nelec,
