@@ -1448,17 +1448,8 @@ int launch_opacity_bwd(slg_ctx* ctx, const slg_gas* gas, const double* gcap, con
   return cuda_check(ctx, cudaGetLastError(), "opacity adjoint launch");
 }
 
-// Sanity bitmask of physical_opacity.f:282-291.
-int opacity_flags(slg_ctx* ctx, int32_t* sanity) {
-  int* d_flags = (int*)scratch(ctx, 3, sizeof(int) * 4);
-  int h = 0;
-  int rc = cuda_check(ctx, cudaMemcpyAsync(&h, d_flags, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream),
-                      "flags download");
-  if (rc) return rc;
-  if ((rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "flags sync"))) return rc;
-  if (sanity) *sanity = h;
-  return SLG_OK;
-}
+// Sanity bitmask of physical_opacity.f:282-291 of the last build, on the device.
+const int32_t* opacity_flags(slg_ctx* ctx) { return (const int32_t*)scratch(ctx, 3, sizeof(int) * 4); }
 
 int launch_analytic_opacity(slg_ctx* ctx, const double* temp, const double* rho, int kind,
                             const double* c, double* gas_sig, float* gas_cap) {

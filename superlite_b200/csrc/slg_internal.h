@@ -133,6 +133,14 @@ static_assert(sizeof(MixCell) == 128, "MixCell is one 128-byte line");
 enum { SCAL_EMITLUMP = 0, SCAL_CAPLUMP, SCAL_DOPLUMP, SCAL_CAPGREYINV, SCAL_SPECLUMP, SCAL_FAR,
        SCAL_DX3, SCAL_DVDR, SCAL_N };
 
+// A result on its way to a host array through the context's pinned block.
+struct HostOut {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+constexpr int kHostOut = 16;
+
 // Accumulators written by the transport kernel (device memory).
 struct TransportAcc {
   double evelo, eout, sflux;
@@ -202,6 +210,12 @@ struct slg_ctx {
   int plan_ngs = 0;
   bool plan_edges = false, plan_bb = false, plan_bf = false;
   slg::TransportAcc* d_acc = nullptr;
+  // a host call's small results on their way (capi.cu, down and finish)
+  char* h_block = nullptr;                    // pinned, taken by the first such call
+  bool host_tried = false;                    // (once)
+  size_t host_used = 0;                       // bytes of it that the current call took
+  slg::HostOut host_out[slg::kHostOut] = {};  // what finish() copies out of it
+  int nhost_out = 0;
   slg::TransportAcc* h_acc = nullptr;  // pinned
   // optional trace (host arrays) for the next particle_advance call
   uint64_t* trace_hash = nullptr;
