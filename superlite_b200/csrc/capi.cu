@@ -95,12 +95,14 @@ T* out_buf(slg_ctx* ctx, int slot, size_t n, int* rc) {
 // pageable memory makes the host wait for the stream each time, while these are
 // queued, the call waits once, in finish(), and hands the results out.  Opacity
 // build on host arrays, four results and a flag: 32 shells x 100 groups 162 ->
-// 121 us, 64 x 500 (512 kB) 290 -> 195, 100 x 1000 555 -> 500; what is past the
-// block takes the direct copies, as does everything during a capture, where
-// finish()'s wait is the refusal.  (A block of 2 MB: 370 us at 100 x 1000, but
-// three times the 0.8 ms that the first call spends on getting the block.  The
-// same for the arrays that go up gave nothing: those copies return at once.)
-constexpr size_t kHostBlock = 1 << 20, kHostResult = 512 << 10;
+// 120 us, 64 x 200 (205 kB) 213 -> 152; what is past the block takes the direct
+// copies, as does everything during a capture, where finish()'s wait is the
+// refusal.  The driver hands out pinned memory from chunks of 2 MB: a block of
+// this size costs the call that takes it 13 us, and one call in several contexts
+// a new chunk, 1 to 3 ms; blocks of 1 and 2 MB (64 x 500 290 -> 195 us, 100 x 1000
+// 555 -> 370) pay for a chunk each.  (The same for the arrays that go up gave
+// nothing: those copies return at once.)
+constexpr size_t kHostBlock = 256 << 10;
 bool host_block(slg_ctx* ctx, size_t need) {
   if (ctx->capturing || ctx->nhost_out >= kHostOut || ctx->host_used + need > kHostBlock) return false;
   if (!ctx->h_block && !ctx->host_tried) {
@@ -117,7 +119,7 @@ void down(slg_ctx* ctx, T* h, const T* d, size_t n, int* rc) {
   if (*rc || !h || !d) return;
   void* dst = h;
   const size_t bytes = sizeof(T) * n, need = (bytes + 63) & ~(size_t)63;
-  if (bytes <= kHostResult && host_block(ctx, need)) {
+  if (host_block(ctx, need)) {
     dst = ctx->h_block + ctx->host_used;
     ctx->host_used += need;
     ctx->host_out[ctx->nhost_out++] = {h, dst, bytes};

@@ -1,5 +1,5 @@
 """Results of host calls around the sizes where their copies change from the
-context's pinned block to direct ones (512 KiB a result, 1 MiB a call): the opacity build
+context's pinned block to direct ones (256 KiB a call): the opacity build
 on host arrays against the CPU oracle (as in test_gpu_opacity.py), and after a call
 that failed on the way."""
 import ctypes as C
@@ -14,7 +14,7 @@ from test_gpu_opacity import _assert_opacity_parity, _gpu_opacity, _setup
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nc,ng", [(3, 10), (64, 512), (64, 1024), (128, 1024), (129, 1025), (200, 150)])
+@pytest.mark.parametrize("nc,ng", [(3, 10), (64, 200), (64, 256), (64, 511), (128, 513), (200, 50)])
 def test_opacity_on_host_arrays(hot, oracle, nc, ng):
     case = cases.reference_opacity_case(oracle, ncell=nc, ng=ng, nline=500, seed=nc, lines="synthetic")
     _setup(hot, case)
