@@ -1213,16 +1213,34 @@ __global__ void opac_cell_bwd_kernel(int nc, int nelem, int nst, const int32_t* 
 }  // namespace
 
 // ============================================================ launchers
-// One launch of opacity_fwd_kernel on the stream.  Two shells per lane, one where
-// that leaves lanes without a shell (measured on B200: 77 shells x 333 groups of
-// three sub-groups 16 against 19 us, 32 x 100 148 against 154 us a host call;
-// from 128 shells on two: 256 x 2000 178 against 265 us); four hold too many
-// registers for the warps they leave (256 x 2000 214 us, 4096 x 10000 9.23
-// against 8.86 ms).
+// Groups that a block of the line kernels takes one after another: one, except on
+// the largest grids, where more save filling the exp table (warps: of two shells
+// per lane over all groups).  Measured on B200, one against `most` groups: forward
+// 4096 x 10000 (640000 warps) 5.37 against 5.30 ms, 10000 x 1000 (157000) 1.34
+// against 1.36, 1024 x 500 248 against 311 us, 1024 x 64 240 against 847 us, whose
+// grid then leaves the chip idle; adjoint 9.62 against 9.10 ms, 4096 x 2000 (128000)
+// 3.12 against 3.22, 1024 x 64 345 against 1621 us (whole calls).
+static int groups_per_block(int nc, int ng, int most) {
+  const long long warps = (long long)ng * ((nc + 2 * OPAC_CT - 1) / (2 * OPAC_CT));
+  return warps >= 400000 ? most : 1;
+}
+
+// One launch of opacity_fwd_kernel on the stream.  One shell per lane where two
+// would leave lanes without a shell, or less than three warps for a scheduler:
+// with so few, the chain of a warp's lines is what counts, and it is shorter with
+// one exp a line.  Measured on B200, whole calls with one / two shells per lane:
+// 128 shells x 20 groups (40 warps of two) 542 / 661 us, 1024 x 64 (1024) 203 /
+// 240, 256 x 500 (2000) 103 / 95, 512 x 300 (2400) 187 / 166, 256 x 2000 196 / 175;
+// 96 x 10000 186 / 199 and 97 x 10000 230 / 197 (a fourth of two shells' lanes idle,
+// none); 77 x 333 of three sub-groups 16 / 19.  Four shells hold too many registers
+// for the warps they leave (256 x 2000 214 against 178 us, 4096 x 10000 9.23 against
+// 8.86 ms).
 static int launch_fwd(slg_ctx* ctx, OpacArgs& A) {
-  const int fs = A.nc < 128 ? 1 : 2;
-  const int tiles = (A.nc + fs * OPAC_CT - 1) / (fs * OPAC_CT), warps = tiles < kOpacWarps ? tiles : kOpacWarps;
-  const int gpb = A.nc < 1024 ? 1 : 4;
+  const int t1 = (A.nc + OPAC_CT - 1) / OPAC_CT, t2 = (t1 + 1) / 2;
+  const bool fill = (long long)A.ng * t2 >= 3LL * 4 * ctx->num_sms;
+  const int fs = fill && t1 != 1 && t1 != 3 ? 2 : 1;
+  const int tiles = fs == 2 ? t2 : t1, warps = tiles < kOpacWarps ? tiles : kOpacWarps;
+  const int gpb = groups_per_block(A.nc, A.ng, 4);
   const dim3 grid((A.ng + gpb - 1) / gpb, (tiles + warps - 1) / warps);
   if (fs == 2) opacity_fwd_kernel<2><<<grid, warps * 32, 0, ctx->stream>>>(A, ExpConst{}, gpb);
   else opacity_fwd_kernel<1><<<grid, warps * 32, 0, ctx->stream>>>(A, ExpConst{}, gpb);
@@ -1414,11 +1432,10 @@ int launch_opacity_bwd(slg_ctx* ctx, const slg_gas* gas, const double* gcap, con
   ion_compact_kernel<<<1, 32, 0, st>>>(A.nelem, A.nst, ctx->d_ion_ni, A.active, d_act, d_nact);
   A.act_slot = d_act;
   A.pnact = d_nact;
-  // two shells per lane where there are two warps of them, several groups per block
-  // where that leaves blocks enough (whole adjoint calls on B200: 4096 x 10000 13.7 ms
-  // with two, 15.9 with one, 13.4 with one group; 256 x 2000 0.384 ms with two
-  // shells and one group, 0.442 with one shell, 0.42 with two or four groups)
-  const int fs = nc <= OPAC_CT ? 1 : 2, gpb = nc < 1024 ? 1 : 8;
+  // two shells per lane where there are two warps of them (whole adjoint calls on
+  // B200, one / two shells: 32 x 100 353 / 366 us, 64 x 100 354 / 365, 256 x 2000
+  // 393 / 351, 4096 x 2000 3.70 / 3.12 ms)
+  const int fs = nc <= OPAC_CT ? 1 : 2, gpb = groups_per_block(nc, A.ng, 8);
   const int tiles = (nc + fs * OPAC_CT - 1) / (fs * OPAC_CT), warps = tiles < kOpacWarps ? tiles : kOpacWarps;
   const dim3 grid((A.ng + gpb - 1) / gpb, (tiles + warps - 1) / warps);
   if (A.nobb) {  // no lines set

@@ -1,0 +1,102 @@
+"""Launches that would leave the chip idle: the time of a call on a grid beside the
+time of one that differs from it only where a launch rule could go wrong.  Ratios
+of device times (the smallest of several runs of many calls each), with a bar
+well between what idle SMs cost and what the calls take.
+"""
+import numpy as np
+import pytest
+import torch
+
+import cases
+from superlite_b200 import HotPath
+from superlite_b200 import workloads as W
+from superlite_b200.differentiable import DifferentiableOpacity
+from test_gpu_opacity import _assert_opacity_parity, _gpu_opacity, _setup
+
+pytestmark = pytest.mark.gpu
+
+
+def _us(hot, call, n=20, runs=5):
+    stream = torch.cuda.ExternalStream(hot.stream())
+    for _ in range(3):
+        call()
+    hot.sync()
+    best = float("inf")
+    for _ in range(runs):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record(stream)
+        for _ in range(n):
+            call()
+        b.record(stream)
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) * 1e3 / n)
+    return best
+
+
+def _t(a, dtype=torch.float64):
+    return torch.as_tensor(np.ascontiguousarray(a), dtype=dtype, device="cuda")
+
+
+def _build_us(ncell, ng, nline):
+    """Device time of a physical opacity build of ncell shells (a few shells' states repeated)."""
+    base = W.opacity_case(ncell=16, ng=ng, nline=nline, seed=2)
+    k = np.arange(ncell) % 16
+    grid = W.homologous_grid(ncell, 10 * W.PC_DAY)
+    hot = HotPath(0)
+    hot.set_groups(base.groups.wl)
+    hot.set_grid(grid.xarr, grid.vxarr, grid.vol, grid.divv)
+    g = base.gas
+    hot.set_atomic_data(g.ion_ni, g.oc.shape[1], base.lines, base.bf_ph1, base.bf_ph2, base.ff_gff)
+    gas = dict(temp=_t(g.temp[k]), natom=_t(g.natom[k]), nelec=_t(g.nelec[k]), vol=_t(base.grid.vol[k]),
+               mass=_t(g.mass[k]), natomfr=_t(g.natomfr[k]), oc=_t(g.oc[:, :, k]), ginv=_t(g.ginv[:, :, k]))
+    out = dict(sig=torch.zeros(ncell, dtype=torch.float64, device="cuda"), cap=torch.zeros(ncell, ng, device="cuda"),
+               emiss=torch.zeros(ncell, ng, device="cuda"))
+    torch.cuda.synchronize()
+    us = _us(hot, lambda: hot.physical_opacity_dev(gas, out))
+    hot.close()
+    return us
+
+
+def test_few_groups_on_many_shells():
+    """64 groups fill neither 256 nor 1024 shells' lanes: four times the shells run
+    beside one another (1.3 times the time; four groups after another in a block
+    took 4.5 times)."""
+    assert _build_us(1024, 64, 100_000) < 2.2 * _build_us(256, 64, 100_000)
+
+
+@pytest.mark.parametrize("ncell,ng", [(96, 600), (97, 900), (128, 20), (1024, 13), (1025, 112), (2100, 7)])
+def test_lines_at_the_edges_of_the_rules(hot, oracle, ncell, ng):
+    case = cases.reference_opacity_case(oracle, ncell=ncell, ng=ng, nline=1500, seed=ncell, lines="synthetic")
+    _setup(hot, case)
+    _assert_opacity_parity(_gpu_opacity(hot, case), oracle.physical_opacity(case))
+
+
+def test_several_groups_in_a_block():
+    """The largest grids take groups one after another in a block: 64 shells repeated
+    to 12800, 2001 groups (a remainder for four and for eight a block), against the
+    64 alone, the build and its adjoint."""
+    ng, n0, reps = 2001, 64, 200
+    base = W.opacity_case(ncell=n0, ng=ng, nline=5000, seed=6)
+    ion, g = W.ion_table(), base.gas
+    rng = np.random.default_rng(8)
+    weight = rng.uniform(0.5, 1.5, (n0, ng))
+    res = []
+    for nc in (n0, n0 * reps):
+        k = np.arange(nc) % n0
+        grid = W.homologous_grid(nc, 10 * W.PC_DAY)
+        hot = HotPath(0)
+        hot.set_groups(base.groups.wl)
+        hot.set_grid(grid.xarr, grid.vxarr, grid.vol, grid.divv)
+        hot.set_atomic_data(np.ascontiguousarray(ion.ni, dtype=np.int32), g.oc.shape[1], base.lines, base.bf_ph1,
+                            base.bf_ph2, base.ff_gff)
+        eng = DifferentiableOpacity(hot, ion, 9000.0, np.linspace(1.0, 60.0, W.NELEM), acc=1e-12)
+        leaf = [_t(v).requires_grad_() for v in (g.temp[k], g.rho[k], g.massfr[k])]
+        cap = eng.opacity(*leaf)[0]
+        cap.backward(_t(weight)[torch.as_tensor(k, device="cuda")])
+        res.append((cap.detach().cpu().numpy(), [p.grad.cpu().numpy() for p in leaf]))
+        hot.close()
+    (cap, grad), (caps, grads) = res
+    np.testing.assert_allclose(caps.reshape(reps, n0, ng), np.broadcast_to(cap, (reps, n0, ng)), rtol=1e-11)
+    for a, b in zip(grad, grads):
+        b = b.reshape((reps, *a.shape))
+        np.testing.assert_allclose(b, np.broadcast_to(a, b.shape), rtol=1e-8, atol=1e-10 * np.abs(a).max())
