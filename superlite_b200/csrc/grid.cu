@@ -66,18 +66,19 @@ __device__ inline LeakArgsT<CT> leak_view(LeakArgsT<CT> A, int c, int* i) {
   return A;
 }
 
-// leakage_opacity11.f90:30-171, TPC threads per cell.  One pass over the groups:
+// leakage_opacity11.f90:30-171.  One pass over the groups:
 // one Planck weight per group and one division per face, the factors that the
 // terms of a sum share (speclump, x^2 / vterm, divv / 3c) taken out of it.  The sums
 // are fixed-shape tree reductions (the reference sums sequentially).  In four
-// passes that each formed the weight anew, with eight block-wide reductions and
-// a block per cell: 341 us at 28800 cells x 100 groups (now 72), 988 us at 4096 x 10000
-// in FP64 (640).
-template <class CT, int TPC>
+// passes that each formed the weight anew, with eight block-wide reductions:
+// 277 us at 28800 cells x 100 groups (now 39), 988 us at 4096 x 10000 in FP64 (640).
+template <class CT, int FORM>
 __global__ void __launch_bounds__(GB) leakage_kernel(const LeakArgsT<CT> A0, int nc) {
+  constexpr int TPC = FORM == CELL_WARP ? 32 : GB;
   __shared__ double sh[6 * (GB / 32)];
   __shared__ double shv[GB / 32];
   __shared__ int shi[GB / 32];
+  __shared__ double part[FORM == CELL_BLOCK_WARP_ORDER ? 6 * kWarpCellGroups : 1];
   const int cell = blockIdx.x * (GB / TPC) + threadIdx.x / TPC, t = threadIdx.x % TPC;
   if (cell >= nc) return;  // uniform over the cell's threads
   int i0;
@@ -96,11 +97,10 @@ __global__ void __launch_bounds__(GB) leakage_kernel(const LeakArgsT<CT> A0, int
   const CT* cap2 = out ? capl + ng : capl;
   const double sig1 = in ? A.sig[l - 2] : 0.0, sig2 = out ? A.sig[l] : 0.0;
   const double dx1 = in ? Xa - A.xarr[i - 2] : 0.0, dx2 = out ? A.xarr[i + 1] - Xb : 0.0;
-  // sums: speclump, caplump, capemitlump, leakage left and right, doplump
-  double a[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   double bestv = 0.0;
   int besto = 0x7fffffff;
-  for (int ig = t + 1; ig <= ng; ig += TPC) {
+  // adds group ig to the sums: speclump, caplump, capemitlump, leakage left and right, doplump
+  auto add = [&](int ig, double* a) {
     const double c = (double)capl[ig - 1];
     const double tau = (sigl + c) * dist;
     if (c * dist >= A.taulump && tau >= A.tauddmc) {
@@ -129,8 +129,20 @@ __global__ void __launch_bounds__(GB) leakage_kernel(const LeakArgsT<CT> A0, int
         if (ig > 1 && !((double)capl[ig - 2] * dist >= A.taulump)) a[5] = a[5] - dopspeccalc(tinv, A.wlinv, ig - 1);
       }
     }
+  };
+  double a[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  if (FORM == CELL_BLOCK_WARP_ORDER) {
+    for (int g = t; g < ng; g += TPC) {
+      double e[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+      add(g + 1, e);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) part[k * kWarpCellGroups + g] = e[k];
+    }
+    cell_sum_of_block<6>(part, kWarpCellGroups, ng, a, sh);
+  } else {
+    for (int ig = t + 1; ig <= ng; ig += TPC) add(ig, a);
+    cell_sum<TPC, 6>(a, sh);
   }
-  cell_sum<TPC, 6>(a, sh);
   auto better = [](double v2, int o2, double& v, int& o) {
     if (v2 > v || (v2 == v && o2 < o)) {
       v = v2;
@@ -171,7 +183,7 @@ __global__ void __launch_bounds__(GB) leakage_kernel(const LeakArgsT<CT> A0, int
 // in the reference.  The terms are formed by all TPC threads of a cell first,
 // bins_per_tile whole bins at a time, in shared memory (tile doubles per cell,
 // then nep for the bin sums); with a thread per bin forming its own terms most
-// of a block idled: 91 us at 28800 cells x 100 groups (now 25), 55 us at 1001 x 4003
+// of a block idled: 84 us at 28800 cells x 100 groups (now 24), 55 us at 1001 x 4003
 // (35).
 template <int TPC>
 __global__ void __launch_bounds__(GB) emitprob_kernel(int nc, int ng, int nep, int nepg, int bins_per_tile,
@@ -778,10 +790,11 @@ __global__ void __launch_bounds__(256) ddmc_rate_kernel(const TabArgs A0, int nc
 template <class CT>
 static void launch_leakage_kernel(slg_ctx* ctx, const LeakArgsT<CT>& A) {
   const int nc = ctx->nx;
-  if (ctx->ng <= kWarpCellGroups)
-    leakage_kernel<CT, 32><<<(nc + GB / 32 - 1) / (GB / 32), GB, 0, ctx->stream>>>(A, nc);
-  else
-    leakage_kernel<CT, GB><<<nc, GB, 0, ctx->stream>>>(A, nc);
+  switch (cell_form(nc, ctx->ng, ctx->num_sms)) {
+    case CELL_WARP: leakage_kernel<CT, CELL_WARP><<<(nc + GB / 32 - 1) / (GB / 32), GB, 0, ctx->stream>>>(A, nc); break;
+    case CELL_BLOCK_WARP_ORDER: leakage_kernel<CT, CELL_BLOCK_WARP_ORDER><<<nc, GB, 0, ctx->stream>>>(A, nc); break;
+    default: leakage_kernel<CT, CELL_BLOCK><<<nc, GB, 0, ctx->stream>>>(A, nc);
+  }
 }
 
 int launch_leakage(slg_ctx* ctx, const double* tempinv, const double* sig, const float* cap,
@@ -820,7 +833,7 @@ int launch_emitprob(slg_ctx* ctx, const double* tempinv, const float* cap, const
   // a tile: all bins of a cell where a warp takes it, else up to 4096 groups
   // (nepg is at most 181 for the largest group count)
   const int nc = ctx->nx, ng = ctx->ng, nep = ctx->nep, nepg = ctx->nepg;
-  const bool warp = ng <= kWarpCellGroups;
+  const bool warp = cell_form(nc, ng, ctx->num_sms) == CELL_WARP;  // (bins have one order in any form)
   const int cells = warp ? GB / 32 : 1, bins = warp ? nep : (4096 / nepg < nep ? 4096 / nepg : nep);
   const size_t shm = sizeof(double) * cells * ((size_t)bins * nepg + nep);  // at most 36 KB
   if (warp)

@@ -701,33 +701,45 @@ __global__ void analytic_opacity_kernel(int nc, int ng, const double* __restrict
 }
 
 // ------------------------------------------------------------ Planck / Rosseland means
-// TPC threads per shell, both integrals' weights from one exp, a fixed-shape tree
-// reduction over groups.  CT: float (gas_cap) or double (the FP64 opacity of the
-// differentiable path), (ng, ncell).  With a block per shell, two exps per group
-// and a reduction
-// through nine block-wide steps: 103 us at 28800 shells x 100 groups (now 28), 303 us
-// at 4096 x 10000 in FP64 (227).
-template <class CT, int TPC>
+// Both integrals' weights from one exp, a fixed-shape tree reduction over groups.
+// CT: float (gas_cap) or double (the FP64 opacity of the differentiable path),
+// (ng, ncell).  With two exps per group and a reduction through nine block-wide
+// steps: 90 us at 28800 shells x 100 groups (now 28), 303 us at 4096 x 10000 in
+// FP64 (227).
+template <class CT, int FORM>
 __global__ void __launch_bounds__(256) opacity_means_kernel(int nc, int ng, const double* __restrict__ wlinv,
                                                             const double* __restrict__ temp,
                                                             const double* __restrict__ sig,
                                                             const CT* __restrict__ cap, double* __restrict__ capgrey,
                                                             double* __restrict__ capross) {
+  constexpr int TPC = FORM == CELL_WARP ? 32 : 256;
   __shared__ double sh[2 * 8];
+  __shared__ double part[FORM == CELL_BLOCK_WARP_ORDER ? 2 * kWarpCellGroups : 1];
   const int i = blockIdx.x * (256 / TPC) + threadIdx.x / TPC, t = threadIdx.x % TPC;
   if (i >= nc) return;  // uniform over the cell's threads
   const double tinv = 1.0 / temp[i];
   const double hct = hck * tinv;
   const double s = sig ? sig[i] : 0.0;
-  double a[2] = {0.0, 0.0};
-  for (int g = t; g < ng; g += TPC) {
+  auto add = [&](int g, double* a) {
     const double c = (double)cap[(size_t)i * ng + g];
     double w, wr;
     spec_weights(hct, wlinv, g, w, wr);
     a[0] = a[0] + c * w;
     a[1] = a[1] + (1.0 / (s + c)) * wr;
+  };
+  double a[2] = {0.0, 0.0};
+  if (FORM == CELL_BLOCK_WARP_ORDER) {
+    for (int g = t; g < ng; g += TPC) {
+      double e[2] = {0.0, 0.0};
+      add(g, e);
+      part[g] = e[0];
+      part[kWarpCellGroups + g] = e[1];
+    }
+    cell_sum_of_block<2>(part, kWarpCellGroups, ng, a, sh);
+  } else {
+    for (int g = t; g < ng; g += TPC) add(g, a);
+    cell_sum<TPC, 2>(a, sh);
   }
-  cell_sum<TPC, 2>(a, sh);
   if (t == 0) {
     capgrey[i] = a[0];
     if (capross) capross[i] = 1.0 / a[1];
@@ -1388,11 +1400,12 @@ template <class CT>
 static void launch_means(slg_ctx* ctx, const double* temp, const double* sig, const CT* cap, double* capgrey,
                          double* capross) {
   const int nc = ctx->nx, ng = ctx->ng;
-  if (ng <= kWarpCellGroups)
-    opacity_means_kernel<CT, 32><<<(nc + 7) / 8, 256, 0, ctx->stream>>>(nc, ng, ctx->d_wlinv, temp, sig, cap, capgrey,
-                                                                       capross);
-  else
-    opacity_means_kernel<CT, 256><<<nc, 256, 0, ctx->stream>>>(nc, ng, ctx->d_wlinv, temp, sig, cap, capgrey, capross);
+  const CellForm form = cell_form(nc, ng, ctx->num_sms);
+  const int nblk = form == CELL_WARP ? (nc + 7) / 8 : nc;
+  auto* kernel = form == CELL_WARP               ? opacity_means_kernel<CT, CELL_WARP>
+                 : form == CELL_BLOCK_WARP_ORDER ? opacity_means_kernel<CT, CELL_BLOCK_WARP_ORDER>
+                                                 : opacity_means_kernel<CT, CELL_BLOCK>;
+  kernel<<<nblk, 256, 0, ctx->stream>>>(nc, ng, ctx->d_wlinv, temp, sig, cap, capgrey, capross);
 }
 
 int launch_opacity_means64(slg_ctx* ctx, const double* temp, const double* sig, const double* cap,

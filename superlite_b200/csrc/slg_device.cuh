@@ -258,6 +258,24 @@ __device__ inline void cell_sum(double* v, double* sh) {
   }
 }
 
+// The values of cell_sum<32, N> where a block formed a cell's terms: term k of
+// group g at part[k * ld + g], N at most eight.  Warp k adds term k in a warp's
+// order; every thread of the block gets the sums.  sh: N doubles of the block.
+template <int N>
+__device__ inline void cell_sum_of_block(const double* part, int ld, int ng, double* v, double* sh) {
+  __syncthreads();
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (k < N) {
+    double a[1] = {0.0};
+    for (int g = lane; g < ng; g += 32) a[0] = a[0] + part[k * ld + g];
+    cell_sum<32, 1>(a, nullptr);
+    if (lane == 0) sh[k] = a[0];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < N; ++j) v[j] = sh[j];
+}
+
 // physconstmod.f:79-93
 __device__ inline double planck(double wl, double temp) {
   double b = 1.0 / (wl * temp);

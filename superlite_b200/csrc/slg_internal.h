@@ -266,10 +266,22 @@ int set_error(slg_ctx* ctx, int code, const char* fmt, ...);
 int cuda_check(slg_ctx* ctx, cudaError_t e, const char* what);
 void* scratch(slg_ctx* ctx, int slot, size_t bytes);  // nullptr on failure (error set)
 
-// Threads that share a cell in the kernels that sum over a cell's groups: a warp
-// up to this many groups (eight cells per block, no block-wide steps), else a
-// block of 256.
+// Threads that share a cell in the kernels that sum over a cell's groups.  Above
+// kWarpCellGroups a block of 256 with a tree over its threads.  Up to there the
+// sums have a warp's order and a warp takes a cell (eight cells per block, no
+// block-wide steps) where that fills the chip, about one block per SM and 32 groups;
+// with fewer cells a block forms a cell's terms and a warp adds them.  The order
+// must not depend on the number of cells: a model of a batch has the values that
+// it has alone.  Measured on B200, means + leakage + emission probabilities, warp /
+// block: 64 cells x 512 groups 46 / 19 us, 400 x 100 21.2 / 16.6, 800 x 100 21 / 23,
+// 1200 x 256 33.5 / 30.9, 2000 x 256 33.5 / 43.6, 2000 x 512 52 / 54, 16000 x 100 56 /
+// 178; 8000 x 1024 239 / 255, where a block has its own order.
 constexpr int kWarpCellGroups = 512;
+enum CellForm { CELL_WARP, CELL_BLOCK_WARP_ORDER, CELL_BLOCK };
+inline CellForm cell_form(long long cells, int ng, int num_sms) {
+  if (ng > kWarpCellGroups) return CELL_BLOCK;
+  return cells * 32 >= (long long)ng * num_sms ? CELL_WARP : CELL_BLOCK_WARP_ORDER;
+}
 
 // kernels launch wrappers (return SLG_OK or error)
 int launch_physical_opacity(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_flags* flags,
