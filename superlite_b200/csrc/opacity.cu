@@ -442,6 +442,7 @@ struct OpacArgs {
 };
 
 constexpr int kOpacWarps = 4;  // most warps of a forward or adjoint block
+constexpr int kExpTabBytes = sizeof(double) * kExpTabN * kExpCopies;
 // N neighbouring doubles, N * 8 bytes aligned (at most 16).
 template <int N>
 __device__ __forceinline__ void load_run(const double* __restrict__ p, double* v) {
@@ -499,19 +500,31 @@ __device__ __forceinline__ void bb_sums(const LineTerm* __restrict__ lt, int n, 
     load_run<FS>(pop + (size_t)line_slot(t.idx) * ld, og);  // (any row's where none follows)
   } while (lt < end);
 }
-// The same for any arguments (a shell too cool for exp_scaled's range, or not a number).
+// The sum of one shell of a warp with one whose arguments may leave exp_scaled's
+// range (or are not numbers): out of line and in few registers, so that the loop
+// of all other warps keeps its own (inlined, or with two shells at once, it cost
+// that loop 6 to 13 %), and to the same bits, so that a shell's value does not
+// depend on the warp it is in.  256 shells x 2000 groups, a fourth of the shells beyond
+// the range: 341 us a build, with exp for every term of such a warp 401.
 __device__ __noinline__ double bb_sum_any(const LineTerm* __restrict__ lt, int n, double h,
                                           const double* __restrict__ pop, int ld) {
-  double a = 0.0;
+  extern __shared__ double etab[];  // opacity_fwd_kernel's
+  double a = 0.0, acc = 0.0;
+#pragma unroll 1
   for (int k = 0; k < n; ++k) {
     const LineVals t = load_line(lt + k);
-    const double og = __ldg(pop + (size_t)line_slot(t.idx) * ld);
-    if (og <= 0.0) continue;
-    a = fma(t.pg * og, exp(-(t.chi * h)), a);
+    const double x = t.chi * h;
+    double e;
+    if (fabs(x) <= 700.0) e = exp_scaled(t.chi, exp_arg(h), ExpConst{}, etab, exp_table_mine());
+    else e = x > 746.0 ? 0.0 : exp(-x);  // (exp's zero, without its call)
+    acc = fma(t.pg, e, acc);
+    if (t.idx & kLineRowEnd) {
+      a = fma(acc, __ldg(pop + (size_t)line_slot(t.idx) * ld), a);
+      acc = 0.0;
+    }
   }
   return a;
 }
-
 // Free-free of sub-group igs for shell i (h = hc/kT), added to cap.
 __device__ inline double ff_add(const OpacArgs& A, int i, int igs, double h, double cap) {
   if (!A.noff) {
@@ -566,7 +579,7 @@ __device__ __forceinline__ double bb_expfac(const OpacArgs& A, int igs, double h
 template <int FS>
 __global__ void __launch_bounds__(kOpacWarps * 32, 7) opacity_fwd_kernel(const OpacArgs A, const ExpConst C, int gpb) {
   constexpr int FC = FS * OPAC_CT;
-  __shared__ double etab[kExpTabN * kExpCopies];
+  extern __shared__ double etab[];  // kExpTabBytes
   exp_table_spread(etab);
   __syncthreads();
   const uint32_t mine = exp_table_mine();
@@ -1254,8 +1267,8 @@ static int launch_fwd(slg_ctx* ctx, OpacArgs& A) {
   const int tiles = fs == 2 ? t2 : t1, warps = tiles < kOpacWarps ? tiles : kOpacWarps;
   const int gpb = groups_per_block(A.nc, A.ng, 4);
   const dim3 grid((A.ng + gpb - 1) / gpb, (tiles + warps - 1) / warps);
-  if (fs == 2) opacity_fwd_kernel<2><<<grid, warps * 32, 0, ctx->stream>>>(A, ExpConst{}, gpb);
-  else opacity_fwd_kernel<1><<<grid, warps * 32, 0, ctx->stream>>>(A, ExpConst{}, gpb);
+  if (fs == 2) opacity_fwd_kernel<2><<<grid, warps * 32, kExpTabBytes, ctx->stream>>>(A, ExpConst{}, gpb);
+  else opacity_fwd_kernel<1><<<grid, warps * 32, kExpTabBytes, ctx->stream>>>(A, ExpConst{}, gpb);
   return cuda_check(ctx, cudaGetLastError(), "opacity_fwd launch");
 }
 

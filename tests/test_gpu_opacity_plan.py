@@ -116,3 +116,18 @@ def test_layout_of_a_captured_graph(oracle):
     hot.physical_opacity_dev(gas, one)
     ok(one, ref1)
     hot.close()
+
+
+def test_cool_shell_leaves_its_neighbours_alone(hot, oracle):
+    """A shell beyond the fast exp's range does not change a bit of the others',
+    whatever lane or warp they are in."""
+    case = cases.reference_opacity_case(oracle, ncell=140, ng=9, nline=2000, seed=5, lines="synthetic")
+    _setup(hot, case)
+    a = _gpu_opacity(hot, case)["cap64"]
+    cool = [6, 77, 139]
+    temp = case.gas.temp.copy()
+    temp[cool] = 60.0
+    b = _gpu_opacity(hot, dataclasses.replace(case, gas=dataclasses.replace(case.gas, temp=temp)))["cap64"]
+    rest = np.setdiff1d(np.arange(140), cool)
+    assert np.array_equal(a[rest], b[rest])
+    assert not np.array_equal(a[cool], b[cool])
