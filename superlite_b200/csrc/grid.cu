@@ -385,25 +385,47 @@ __device__ inline int group_info(const TabArgs& A, int l, double dist, int ig, d
   return lumped ? ig | kInfoLumped : ig;
 }
 
-// In-place running sum in index order by one thread.  A chain of dependent FP64
-// additions; the terms of the next round are loaded while a round is added
-// (a load per addition made it wait on memory each time).
-__device__ inline void running_sum(CdfEntry* __restrict__ a, int n) {
-  constexpr int N = 16;
-  double v[N], s = 0.0;
+// In-place running sum in index order by a warp: a chain of dependent FP64
+// additions by its first lane, over tiles that the warp loads and stores together
+// (tile: kSumTile doubles of shared memory; the next tile's terms are under way
+// meanwhile).  With a load and a store in memory for each entry the requests of all
+// blocks' four chains took 600 of the kernel's 1060 us at 1024 cells x 4000 groups; as
+// an addition of every lane, with the terms exchanged by shuffles, 230.
+constexpr int kSumTile = 128;
+__device__ inline void running_sum(CdfEntry* __restrict__ a, int n, double* tile) {
+  constexpr int PER = kSumTile / 32, N = 8;
+  const int lane = threadIdx.x & 31;
+  double v[PER], s = 0.0;
 #pragma unroll
-  for (int j = 0; j < N; ++j) v[j] = j < n ? a[j].sum : 0.0;
-  for (int q = 0; q < n; q += N) {
-    double w[N];
+  for (int k = 0; k < PER; ++k) v[k] = 32 * k + lane < n ? a[32 * k + lane].sum : 0.0;
+  for (int q = 0; q < n; q += kSumTile) {
 #pragma unroll
-    for (int j = 0; j < N; ++j) w[j] = q + N + j < n ? a[q + N + j].sum : 0.0;
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      s = s + v[j];
-      if (q + j < n) a[q + j].sum = s;
+    for (int k = 0; k < PER; ++k) {
+      tile[32 * k + lane] = v[k];
+      const int next = q + kSumTile + 32 * k + lane;
+      v[k] = next < n ? a[next].sum : 0.0;
     }
+    __syncwarp();
+    if (lane == 0) {
+      const int m = min(n - q, kSumTile);
+      for (int k = 0; k < m; k += N) {
+        double2 t[N / 2];
 #pragma unroll
-    for (int j = 0; j < N; ++j) v[j] = w[j];
+        for (int j = 0; j < N / 2; ++j) t[j] = reinterpret_cast<double2*>(tile + k)[j];
+#pragma unroll
+        for (int j = 0; j < N / 2; ++j) {
+          t[j].x = s + t[j].x;
+          t[j].y = t[j].x + t[j].y;
+          s = t[j].y;
+          reinterpret_cast<double2*>(tile + k)[j] = t[j];
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+      if (q + 32 * k + lane < n) a[q + 32 * k + lane].sum = tile[32 * k + lane];
+    __syncwarp();
   }
 }
 
@@ -429,12 +451,94 @@ __device__ inline int count_le(const CdfEntry* __restrict__ a, int n, double v) 
   return lo;
 }
 
+// The ranges {first, last} of one table of CellTables::fine, by the whole block:
+// range k holds the numbers of entries that limits k and k + 1 do not lie below.
+// first_limit(i): the first limit that does not lie below entry i (fm + 1: none of the
+// fm + 1), non-decreasing in i, so that a limit's number is the largest i + 1 of the
+// entries whose first limit is not above it: a maximum per limit, then a running one.
+// lim: fm + 1 ints of shared memory, wmax: GB / 32.  (A search of the table for every
+// limit took 290 of the kernel's 1060 us at 1024 cells x 4000 groups, this 107.)
+template <class First>
+__device__ inline void fine_ranges(short2* __restrict__ fd, int fm, int n, int* lim, int* wmax, First first_limit) {
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  for (int k = t; k <= fm; k += GB) lim[k] = 0;
+  __syncthreads();
+  for (int i = t; i < n; i += GB) {
+    const int k = first_limit(i);
+    if (k <= fm) atomicMax(&lim[k], i + 1);
+  }
+  __syncthreads();
+  const int per = fm / GB + 1, k0 = min(t * per, fm + 1), k1 = min(k0 + per, fm + 1);
+  int m = 0;
+  for (int k = k0; k < k1; ++k) m = max(m, lim[k]);
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, m, o);
+    if (lane >= o) m = max(m, v);
+  }
+  if (lane == 31) wmax[wid] = m;
+  m = __shfl_up_sync(0xffffffffu, m, 1);
+  if (lane == 0) m = 0;
+  __syncthreads();
+  for (int w = 0; w < wid; ++w) m = max(m, wmax[w]);
+  for (int k = k0; k < k1; ++k) {
+    m = max(m, lim[k]);
+    lim[k] = m;
+  }
+  __syncthreads();
+  for (int k = t; k < fm; k += GB) fd[k] = make_short2((short)lim[k], (short)lim[k + 1]);
+  __syncthreads();
+}
+
+// TrnCell record of shell ix, from its scalars (CellTables::scal, nlump).
+__device__ inline TrnCell cell_record(const TabArgs& A, int ix) {
+  const double* X = A.xarr;
+  const double* sc = A.T.scal + (size_t)SCAL_N * (ix - 1);
+  TrnCell r;
+  r.xa = X[ix - 1];
+  r.xb = X[ix];
+  r.vxa = A.vxarr[ix - 1];
+  r.vxb = A.vxarr[ix];
+  r.dist = r.xb - r.xa;
+  r.sig = A.sig[ix - 1];
+  r.divv = A.divv[ix - 1];
+  r.capgrey = A.capgrey[ix - 1];
+  r.x0 = X[0];
+  r.far = sc[SCAL_FAR];
+  r.dvdr = sc[SCAL_DVDR];
+  r.vhelp = r.vxa - r.dvdr * r.xa;
+  r.dopc = 3.0 * pc_c / r.divv;
+  r.sigl = ix > 1 ? A.sig[ix - 2] : 0.0;
+  r.dxl = ix > 1 ? X[ix - 1] - X[ix - 2] : 0.0;
+  r.divvl = ix > 1 ? A.divv[ix - 2] : 0.0;
+  r.sigr = ix < A.nx ? A.sig[ix] : 0.0;
+  r.dxr = ix < A.nx ? X[ix + 1] - X[ix] : 0.0;
+  r.divvr = ix < A.nx ? A.divv[ix] : 0.0;
+  r.xa3 = cube(r.xa);
+  r.xb3 = cube(r.xb);
+  r.nlump = A.T.nlump[ix - 1];
+  r.pad = 0;
+  const double* OL = A.opaclump + (size_t)11 * (ix - 1);
+  const double2 lo = ddmc_rates(OL[0], OL[1], sc[SCAL_EMITLUMP], sc[SCAL_CAPLUMP], sc[SCAL_DOPLUMP], &r.denom);
+  r.pdop = lo.x;
+  r.pleft = lo.y;
+  r.pleak = lo.x + (OL[0] * r.denom + OL[1] * r.denom);
+  return r;
+}
+
 // Per-cell transport tables (see CellTables).  Phase A computes every term in
-// parallel; phase B forms the running sums sequentially, one thread per table,
-// in the order of the reference's loops.
+// parallel; phase B forms the running sums sequentially, a warp per table,
+// in the order of the reference's loops; phase C the guides.  Bound by phase A's
+// exponentials and divisions and by the chains of phase B.  A whole FP64 launch
+// without a particle on B200 (with ddmc_rate_kernel; what a launch pays before its
+// events): 256 cells x 2000 groups 225 -> 128 us, 1024 x 4000 1190 -> 583, 4000 x 100 235
+// -> 178, against 116, 420 and 123 without tables for the events, each of which
+// takes a microsecond or two less with them: longest histories of some hundred
+// events pay for the tables.
 __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
   __shared__ int warp_l[GB / 32], warp_u[GB / 32];
   __shared__ int base_l, base_u;
+  __shared__ __align__(16) double tile[4][kSumTile];
+  __shared__ int lim[kFineMax + 1];
   int ic0;
   const TabArgs A = tab_view(A0, blockIdx.x, &ic0);
   const int ic = ic0, ix = ic;
@@ -509,6 +613,7 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
     sc[SCAL_FAR] = 2.0 * fabs(sqrt(sq(X1) - sq(X0)));
     sc[SCAL_DX3] = dx3;
     sc[SCAL_DVDR] = (A.vxarr[ix] - A.vxarr[ix - 1]) / dist;
+    if (A.fp64) A0.T.cell[blockIdx.x] = cell_record(A, ix);
   }
   __syncthreads();  // glumps and specarr visible to the block
   const double divv = A.divv[ix - 1];
@@ -624,10 +729,10 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
   __syncthreads();
   // ---- phase B: running sums
   if (nlump > 0) {
-    if (threadIdx.x == 0) running_sum(cdop, nlump);
-    else if (threadIdx.x == 32 && ix > 1) running_sum(cleft, nlump);
-    else if (threadIdx.x == 64) running_sum(cright, nlump);
-    else if (threadIdx.x == 96) running_sum(cscat, ng - nlump);
+    if (wid == 0) running_sum(cdop, nlump, tile[0]);
+    else if (wid == 1 && ix > 1) running_sum(cleft, nlump, tile[1]);
+    else if (wid == 2) running_sum(cright, nlump, tile[2]);
+    else if (wid == 3) running_sum(cscat, ng - nlump, tile[3]);
   }
   // ---- phase C: guide tables: the mixed loop's (CellTables::guide) or the FP64 loop's
   __syncthreads();
@@ -642,77 +747,37 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
     }
   }
   if (A.fp64 && A.T.fine) {
-    // a thread per limit k / fm (exact: fm is a power of two): the number of
-    // entries not above it is the end of range k - 1 and the start of range k
     const int fm = A.T.fine_m;
     short2* fd = A.T.fine + (size_t)(ic - 1) * kFineTables * fm;
-    auto limit = [&](int t, int k, int n) {
-      if (k < fm) fd[t * fm + k].x = (short)n;
-      if (k > 0) fd[t * fm + k - 1].y = (short)n;
-    };
     if (nlump > 0) {
       for (int t = 0; t < 4; ++t) {
         const CdfEntry* a = t == 0 ? cdop : (t == 1 ? cleft : (t == 2 ? cright : cscat));
         const int n = t == 1 && ix == 1 ? 0 : (t == 3 ? ng - nlump : nlump);  // no left leak from the first shell
-        for (int k = threadIdx.x; k <= fm; k += blockDim.x) limit(t, k, count_le(a, n, (double)k / (double)fm));
+        // limit k is k / fm (fm is a power of two: the products are exact)
+        fine_ranges(fd + (size_t)t * fm, fm, n, lim, warp_l, [&](int i) {
+          const double x = a[i].sum * (double)fm;
+          return x <= (double)fm ? max((int)ceil(x), 0) : fm + 1;
+        });
       }
     }
-    // the emission thresholds against (k / fine_m) capgrey, rounded as a draw's
+    // the emission thresholds: limit k is (k / fm) capgrey, rounded as a draw's
     // product by capgrey is
     const int n = emit_last_group(A.nep, A.nepg, ng) - 1;
     const double cg = A.capgrey[ic - 1];
     const int one = emit_only_group(A.nep, A.nepg, ng, cg != cg);
-    for (int k = threadIdx.x; k <= fm; k += blockDim.x) {
-      const double v = ((double)k / (double)fm) * cg;
-      int lo = 0, hi = n;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (ecum[mid] > v) hi = mid;
-        else lo = mid + 1;
-      }
-      limit(4, k, one ? one - 1 : lo);
+    if (one) {
+      for (int k = threadIdx.x; k < fm; k += GB) fd[4 * fm + k] = make_short2((short)(one - 1), (short)(one - 1));
+    } else {
+      const double scale = (double)fm / cg;
+      fine_ranges(fd + (size_t)4 * fm, fm, n, lim, warp_l, [&](int i) {
+        const double e = ecum[i], x = e * scale;
+        int k = x <= (double)fm ? max((int)x, 0) : (x != x ? 0 : fm + 1);  // near the limit: then to it
+        while (k > 0 && !(e > ((double)(k - 1) / (double)fm) * cg)) --k;
+        while (k <= fm && e > ((double)k / (double)fm) * cg) ++k;
+        return k;
+      });
     }
   }
-}
-
-// TrnCell records of the FP64 loop, one thread per cell, after cell_tables_kernel.
-__global__ void trn_cell_kernel(const TabArgs A0, int nc, TrnCell* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nc) return;
-  int ix;
-  const TabArgs A = tab_view(A0, c, &ix);
-  const double* X = A.xarr;
-  const double* sc = A.T.scal + (size_t)SCAL_N * (ix - 1);
-  TrnCell r;
-  r.xa = X[ix - 1];
-  r.xb = X[ix];
-  r.vxa = A.vxarr[ix - 1];
-  r.vxb = A.vxarr[ix];
-  r.dist = r.xb - r.xa;
-  r.sig = A.sig[ix - 1];
-  r.divv = A.divv[ix - 1];
-  r.capgrey = A.capgrey[ix - 1];
-  r.x0 = X[0];
-  r.far = sc[SCAL_FAR];
-  r.dvdr = sc[SCAL_DVDR];
-  r.vhelp = r.vxa - r.dvdr * r.xa;
-  r.dopc = 3.0 * pc_c / r.divv;
-  r.sigl = ix > 1 ? A.sig[ix - 2] : 0.0;
-  r.dxl = ix > 1 ? X[ix - 1] - X[ix - 2] : 0.0;
-  r.divvl = ix > 1 ? A.divv[ix - 2] : 0.0;
-  r.sigr = ix < A.nx ? A.sig[ix] : 0.0;
-  r.dxr = ix < A.nx ? X[ix + 1] - X[ix] : 0.0;
-  r.divvr = ix < A.nx ? A.divv[ix] : 0.0;
-  r.xa3 = cube(r.xa);
-  r.xb3 = cube(r.xb);
-  r.nlump = A.T.nlump[ix - 1];
-  r.pad = 0;
-  const double* OL = A.opaclump + (size_t)11 * (ix - 1);
-  const double2 lo = ddmc_rates(OL[0], OL[1], sc[SCAL_EMITLUMP], sc[SCAL_CAPLUMP], sc[SCAL_DOPLUMP], &r.denom);
-  r.pdop = lo.x;
-  r.pleft = lo.y;
-  r.pleak = lo.x + (OL[0] * r.denom + OL[1] * r.denom);
-  out[c] = r;
 }
 
 // CellTables::rates, one thread per (cell, group): the branch rates that
@@ -849,7 +914,6 @@ namespace {
 void launch_tables(cudaStream_t st, int nx, const TabArgs& A) {
   cell_tables_kernel<<<nx, GB, 0, st>>>(A);
   if (!A.fp64) return;
-  trn_cell_kernel<<<(nx + 127) / 128, 128, 0, st>>>(A, nx, A.T.cell);
   const size_t n = (size_t)nx * A.ng;
   ddmc_rate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A, nx, A.T.rates);
 }

@@ -3,14 +3,17 @@ time of one that differs from it only where a launch rule could go wrong.  Ratio
 of device times (the smallest of several runs of many calls each), with a bar
 well between what idle SMs cost and what the calls take.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 import cases
-from superlite_b200 import HotPath
+from superlite_b200 import HotPath, capi
 from superlite_b200 import workloads as W
 from superlite_b200.differentiable import DifferentiableOpacity
+from superlite_b200.timestep import DeviceTimestep
 from test_gpu_opacity import _assert_opacity_parity, _gpu_opacity, _setup
 
 pytestmark = pytest.mark.gpu
@@ -148,7 +151,32 @@ def test_coefficients_of_few_cells():
         temp = _t(rng.uniform(6000.0, 14000.0, 64))
         cap = _t(10 ** rng.uniform(-16.0, -10.0, (64, ng)), torch.float32)
         sig, tinv = 0.1 * cap[:, 0].double().contiguous(), 1.0 / temp
+        grey, ross, lump = torch.empty_like(temp), torch.empty_like(temp), temp.new_empty((64, 11))
+        p = [capi.ptr(v) for v in (temp, sig, cap, grey, ross, tinv, lump)]
         torch.cuda.synchronize()
-        us.append(_us(hot, lambda: (hot.opacity_means(temp, sig, cap), hot.leakage_opacity(tinv, sig, cap)), n=50))
+
+        def call():
+            hot.lib.slg_dev_opacity_means(hot.h, *p[:5])
+            hot.lib.slg_dev_leakage_opacity11(hot.h, p[5], p[1], p[2], None, 5.0, 10.0, p[6])
+
+        us.append(_us(hot, call, n=100))
         hot.close()
     assert us[0] < 1.6 * us[1]
+
+
+def test_tables_of_a_launch_without_particles():
+    """What a particle loop pays before its events: the FP64 loop's tables take less
+    than the mixed loop's, which include the same sums (0.57; with a search for every
+    guide entry and a memory access for every running sum's entry 0.81)."""
+    case = W.opacity_case(ncell=256, ng=2000, nline=20000, seed=5, t_days=12.0)
+    us = []
+    for precision in (0, 1):
+        hot = HotPath(0)
+        ts = DeviceTimestep(hot, case, W.TransportParams(), npart=100, precision=precision)  # every slot vacant
+        ts.opacity()
+        ts.coefficients()
+        hot.sync()
+        us.append(_us(hot, lambda: hot.lib.slg_dev_particle_advance(
+            hot.h, C.byref(ts._tin), capi.ptr(ts.prt), capi.ptr(ts.isv), 100, 7, C.byref(ts._tout))))
+        hot.close()
+    assert us[0] < 0.7 * us[1]
