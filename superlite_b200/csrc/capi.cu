@@ -39,7 +39,7 @@ void* scratch(slg_ctx* ctx, int slot, size_t bytes) {
     cudaFree(b.p);
     b.p = nullptr;
     b.bytes = 0;
-    if ((slot >= 12 && slot <= 20) || slot == 72 || (slot >= 91 && slot <= 93)) ctx->tables.nx = ctx->tables.ng = 0;
+    if ((slot >= 12 && slot <= 20) || slot == 72 || (slot >= 91 && slot <= 97)) ctx->tables.nx = ctx->tables.ng = 0;
   }
   const size_t alloc = bytes + bytes / 8;  // headroom for small growth
   if (cudaMalloc(&b.p, alloc) != cudaSuccess) {

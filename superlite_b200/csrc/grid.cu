@@ -14,6 +14,7 @@
 // sequence of partial sums (all terms are >= 0, so the sums are monotone).
 #include <cuda_runtime.h>
 #include <cfloat>
+#include <type_traits>
 #include "slg_device.cuh"
 #include "slg_internal.h"
 
@@ -368,8 +369,13 @@ __device__ inline TabArgs tab_view(TabArgs A, int c, int* ic) {
     A.opaclump += (size_t)11 * co;
     A.emitprob += (size_t)A.nep * co;
     A.cap += cg;
-    A.T.specarr += cg; A.T.glumps += cg; A.T.cdf_dop += cg; A.T.cdf_left += cg; A.T.cdf_right += cg;
-    A.T.cdf_scat += cg; A.T.emitcum += cg;
+    A.T.specarr += cg; A.T.glumps += cg;
+    if (A.fp64) {
+      A.T.cdf_dop += cg; A.T.cdf_left += cg; A.T.cdf_right += cg; A.T.cdf_scat += cg;
+      A.T.emitcum += cg;
+    } else {
+      A.T.sum_dop += cg; A.T.sum_left += cg; A.T.sum_right += cg; A.T.sum_scat += cg;
+    }
     if (A.T.guide) A.T.guide += (size_t)co * 4 * (A.T.guide_m + 1);
     if (A.T.fine) A.T.fine += (size_t)co * kFineTables * A.T.fine_m;
     A.T.nlump += co;
@@ -385,6 +391,12 @@ __device__ inline int group_info(const TabArgs& A, int l, double dist, int ig, d
   return lumped ? ig | kInfoLumped : ig;
 }
 
+// An entry of a running sum in either loop's form.
+__device__ inline double& sum_of(CdfEntry& e) { return e.sum; }
+__device__ inline double& sum_of(double& e) { return e; }
+__device__ inline CdfEntry make_entry(const CdfEntry*, double sum, int info) { return CdfEntry{sum, info, 0}; }
+__device__ inline double make_entry(const double*, double sum, int) { return sum; }
+
 // In-place running sum in index order by a warp: a chain of dependent FP64
 // additions by its first lane, over tiles that the warp loads and stores together
 // (tile: kSumTile doubles of shared memory; the next tile's terms are under way
@@ -392,18 +404,19 @@ __device__ inline int group_info(const TabArgs& A, int l, double dist, int ig, d
 // blocks' four chains took 600 of the kernel's 1060 us at 1024 cells x 4000 groups; as
 // an addition of every lane, with the terms exchanged by shuffles, 230.
 constexpr int kSumTile = 128;
-__device__ inline void running_sum(CdfEntry* __restrict__ a, int n, double* tile) {
+template <class E>
+__device__ inline void running_sum(E* __restrict__ a, int n, double* tile) {
   constexpr int PER = kSumTile / 32, N = 8;
   const int lane = threadIdx.x & 31;
   double v[PER], s = 0.0;
 #pragma unroll
-  for (int k = 0; k < PER; ++k) v[k] = 32 * k + lane < n ? a[32 * k + lane].sum : 0.0;
+  for (int k = 0; k < PER; ++k) v[k] = 32 * k + lane < n ? sum_of(a[32 * k + lane]) : 0.0;
   for (int q = 0; q < n; q += kSumTile) {
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
       tile[32 * k + lane] = v[k];
       const int next = q + kSumTile + 32 * k + lane;
-      v[k] = next < n ? a[next].sum : 0.0;
+      v[k] = next < n ? sum_of(a[next]) : 0.0;
     }
     __syncwarp();
     if (lane == 0) {
@@ -424,7 +437,7 @@ __device__ inline void running_sum(CdfEntry* __restrict__ a, int n, double* tile
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < PER; ++k)
-      if (q + 32 * k + lane < n) a[q + 32 * k + lane].sum = tile[32 * k + lane];
+      if (q + 32 * k + lane < n) sum_of(a[q + 32 * k + lane]) = tile[32 * k + lane];
     __syncwarp();
   }
 }
@@ -441,11 +454,11 @@ __device__ inline double2 ddmc_rates(double o1, double o2, double emitlump, doub
 }
 
 // number of leading entries of a (n, non-decreasing) not above v
-__device__ inline int count_le(const CdfEntry* __restrict__ a, int n, double v) {
+__device__ inline int count_le(const double* __restrict__ a, int n, double v) {
   int lo = 0, hi = n;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
-    if (a[mid].sum <= v) lo = mid + 1;
+    if (a[mid] <= v) lo = mid + 1;
     else hi = mid;
   }
   return lo;
@@ -530,11 +543,13 @@ __device__ inline TrnCell cell_record(const TabArgs& A, int ix) {
 // in the order of the reference's loops; phase C the guides.  Bound by phase A's
 // exponentials and divisions and by the chains of phase B.  A whole FP64 launch
 // without a particle on B200 (with ddmc_rate_kernel; what a launch pays before its
-// events): 256 cells x 2000 groups 225 -> 128 us, 1024 x 4000 1190 -> 583, 4000 x 100 235
-// -> 178, against 116, 420 and 123 without tables for the events, each of which
+// events): 256 cells x 2000 groups 225 -> 130 us, 1024 x 4000 1190 -> 529, 4000 x 100 235
+// -> 154, against 116, 420 and 123 without tables for the events, each of which
 // takes a microsecond or two less with them: longest histories of some hundred
-// events pay for the tables.
-__global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
+// events pay for the tables.  Four blocks per SM: three / four / five 592 / 529 / 545 us
+// at 1024 x 4000.
+template <bool FP64>
+__global__ void __launch_bounds__(GB, 4) cell_tables_kernel(const TabArgs A0) {
   __shared__ int warp_l[GB / 32], warp_u[GB / 32];
   __shared__ int base_l, base_u;
   __shared__ __align__(16) double tile[4][kSumTile];
@@ -613,14 +628,17 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
     sc[SCAL_FAR] = 2.0 * fabs(sqrt(sq(X1) - sq(X0)));
     sc[SCAL_DX3] = dx3;
     sc[SCAL_DVDR] = (A.vxarr[ix] - A.vxarr[ix - 1]) / dist;
-    if (A.fp64) A0.T.cell[blockIdx.x] = cell_record(A, ix);
+    if (FP64) A0.T.cell[blockIdx.x] = cell_record(A, ix);
   }
   __syncthreads();  // glumps and specarr visible to the block
   const double divv = A.divv[ix - 1];
-  CdfEntry* cdop = A.T.cdf_dop + off;
-  CdfEntry* cleft = A.T.cdf_left + off;
-  CdfEntry* cright = A.T.cdf_right + off;
-  CdfEntry* cscat = A.T.cdf_scat + off;
+  using E = typename std::conditional<FP64, CdfEntry, double>::type;
+  E *cdop, *cleft, *cright, *cscat;
+  if constexpr (FP64) {
+    cdop = A.T.cdf_dop + off; cleft = A.T.cdf_left + off; cright = A.T.cdf_right + off; cscat = A.T.cdf_scat + off;
+  } else {
+    cdop = A.T.sum_dop + off; cleft = A.T.sum_left + off; cright = A.T.sum_right + off; cscat = A.T.sum_scat + off;
+  }
   double* ecum = A.T.emitcum + off;
   // ---- phase A: terms
   if (nlump > 0) {
@@ -650,7 +668,7 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
             t = -(res * speclump * hdop);
           }
         }
-        cdop[q - 1] = CdfEntry{t, from | (group_info(A, ic, dist, to, (double)capc[to - 1]) & ~0xffff), 0};
+        cdop[q - 1] = make_entry(cdop, t, from | (group_info(A, ic, dist, to, (double)capc[to - 1]) & ~0xffff));
         // left leak (:378-397)
         const int iiig = glumps[q - 1];
         const double specig = specarr[iiig - 1];
@@ -668,7 +686,7 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
             const double mfphelp = (sigc + capi) * dist + (A.sig[l - 1] + capl) * dxl;
             res = 2.0 * sq(X0) / (mfphelp * dx3);
           }
-          cleft[q - 1] = CdfEntry{specig * res * speclump * hl, group_info(A, l, dxl, iiig, capl), 0};
+          cleft[q - 1] = make_entry(cleft, specig * res * speclump * hl, group_info(A, l, dxl, iiig, capl));
         }
         // right leak: boundary (:450-460) or interior (:492-511)
         double res;
@@ -691,14 +709,14 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
             res = 2.0 * sq(X1) / (mfphelp * dx3);
           }
         }
-        cright[q - 1] = CdfEntry{specig * res * speclump * hr, info, 0};
+        cright[q - 1] = make_entry(cright, specig * res * speclump * hr, info);
       }
       // effective scattering over unlumped groups (:571-584), loop order q
       if (q <= ng - nlump) {
         const int iig = ng + 1 - q;
         const int iiig = glumps[iig - 1];
         const double help = specarr[iiig - 1] * (double)capc[iiig - 1] * capgreyinv;
-        cscat[q - 1] = CdfEntry{help * denom2, group_info(A, ic, dist, iiig, (double)capc[iiig - 1]), 0};
+        cscat[q - 1] = make_entry(cscat, help * denom2, group_info(A, ic, dist, iiig, (double)capc[iiig - 1]));
       }
     }
   }
@@ -710,7 +728,7 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
   // next bin's start (which rounding could otherwise do), and that start at
   // the bin's last group.  The entries are non-decreasing, so the answer is
   // one plus the number of entries not above r1.
-  if (A.fp64) {
+  if (FP64) {
     const double* ep = A.emitprob + (size_t)A.nep * (ic - 1);
     const int last = emit_last_group(A.nep, A.nepg, ng);
     for (int iep = threadIdx.x; iep < A.nep; iep += GB) {
@@ -736,17 +754,19 @@ __global__ void __launch_bounds__(GB) cell_tables_kernel(const TabArgs A0) {
   }
   // ---- phase C: guide tables: the mixed loop's (CellTables::guide) or the FP64 loop's
   __syncthreads();
-  if (!A.fp64 && A.T.guide && nlump > 0) {
+  if constexpr (!FP64) {
+    if (!A.T.guide || nlump == 0) return;
     const int gm = A.T.guide_m;
     int16_t* gd = A.T.guide + (size_t)(ic - 1) * 4 * (gm + 1);
     for (int t = 0; t < 4; ++t) {
-      const CdfEntry* a = t == 0 ? cdop : (t == 1 ? cleft : (t == 2 ? cright : cscat));
+      const E* a = t == 0 ? cdop : (t == 1 ? cleft : (t == 2 ? cright : cscat));
       const int n = t == 3 ? ng - nlump : nlump;
       for (int k = threadIdx.x; k <= gm; k += blockDim.x)  // no left leak from the first shell
         gd[t * (gm + 1) + k] = (int16_t)count_le(a, t == 1 && ix == 1 ? 0 : n, (double)k / (double)gm);
     }
   }
-  if (A.fp64 && A.T.fine) {
+  if constexpr (FP64) {
+    if (!A.T.fine) return;
     const int fm = A.T.fine_m;
     short2* fd = A.T.fine + (size_t)(ic - 1) * kFineTables * fm;
     if (nlump > 0) {
@@ -912,8 +932,11 @@ int launch_emitprob(slg_ctx* ctx, const double* tempinv, const float* cap, const
 
 namespace {
 void launch_tables(cudaStream_t st, int nx, const TabArgs& A) {
-  cell_tables_kernel<<<nx, GB, 0, st>>>(A);
-  if (!A.fp64) return;
+  if (!A.fp64) {
+    cell_tables_kernel<false><<<nx, GB, 0, st>>>(A);
+    return;
+  }
+  cell_tables_kernel<true><<<nx, GB, 0, st>>>(A);
   const size_t n = (size_t)nx * A.ng;
   ddmc_rate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A, nx, A.T.rates);
 }
@@ -923,31 +946,48 @@ int build_cell_tables(slg_ctx* ctx, const slg_transport_in* in) {
   const int nx = ctx->nx, ng = ctx->ng;
   const size_t n = (size_t)nx * ng;
   CellTables& T = ctx->tables;
+  const bool fp64 = in->precision == 0;  // the mixed loop has its own rates and emission CDF
   if (T.nx != nx || T.ng != ng) {
+    T.have_fp64 = T.have_mixed = false;
     T.specarr = (double*)scratch(ctx, 12, sizeof(double) * n);
     T.glumps = (int16_t*)scratch(ctx, 13, sizeof(int16_t) * n);
-    T.cdf_dop = (CdfEntry*)scratch(ctx, 14, sizeof(CdfEntry) * n);
-    T.cdf_left = (CdfEntry*)scratch(ctx, 15, sizeof(CdfEntry) * n);
-    T.cdf_right = (CdfEntry*)scratch(ctx, 16, sizeof(CdfEntry) * n);
-    T.cdf_scat = (CdfEntry*)scratch(ctx, 17, sizeof(CdfEntry) * n);
-    T.emitcum = (double*)scratch(ctx, 18, sizeof(double) * n);
     T.nlump = (int32_t*)scratch(ctx, 19, sizeof(int32_t) * nx);
     T.scal = (double*)scratch(ctx, 20, sizeof(double) * SCAL_N * nx);
-    // guide entries are int16 positions
     T.guide_m = guide_size(ng);
-    T.guide = ng < 32768 ? (int16_t*)scratch(ctx, 72, sizeof(int16_t) * 4 * (T.guide_m + 1) * (size_t)nx) : nullptr;
-    T.rates = (double2*)scratch(ctx, 91, sizeof(double2) * 2 * n);
-    T.cell = (TrnCell*)scratch(ctx, 92, sizeof(TrnCell) * (size_t)nx);
     T.fine_m = fine_size(ng);
-    T.fine = ng < 32768 ? (short2*)scratch(ctx, 93, sizeof(short2) * kFineTables * T.fine_m * (size_t)nx) : nullptr;
-    if (!T.specarr || !T.glumps || !T.cdf_dop || !T.cdf_left || !T.cdf_right || !T.cdf_scat ||
-        !T.emitcum || !T.nlump || !T.scal || !T.rates || !T.cell || (ng < 32768 && (!T.guide || !T.fine))) {
+    if (!T.specarr || !T.glumps || !T.nlump || !T.scal) {
       T.nx = T.ng = 0;
       return SLG_ERR_OOM;
     }
-    T.nx = nx;
-    T.ng = ng;
   }
+  // Each loop's tables have buffers of their own: a launch of one loop between the
+  // replays of a graph that holds the other's moves nothing that the graph reads.
+  // (Guide entries are int16 positions; SLG_MAX_GROUPS keeps to them.)
+  bool ok = true;
+  if (fp64 && !T.have_fp64) {
+    T.cdf_dop = (CdfEntry*)scratch(ctx, 94, sizeof(CdfEntry) * n);
+    T.cdf_left = (CdfEntry*)scratch(ctx, 95, sizeof(CdfEntry) * n);
+    T.cdf_right = (CdfEntry*)scratch(ctx, 96, sizeof(CdfEntry) * n);
+    T.cdf_scat = (CdfEntry*)scratch(ctx, 97, sizeof(CdfEntry) * n);
+    T.emitcum = (double*)scratch(ctx, 18, sizeof(double) * n);
+    T.rates = (double2*)scratch(ctx, 91, sizeof(double2) * 2 * n);
+    T.cell = (TrnCell*)scratch(ctx, 92, sizeof(TrnCell) * (size_t)nx);
+    T.fine = (short2*)scratch(ctx, 93, sizeof(short2) * kFineTables * T.fine_m * (size_t)nx);
+    T.have_fp64 = ok = T.cdf_dop && T.cdf_left && T.cdf_right && T.cdf_scat && T.emitcum && T.rates && T.cell && T.fine;
+  } else if (!fp64 && !T.have_mixed) {
+    T.sum_dop = (double*)scratch(ctx, 14, sizeof(double) * n);
+    T.sum_left = (double*)scratch(ctx, 15, sizeof(double) * n);
+    T.sum_right = (double*)scratch(ctx, 16, sizeof(double) * n);
+    T.sum_scat = (double*)scratch(ctx, 17, sizeof(double) * n);
+    T.guide = (int16_t*)scratch(ctx, 72, sizeof(int16_t) * 4 * (T.guide_m + 1) * (size_t)nx);
+    T.have_mixed = ok = T.sum_dop && T.sum_left && T.sum_right && T.sum_scat && T.guide;
+  }
+  if (!ok) {
+    T.nx = T.ng = 0;
+    return SLG_ERR_OOM;
+  }
+  T.nx = nx;
+  T.ng = ng;
   TabArgs A;
   A.nx = nx; A.ng = ng; A.nep = ctx->nep; A.nepg = ctx->nepg;
   A.xarr = ctx->d_xarr; A.vxarr = ctx->d_vxarr; A.divv = ctx->d_divv; A.wlinv = ctx->d_wlinv;
@@ -955,7 +995,7 @@ int build_cell_tables(slg_ctx* ctx, const slg_transport_in* in) {
   A.emitprob = in->emitprob; A.cap = in->cap; A.tauddmc = in->tauddmc; A.taulump = in->taulump;
   A.T = T;
   A.cellmap = ctx->nmodel > 1 ? ctx->d_cellmap : nullptr;
-  A.fp64 = in->precision == 0;  // the mixed loop has its own rates and emission CDF
+  A.fp64 = fp64;
   launch_tables(ctx->stream, nx, A);
   return cuda_check(ctx, cudaGetLastError(), "cell tables launch");
 }

@@ -54,11 +54,13 @@ constexpr int kInfoLumped = 1 << 16, kInfoImc = 1 << 17;
 struct CellTables {
   double* specarr = nullptr;  // specintv mode-0 Planck weights
   int16_t* glumps = nullptr;  // diffusion11.f90:103-124 ordering (1-based groups)
-  // resolved-group running sums, each entry with the group it resolves to
+  // resolved-group running sums: for the FP64 loop each entry with the group it
+  // resolves to, for the mixed loop (which reads their FP32 copies) the sums alone
   CdfEntry* cdf_dop = nullptr;  // Doppler (:290-314)
   CdfEntry* cdf_left = nullptr; // left leak (:375-398)
   CdfEntry* cdf_right = nullptr;// right leak (:447-460 at ix==nx, :489-511 else)
   CdfEntry* cdf_scat = nullptr; // effective scatter over unlumped groups (:571-584)
+  double *sum_dop = nullptr, *sum_left = nullptr, *sum_right = nullptr, *sum_scat = nullptr;
   // emitgroup's thresholds (emitgroup.f:3-54): entry g-1 is the draw (times
   // capgrey) from which group g+1 is emitted, see cell_tables_kernel
   double* emitcum = nullptr;
@@ -90,7 +92,10 @@ struct CellTables {
   // FP32 copies of cdf_dop/left/right/scat for the mixed-precision loop (half
   // the bytes per gather; null when only the FP64 loop runs)
   float *cdf32_dop = nullptr, *cdf32_left = nullptr, *cdf32_right = nullptr, *cdf32_scat = nullptr;
+  // the grid that the tables are for, and which loops' tables are in place (each is
+  // allocated by the first launch that reads it)
   int nx = 0, ng = 0;
+  bool have_fp64 = false, have_mixed = false;
 };
 // emitgroup's last reachable group, and its constant answer where it has one
 // (0: none): one emission bin, or a draw that is not a number (nan).

@@ -452,14 +452,14 @@ __global__ void mix_cell_kernel(int nc, const int4* __restrict__ cellmap, const 
 }
 
 // FP32 copies of the four running-sum tables (n entries each).
-__global__ void cdf32_kernel(size_t n, const CdfEntry* __restrict__ a0, const CdfEntry* __restrict__ a1,
-                             const CdfEntry* __restrict__ a2, const CdfEntry* __restrict__ a3, float* __restrict__ b0,
+__global__ void cdf32_kernel(size_t n, const double* __restrict__ a0, const double* __restrict__ a1,
+                             const double* __restrict__ a2, const double* __restrict__ a3, float* __restrict__ b0,
                              float* __restrict__ b1, float* __restrict__ b2, float* __restrict__ b3) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    b0[i] = (float)a0[i].sum;
-    b1[i] = (float)a1[i].sum;
-    b2[i] = (float)a2[i].sum;
-    b3[i] = (float)a3[i].sum;
+    b0[i] = (float)a0[i];
+    b1[i] = (float)a1[i];
+    b2[i] = (float)a2[i];
+    b3[i] = (float)a3[i];
   }
 }
 
@@ -478,7 +478,7 @@ int build_mix_cells(slg_ctx* ctx, const slg_transport_in* in, TrnArgs& A) {
   const CellTables& T = ctx->tables;
   long long nb = (long long)((n + 255) / 256);
   if (nb > 4LL * ctx->num_sms) nb = 4LL * ctx->num_sms;
-  cdf32_kernel<<<(unsigned)(nb > 0 ? nb : 1), 256, 0, ctx->stream>>>(n, T.cdf_dop, T.cdf_left, T.cdf_right, T.cdf_scat,
+  cdf32_kernel<<<(unsigned)(nb > 0 ? nb : 1), 256, 0, ctx->stream>>>(n, T.sum_dop, T.sum_left, T.sum_right, T.sum_scat,
                                                                     c32[0], c32[1], c32[2], c32[3]);
   A.T.cdf32_dop = c32[0];
   A.T.cdf32_left = c32[1];
