@@ -22,6 +22,7 @@
 //  * FP64 throughout, no FMA contraction (-fmad=false), so sums round like the
 //    single-threaded Fortran; only exp/log10/pow may differ in the last ulp.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cfloat>
 #include "slg_device.cuh"
 #include "slg_internal.h"
@@ -79,13 +80,16 @@ __global__ void line_range_kernel(const slg_bbxs* __restrict__ bb, int64_t nline
 // 17-20 us whatever the grid, besides 9 us for the rest; now 15 us in all at 32 and
 // at 256 shells, 20 us at 4096.)
 constexpr int CELLS = 8;
-constexpr int kRun = 64;  // most shells of a warp: the population rows are padded to whole warps' shells
+// Length of a population row: whole warps' shells (64 of two per lane, 32 up to 32
+// shells, which are one per lane).
+static int padded_shells(int nc) { return nc <= OPAC_CT ? OPAC_CT : (nc + 2 * OPAC_CT - 1) / (2 * OPAC_CT) * (2 * OPAC_CT); }
 __global__ void __launch_bounds__(CELLS * 32) opac_cell_kernel(
     int nc, int nelem, int nst, const int32_t* __restrict__ ion_ni, const double* __restrict__ temp,
     const double* __restrict__ natom, const double* __restrict__ nelec, const double* __restrict__ vol,
     const double* __restrict__ mass, const double* __restrict__ oc, const double* __restrict__ ginv, int nothmson,
     const double* __restrict__ natomfr, const double* __restrict__ G, double* __restrict__ hckt,
-    double* __restrict__ gas_sig, double* __restrict__ hlparr, int ld, double* __restrict__ grndlev,
+    double* __restrict__ gas_sig, double* __restrict__ hlparr, int ld, const int16_t* __restrict__ lrow_of_slot,
+    double* __restrict__ grndlev,
     double* __restrict__ ocp, int* __restrict__ active, int* __restrict__ ffigg, double* __restrict__ ffdgg, double* __restrict__ ffsum,
     double* __restrict__ ffdsum, unsigned* __restrict__ ffclamp, unsigned* __restrict__ ffclamp_all) {
   __shared__ double s_w[CELLS][32], s_dgg[CELLS][32];
@@ -101,7 +105,8 @@ __global__ void __launch_bounds__(CELLS * 32) opac_cell_kernel(
       if (ii <= min(iz, ion_ni[iz - 1] - 1) && mass[i] > 0.0) v = o * ginv[(size_t)k * nc + i];
     }
     if (i < ld) {
-      grndlev[(size_t)k * ld + i] = v < 0.0 ? 0.0 : v;  // the reference skips lines with ocg <= 0
+      const int row = lrow_of_slot ? lrow_of_slot[k] : -1;  // of the lines' population rows
+      if (row >= 0) grndlev[(size_t)row * ld + i] = v < 0.0 ? 0.0 : v;  // the reference skips lines with ocg <= 0
       ocp[(size_t)k * ld + i] = o;
     }
     if (o != 0.0) active[k] = 1;
@@ -288,19 +293,19 @@ struct __align__(16) BfTerm {
 // slot order (the reference's loop order; it skips xs == 0,
 // physical_opacity.f:184, and a term of an unpopulated ion adds +0), one warp
 // per sub-group.
-__global__ void bf_select_kernel(int ngsub, int nslot, const double* __restrict__ xstab,
+__global__ void bf_select_kernel(int ngsub, int nslot, int maxbf, const double* __restrict__ xstab,
                                  const int* __restrict__ active, BfTerm* __restrict__ terms,
                                  int* __restrict__ count) {
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (w >= ngsub) return;
-  const size_t base = (size_t)w * nslot;
+  const size_t base = (size_t)w * nslot, out = (size_t)w * maxbf;
   int k = 0;
   for (int a0 = 0; a0 < nslot; a0 += 32) {
     const int a = a0 + lane;
     const double x = a < nslot ? xstab[base + a] : 0.0;
     const bool on = x != 0.0 && active[a] != 0;
     const unsigned m = __ballot_sync(0xffffffffu, on);
-    if (on) terms[base + k + __popc(m & ((1u << lane) - 1u))] = BfTerm{x, a, 0};
+    if (on) terms[out + k + __popc(m & ((1u << lane) - 1u))] = BfTerm{x, a, 0};
     k += __popc(m);
   }
   if (lane == 0) count[w] = k;
@@ -336,6 +341,7 @@ __device__ __forceinline__ LineVals load_line(const LineTerm* p) {
   return LineVals{v.x, __hiloint2double(__double2hiint(v.y), (int)(lo & ~kLineIdxMask)), lo & kLineIdxMask};
 }
 __device__ __forceinline__ int line_slot(unsigned idx) { return (int)((idx >> kLineRowBits) & 0xffffu); }
+__device__ __forceinline__ int line_row(unsigned idx) { return (int)(idx & ((1u << kLineRowBits) - 1u)); }
 
 // The LineTerms of sub-group w + 1, one warp each: its lines counted by row,
 // the rows' first places, then the lines written there in file order (a lane's
@@ -404,22 +410,22 @@ __global__ void __launch_bounds__(LT_WARPS * 32) line_terms_kernel(const slg_bbx
 
 struct OpacArgs {
   int nc, ng, ngs, ngsub, nelem, nst, maxact;
+  int maxbf;                // row length of bf: the slots that can have a cross section
   int nobb, nobf, noff;
   const int* pnact;         // number of active bound-free ion slots (device; adjoint)
   double mix;
   const double* wlsub;
   const double* grp_wl;
   const int* lstart;        // (ngsub+2)+1 line offsets by igs
-  int ld;                   // row length of grndlev and ocp: nc rounded up to kRun
+  int ld;                   // row length of grndlev and ocp (padded_shells)
   const LineTerm* lt;       // per line, by sub-group and row (line_terms_kernel)
   double chimax;            // largest chilw of the lines (infinite: check every exp argument)
-  const double* grndlev;    // [slot][ld], negative values as zero
+  const double* grndlev;    // [row of the lines' population rows][ld], negative values as zero
   const double* ocp;        // [slot][ld]
-  const double* oc;         // [slot][cell]
   const int* active;        // [slot]: nonzero if any cell has population there
   const int16_t* act_slot;  // the active slots, reference order (adjoint)
   const double* xstab;      // [(igs-1) nslot + slot]: bfxs * pc_mbarn
-  const BfTerm* bf;         // [(igs-1) nslot + k]: its nonzero entries of populated ions
+  const BfTerm* bf;         // [(igs-1) maxbf + k]: its nonzero entries of populated ions
   const int* bnnz;          // their count per sub-group
   const double* hckt;
   const double* hlparr;
@@ -471,7 +477,7 @@ __device__ __forceinline__ void bb_sums(const LineTerm* __restrict__ lt, int n, 
                                         double* a) {
   double og[FS];
   LineVals t = load_line(lt);
-  load_run<FS>(pop + (size_t)line_slot(t.idx) * ld, og);
+  load_run<FS>(pop + (size_t)line_row(t.idx) * ld, og);
 #pragma unroll
   for (int s = 0; s < FS; ++s) a[s] = 0.0;
   const LineTerm* const end = lt + n;
@@ -497,7 +503,7 @@ __device__ __forceinline__ void bb_sums(const LineTerm* __restrict__ lt, int n, 
     }
 #pragma unroll
     for (int s = 0; s < FS; ++s) a[s] = fma(acc[s], og[s], a[s]);
-    load_run<FS>(pop + (size_t)line_slot(t.idx) * ld, og);  // (any row's where none follows)
+    load_run<FS>(pop + (size_t)line_row(t.idx) * ld, og);  // (any row's where none follows)
   } while (lt < end);
 }
 // The sum of one shell of a warp with one whose arguments may leave exp_scaled's
@@ -519,7 +525,7 @@ __device__ __noinline__ double bb_sum_any(const LineTerm* __restrict__ lt, int n
     else e = x > 746.0 ? 0.0 : exp(-x);  // (exp's zero, without its call)
     acc = fma(t.pg, e, acc);
     if (t.idx & kLineRowEnd) {
-      a = fma(acc, __ldg(pop + (size_t)line_slot(t.idx) * ld), a);
+      a = fma(acc, __ldg(pop + (size_t)line_row(t.idx) * ld), a);
       acc = 0.0;
     }
   }
@@ -629,7 +635,7 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 7) opacity_fwd_kernel(const O
         }
       }
       if (!A.nobf) {
-        const BfTerm* t = A.bf + (size_t)(igs - 1) * A.maxact;
+        const BfTerm* t = A.bf + (size_t)(igs - 1) * A.maxbf;
         const int n = A.bnnz[igs - 1];
 #pragma unroll 4
         for (int k = 0; k < n; ++k) {
@@ -857,7 +863,7 @@ __device__ __forceinline__ void bb_adjoint(const LineTerm* __restrict__ lt, int 
                                            double* sbb, double* schi) {
   double og[FS];
   auto row_begin = [&](unsigned idx) {
-    const double* g = pop + (size_t)line_slot(idx) * ld;
+    const double* g = pop + (size_t)line_row(idx) * ld;
 #pragma unroll
     for (int s = 0; s < FS; ++s) og[s] = __ldg(g + s * OPAC_CT);
   };
@@ -1348,26 +1354,28 @@ static int opacity_prepare(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_f
   int* d_flags = (int*)scratch(ctx, 3, sizeof(int) * (4 + nslot));  // sanity word, then the active slots
   double* d_hckt = (double*)scratch(ctx, 4, sizeof(double) * nc);
   double* d_hlp = (double*)scratch(ctx, 5, sizeof(double) * nc);
-  const int ld = (nc + kRun - 1) / kRun * kRun;
-  double* d_grnd = (double*)scratch(ctx, 6, sizeof(double) * 2 * (size_t)ld * nslot);
-  double* d_ocp = d_grnd + (size_t)ld * nslot;
+  const int ld = padded_shells(nc), nrow = ctx->nlrow;
+  double* d_ocp = (double*)scratch(ctx, 6, sizeof(double) * (size_t)ld * (nslot + nrow));
+  double* d_grnd = d_ocp + (size_t)ld * nslot;
   int* d_ffigg = (int*)scratch(ctx, 7, sizeof(int) * (size_t)nc * nelem);
   double* d_ffdgg = (double*)scratch(ctx, 8, sizeof(double) * (size_t)nc * nelem);
   double* d_ffsum = (double*)scratch(ctx, 88, sizeof(double) * 2 * (size_t)nc * FF_NU);
   unsigned* d_ffclamp = (unsigned*)scratch(ctx, 89, sizeof(unsigned) * 2 * (size_t)nc);
-  if (!d_flags || !d_hckt || !d_hlp || !d_grnd || !d_ffigg || !d_ffdgg || !d_ffsum || !d_ffclamp) return SLG_ERR_OOM;
+  if (!d_flags || !d_hckt || !d_hlp || !d_ocp || !d_ffigg || !d_ffdgg || !d_ffsum || !d_ffclamp) return SLG_ERR_OOM;
   int* d_active = d_flags + 4;
   cudaMemsetAsync(d_flags, 0, sizeof(int) * (4 + nslot), st);
   double* d_ffdsum = d_ffsum + (size_t)nc * FF_NU;
   opac_cell_kernel<<<(ld + CELLS - 1) / CELLS, CELLS * 32, 0, st>>>(
       nc, nelem, nst, ctx->d_ion_ni, gas->temp, gas->natom, gas->nelec, gas->vol, gas->mass, gas->oc, gas->ginv,
-      flags->nothmson, gas->natomfr, do_ff ? ctx->d_gff : nullptr, d_hckt, gas_sig, d_hlp, ld, d_grnd, d_ocp, d_active, d_ffigg,
-      d_ffdgg, d_ffsum, d_ffdsum, d_ffclamp, d_ffclamp + nc);
+      flags->nothmson, gas->natomfr, do_ff ? ctx->d_gff : nullptr, d_hckt, gas_sig, d_hlp, ld,
+      do_bb ? ctx->d_lrow_of_slot : nullptr, d_grnd, d_ocp, d_active, d_ffigg, d_ffdgg, d_ffsum, d_ffdsum, d_ffclamp, d_ffclamp + nc);
   if (do_bf) {
-    BfTerm* d_bf = (BfTerm*)scratch(ctx, 86, sizeof(BfTerm) * (size_t)ngsub * nslot);
+    A.maxbf = 0;
+    for (int z = 1; z <= nelem; ++z) A.maxbf += std::max(0, std::min(std::min(z, ctx->h_ion_ni[z - 1] - 1), nst));
+    BfTerm* d_bf = (BfTerm*)scratch(ctx, 86, sizeof(BfTerm) * (size_t)ngsub * A.maxbf);
     int* d_bnnz = (int*)scratch(ctx, 87, sizeof(int) * (size_t)ngsub);
     if (!d_bf || !d_bnnz) return SLG_ERR_OOM;
-    bf_select_kernel<<<(ngsub + 7) / 8, 256, 0, st>>>(ngsub, nslot, A.xstab, d_active, d_bf, d_bnnz);
+    bf_select_kernel<<<(ngsub + 7) / 8, 256, 0, st>>>(ngsub, nslot, A.maxbf, A.xstab, d_active, d_bf, d_bnnz);
     A.bf = d_bf;
     A.bnnz = d_bnnz;
   }
@@ -1378,7 +1386,7 @@ static int opacity_prepare(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_f
   A.grp_wl = ctx->d_wl;
   A.chimax = ctx->line_chimax;
   A.ld = ld; A.ocp = d_ocp;
-  A.grndlev = d_grnd; A.oc = gas->oc; A.active = d_active; A.act_slot = nullptr;
+  A.grndlev = d_grnd; A.active = d_active; A.act_slot = nullptr;
   A.hckt = d_hckt; A.hlparr = d_hlp; A.mass = gas->mass; A.natomfr = gas->natomfr; A.temp = gas->temp;
   A.ffigg = d_ffigg; A.ffdgg = d_ffdgg; A.gff = ctx->d_gff;
   A.ffsum = d_ffsum; A.ffdsum = d_ffdsum; A.ffclamp = d_ffclamp; A.ffclamp_all = d_ffclamp + nc;
