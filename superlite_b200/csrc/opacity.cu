@@ -22,6 +22,7 @@
 //  * FP64 throughout, no FMA contraction (-fmad=false), so sums round like the
 //    single-threaded Fortran; only exp/log10/pow may differ in the last ulp.
 #include <cuda_runtime.h>
+#include <math_constants.h>
 #include <algorithm>
 #include <cfloat>
 #include "slg_device.cuh"
@@ -268,7 +269,9 @@ __device__ double bfxs(const float* __restrict__ ph1, const float* __restrict__ 
 
 // xstab[(igs-1) nslot + slot] = bfxs(iz, iz-ii+1, hc/(ev*wlsub(igs))) * pc_mbarn,
 // :177-186 (the reference's first product), for every slot that the reference
-// visits (ii <= min(iz, ni-1)), else 0.
+// visits (ii <= min(iz, ni-1)), else 0.  Without the fits (slg_set_atomic_data took
+// null) a cross section is not a number: a build whose ions have no population needs
+// none, any other gets NaN, which its sanity word reports.
 __global__ void bf_table_kernel(int ngsub, int nslot, const int32_t* __restrict__ ion_ni, int nst,
                                 const double* __restrict__ wlsub, const float* __restrict__ ph1,
                                 const float* __restrict__ ph2, double* __restrict__ xstab) {
@@ -278,7 +281,8 @@ __global__ void bf_table_kernel(int ngsub, int nslot, const int32_t* __restrict_
   const int slot = (int)(t % nslot);
   const int iz = slot / nst + 1, ii = slot % nst + 1;
   double x = 0.0;
-  if (ii <= min(iz, ion_ni[iz - 1] - 1)) x = bfxs(ph1, ph2, iz, iz - ii + 1, pc_hc / (pc_ev * wlsub[igs - 1])) * pc_mbarn;
+  if (ii <= min(iz, ion_ni[iz - 1] - 1))
+    x = ph1 && ph2 ? bfxs(ph1, ph2, iz, iz - ii + 1, pc_hc / (pc_ev * wlsub[igs - 1])) * pc_mbarn : CUDART_NAN;
   xstab[t] = x;
 }
 

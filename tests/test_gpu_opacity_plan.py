@@ -131,3 +131,23 @@ def test_cool_shell_leaves_its_neighbours_alone(hot, oracle):
     rest = np.setdiff1d(np.arange(140), cool)
     assert np.array_equal(a[rest], b[rest])
     assert not np.array_equal(a[cool], b[cool])
+
+
+def test_without_bound_free_tables(hot, oracle):
+    """No bound-free fits set: ions without population need none, and populated ones
+    give NaN and its sanity bit (no read through a null table)."""
+    import ctypes as C
+    from superlite_b200.capi import ptr
+    case = cases.reference_opacity_case(oracle, ncell=20, ng=15, nline=500, seed=4, lines="synthetic")
+    _setup(hot, case)
+    ni, lines = np.ascontiguousarray(case.gas.ion_ni, dtype=np.int32), np.ascontiguousarray(case.lines)
+    gff = np.ascontiguousarray(case.ff_gff, dtype=np.float64)
+    rc = hot.lib.slg_set_atomic_data(hot.h, len(ni), case.gas.oc.shape[1], ptr(ni), C.c_int64(len(lines)), ptr(lines),
+                                     None, None, ptr(gff))
+    assert rc == 0
+    bare = dataclasses.replace(case, gas=dataclasses.replace(case.gas, oc=np.zeros_like(case.gas.oc)))
+    _check(hot, oracle, bare)
+    got = _gpu_opacity(hot, case, nobf=True)
+    _assert_opacity_parity(got, oracle.physical_opacity(case, nobf=True))
+    got = _gpu_opacity(hot, case)
+    assert np.isnan(got["cap64"]).any() and got["sanity"] & 4
