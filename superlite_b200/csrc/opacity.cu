@@ -318,7 +318,7 @@ __global__ void bf_select_kernel(int ngsub, int nslot, int maxbf, const double* 
 // One line's shell-independent factors, 16 bytes (one vector load per line):
 // pg = phi(igs) * gxs, the first product of the reference's expression
 // (physical_opacity.f:148-149), so the evaluation order of that product is
-// kept; and chilw in FP64 with two indices in the low 29 bits of its
+// kept, times kPgScale; and chilw in FP64 with two indices in the low 29 bits of its
 // mantissa.  chilw is single precision in the line record (as in the
 // reference's bbxs type), so those bits of its FP64 value are zero: masking
 // them off gives chilw exactly, without a conversion per line.  The indices:
@@ -330,6 +330,10 @@ struct __align__(16) LineTerm {
   double pg;
   double chi_idx;
 };
+// Keeps pg exp(-chi h) a normal number for the smallest exp (1e-304; pg alone is about
+// 1e-12, and the population comes after the sum over a row); a power of two, so that
+// nothing rounds otherwise.  Taken off the sums by kPgUnscale.
+constexpr double kPgScale = 0x1p100, kPgUnscale = 0x1p-100;
 constexpr int kLineRowBits = 11;
 constexpr unsigned kLineIdxMask = 0x1fffffffu;
 constexpr unsigned kLineRowEnd = 1u << 27;
@@ -393,7 +397,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) line_terms_kernel(const slg_bbx
       const int pos = at[row] + __popc(same & ((1u << lane) - 1u));
       const double chi = (double)r.chilw;  // low 29 mantissa bits zero
       const unsigned idx = ((unsigned)slot << kLineRowBits) | (unsigned)row;
-      lt[pos] = LineTerm{phi * (double)r.gxs,
+      lt[pos] = LineTerm{phi * (double)r.gxs * kPgScale,
                          __hiloint2double(__double2hiint(chi), (int)((unsigned)__double2loint(chi) | idx))};
     }
     __syncwarp();
@@ -635,7 +639,7 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 7) opacity_fwd_kernel(const O
           }
 #pragma unroll
           for (int s = 0; s < FS; ++s)
-            if (live[s]) c[s] = sbb[s] * bb_expfac(A, igs, h[s]);
+            if (live[s]) c[s] = sbb[s] * kPgUnscale * bb_expfac(A, igs, h[s]);
         }
       }
       if (!A.nobf) {
@@ -965,7 +969,7 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 5) opacity_bwd_kernel(const O
 #pragma unroll
     for (int s = 0; s < FS; ++s) {
       eh[s] = exp(-(h[s] * wlinv));
-      ue[s] = u[s] != 0.0 ? u[s] * (1.0 - eh[s]) : 0.0;
+      ue[s] = u[s] != 0.0 ? u[s] * (1.0 - eh[s]) * kPgUnscale : 0.0;  // (a term's pg has kPgScale)
     }
     if (inrange)
       bb_adjoint<FS, true>(A.lt + l0, n, h, arg, C, ue, pop, A.ld, B.ggrnd + ii[0], A.nc, etab, mine, sbb,
@@ -976,6 +980,8 @@ __global__ void __launch_bounds__(kOpacWarps * 32, 5) opacity_bwd_kernel(const O
 #pragma unroll
     for (int s = 0; s < FS; ++s) {
       if (u[s] == 0.0) continue;
+      sbb[s] *= kPgUnscale;
+      schi[s] *= kPgUnscale;
       const double expfac = 1.0 - eh[s], T = A.temp[ii[s]];
       // h = hc/kT: d exp(-chi h)/dT = chi h/T exp(..), d expfac/dT = -(h/T) wlinv eh
       gt[s] = gt[s] + u[s] * ((h[s] / T) * (schi[s] * expfac) - sbb[s] * expfac * (h[s] / T) * wlinv * eh[s] / expfac);
