@@ -464,7 +464,7 @@ int slg_set_atomic_data(slg_ctx* ctx, int32_t nelem, int32_t nstage, const int32
   // the population rows the lines reference (the opacity plan orders a
   // sub-group's lines by them)
   const int nslot = nelem * nstage;
-  std::vector<int16_t> row_of(nslot, (int16_t)-1);
+  std::vector<int16_t> row_of(2 * (size_t)nslot, (int16_t)-1);  // by slot, then the rows' slots
   int nrow = 0;
   // the largest lower-level energy: the opacity kernels skip the range check
   // of their exp for a shell with hc/kT * chimax <= 700 (infinite when a
@@ -477,13 +477,14 @@ int slg_set_atomic_data(slg_ctx* ctx, int32_t nelem, int32_t nstage, const int32
   for (int64_t l = 0; l < nline; ++l) {
     const int sl = (bb_xs[l].iz - 1) * nstage + (bb_xs[l].ii - 1);
     if (row_of[sl] < 0) {
+      row_of[nslot + nrow] = (int16_t)sl;
       row_of[sl] = (int16_t)nrow++;
     }
   }
   free_dev(ctx->d_lrow_of_slot);
   ctx->d_lrow_of_slot = nullptr;
-  if (!rc) rc = cuda_check(ctx, cudaMalloc(&ctx->d_lrow_of_slot, sizeof(int16_t) * nslot), "alloc row map");
-  if (!rc) rc = cuda_check(ctx, cudaMemcpy(ctx->d_lrow_of_slot, row_of.data(), sizeof(int16_t) * nslot,
+  if (!rc) rc = cuda_check(ctx, cudaMalloc(&ctx->d_lrow_of_slot, sizeof(int16_t) * row_of.size()), "alloc row map");
+  if (!rc) rc = cuda_check(ctx, cudaMemcpy(ctx->d_lrow_of_slot, row_of.data(), sizeof(int16_t) * row_of.size(),
                                           cudaMemcpyHostToDevice), "row map");
   if (rc) return rc;
   ctx->nelem = nelem;

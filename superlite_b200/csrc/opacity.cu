@@ -89,8 +89,8 @@ __global__ void __launch_bounds__(CELLS * 32) opac_cell_kernel(
     const double* __restrict__ natom, const double* __restrict__ nelec, const double* __restrict__ vol,
     const double* __restrict__ mass, const double* __restrict__ oc, const double* __restrict__ ginv, int nothmson,
     const double* __restrict__ natomfr, const double* __restrict__ G, double* __restrict__ hckt,
-    double* __restrict__ gas_sig, double* __restrict__ hlparr, int ld, const int16_t* __restrict__ lrow_of_slot,
-    double* __restrict__ grndlev,
+    double* __restrict__ gas_sig, double* __restrict__ hlparr, int ld, int nrow,
+    const int16_t* __restrict__ slot_of_row, double* __restrict__ grndlev,
     double* __restrict__ ocp, int* __restrict__ active, int* __restrict__ ffigg, double* __restrict__ ffdgg, double* __restrict__ ffsum,
     double* __restrict__ ffdsum, unsigned* __restrict__ ffclamp, unsigned* __restrict__ ffclamp_all) {
   __shared__ double s_w[CELLS][32], s_dgg[CELLS][32];
@@ -99,18 +99,18 @@ __global__ void __launch_bounds__(CELLS * 32) opac_cell_kernel(
   const int nslot = nelem * nst;
   for (int t = threadIdx.x; t < nslot * CELLS; t += CELLS * 32) {  // a multiple of CELLS per slot
     const int k = t / CELLS, i = blockIdx.x * CELLS + t % CELLS;
-    double o = 0.0, v = 0.0;
+    const double o = i < nc ? oc[(size_t)k * nc + i] : 0.0;
+    if (i < ld) ocp[(size_t)k * ld + i] = o;
+    if (o != 0.0) active[k] = 1;
+  }
+  for (int t = threadIdx.x; t < nrow * CELLS; t += CELLS * 32) {  // the lines' population rows
+    const int row = t / CELLS, k = slot_of_row[row], i = blockIdx.x * CELLS + t % CELLS;
+    double v = 0.0;
     if (i < nc) {
       const int iz = k / nst + 1, ii = k % nst + 1;
-      o = oc[(size_t)k * nc + i];
-      if (ii <= min(iz, ion_ni[iz - 1] - 1) && mass[i] > 0.0) v = o * ginv[(size_t)k * nc + i];
+      if (ii <= min(iz, ion_ni[iz - 1] - 1) && mass[i] > 0.0) v = oc[(size_t)k * nc + i] * ginv[(size_t)k * nc + i];
     }
-    if (i < ld) {
-      const int row = lrow_of_slot ? lrow_of_slot[k] : -1;  // of the lines' population rows
-      if (row >= 0) grndlev[(size_t)row * ld + i] = v < 0.0 ? 0.0 : v;  // the reference skips lines with ocg <= 0
-      ocp[(size_t)k * ld + i] = o;
-    }
-    if (o != 0.0) active[k] = 1;
+    if (i < ld) grndlev[(size_t)row * ld + i] = v < 0.0 ? 0.0 : v;  // the reference skips lines with ocg <= 0
   }
   const int i = blockIdx.x * CELLS + warp;
   if (i >= nc) return;  // uniform over the warp
@@ -1378,7 +1378,8 @@ static int opacity_prepare(slg_ctx* ctx, const slg_gas* gas, const slg_opacity_f
   opac_cell_kernel<<<(ld + CELLS - 1) / CELLS, CELLS * 32, 0, st>>>(
       nc, nelem, nst, ctx->d_ion_ni, gas->temp, gas->natom, gas->nelec, gas->vol, gas->mass, gas->oc, gas->ginv,
       flags->nothmson, gas->natomfr, do_ff ? ctx->d_gff : nullptr, d_hckt, gas_sig, d_hlp, ld,
-      do_bb ? ctx->d_lrow_of_slot : nullptr, d_grnd, d_ocp, d_active, d_ffigg, d_ffdgg, d_ffsum, d_ffdsum, d_ffclamp, d_ffclamp + nc);
+      do_bb ? nrow : 0, ctx->d_lrow_of_slot + nslot, d_grnd, d_ocp, d_active, d_ffigg, d_ffdgg, d_ffsum, d_ffdsum,
+      d_ffclamp, d_ffclamp + nc);
   if (do_bf) {
     A.maxbf = 0;
     for (int z = 1; z <= nelem; ++z) A.maxbf += std::max(0, std::min(std::min(z, ctx->h_ion_ni[z - 1] - 1), nst));

@@ -191,7 +191,7 @@ struct slg_ctx {
   std::vector<int32_t> h_ion_ni;
   slg_bbxs* d_bb = nullptr;
   // population rows (slot = (iz-1) nstage + ii-1) that the lines reference:
-  // d_lrow_of_slot[slot] = compact row or -1
+  // d_lrow_of_slot[slot] = compact row or -1, after them the rows' slots
   int nlrow = 0;
   double line_chimax = 0.0;  // largest chilw of the lines (infinite if any is negative or NaN)
   int16_t* d_lrow_of_slot = nullptr;
