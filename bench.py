@@ -55,15 +55,13 @@ BYTES_PER_STEP = 128.0
 # instructions issued per particle-step and active lanes per warp instruction,
 # from one ncu capture of each variant on the batched workload at 0.1x particle
 # budgets (--transport-variant V; smsp__inst_executed.sum / particle-steps of
-# the launch; smsp__thread_inst_executed.sum / smsp__inst_executed.sum):
-# profiles/particle_advance_mixed_batched_128models_npart0.1.md
+# the launch; smsp__thread_inst_executed.sum / smsp__inst_executed.sum)
 MIXED_WARP_INST_PER_STEP = {0: 42.6, 1: 44.5, 2: 46.8, 3: 49.9}
 MIXED_LANES_PER_INST = {0: 10.69, 1: 10.27, 2: 9.96, 3: 9.63}
 # The same for the FP64 particle_advance_kernel (variants 0..3: <1, 5, 6, 8>) on
 # the --workload timestep physics (256 shells x 2000 groups, every event a DDMC
-# one), from one ncu capture of each variant at 2e5 particles
-# (profiles/launches_timestep_256x2000_1e6.md): warp instructions, active lanes
-# and DRAM bytes (read + write) per particle-step
+# one), from one ncu capture of each variant at 2e5 particles: warp instructions,
+# active lanes and DRAM bytes (read + write) per particle-step
 FP64_TIMESTEP_INST_PER_STEP = {0: 33.1, 1: 39.2, 2: 44.3, 3: 52.0}
 FP64_TIMESTEP_LANES_PER_INST = {0: 16.2, 1: 14.7, 2: 13.4, 3: 11.6}
 FP64_TIMESTEP_DRAM_PER_STEP = {0: 4.46e7 / 6.529e8, 1: 4.55e7 / 6.529e8, 2: 4.57e7 / 6.529e8, 3: 6.26e7 / 6.529e8}

@@ -107,7 +107,8 @@ int slg_set_models(slg_ctx* ctx, int32_t nmodel, const int32_t* nx, const int64_
  * ion_el(iz)%ni (nelem), the bb line list sorted by wl0 (read_bbxs_data.f:84),
  * bf_ph1(6,7,30,30), bf_ph2(7,30,30) (bfxsmod.f:14) and ff_gff(81,41)
  * (ffxsmod.f:18-20).  nstage = slots per element in the oc/ginv arrays
- * (1..64; nelem 1..30). */
+ * (1..64; nelem 1..30).  Without bf_ph1 and bf_ph2 (NULL) a build with
+ * bound-free gives NaN, and its sanity bit, for the groups of populated ions. */
 int slg_set_atomic_data(slg_ctx* ctx, int32_t nelem, int32_t nstage, const int32_t* ion_ni,
                         int64_t nline, const slg_bbxs* bb_xs, const float* bf_ph1,
                         const float* bf_ph2, const double* ff_gff);

@@ -11,16 +11,20 @@
 //    is laid out once after slg_set_groups / slg_set_atomic_data (opacity_plan):
 //    the sub-groups' line ranges, each line's 16-byte record with its
 //    sub-group's lines ordered by the population row they multiply, and the
-//    nonzero cross sections of every sub-group.
-//  * opac_cell: the shells' scalars, level populations and free-free sums.
+//    cross sections of every sub-group and ion.
+//  * opac_cell: the shells' scalars, populations and free-free sums; bf_select: the
+//    populated ions' nonzero cross sections of every sub-group.
 //  * opacity_fwd: one warp per (group, 32 FS shells).  Every lane walks the
 //    lines of its group (warp-uniform broadcast reads) and accumulates bb row
 //    by row, then bf (ions in the reference's iz,ii order), then ff (elements
-//    in order) into one register per shell.  Sub-groups are collapsed in
-//    registers, then cap and emissivity are written through a shared-memory
-//    tile so each shell's 8 groups leave as one 32-byte sector.
-//  * FP64 throughout, no FMA contraction (-fmad=false), so sums round like the
-//    single-threaded Fortran; only exp/log10/pow may differ in the last ulp.
+//    summed per shell beforehand) into one register per shell.  Sub-groups are
+//    collapsed in registers.  A shell's values go to memory one by one: its
+//    neighbouring groups are the neighbouring blocks', and the parts of a sector
+//    meet in L2.
+//  * FP64 throughout, compiled without FMA contraction; the bb and bf sums use
+//    explicit fused multiply-adds and bb sums run row by row, so opacities agree
+//    with the single-threaded Fortran to rounding (1e-12 relative is tested), not
+//    to the bit.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <algorithm>
@@ -32,7 +36,10 @@ namespace slg {
 
 namespace {
 
-constexpr int kMaxLineSubgroups = 18770;  // sub-groups that the line binning accepts
+// Builds with lines take up to this many sub-groups and refuse more.  Nothing here
+// needs the limit (an earlier layout held the edges in shared memory); callers see the
+// same sizes accepted and refused as ever.
+constexpr int kMaxLineSubgroups = 18770;
 constexpr int OPAC_CT = 32;  // lanes of a warp, each with one or more shells
 
 // ------------------------------------------------------------ line ranges
@@ -77,9 +84,9 @@ __global__ void line_range_kernel(const slg_bbxs* __restrict__ bb, int64_t nline
 // A block takes CELLS shells: first the populations, shells fastest, then a warp
 // per shell: a lane per element finds its columns, the elements that enter the
 // sums are compacted into shared memory, and the lanes take the 81 table rows.
-// (As one thread per (shell, row) that walked all elements the sums alone took
-// 17-20 us whatever the grid, besides 9 us for the rest; now 15 us in all at 32 and
-// at 256 shells, 20 us at 4096.)
+// (Cold caches, under the profiler: as one thread per (shell, row) that walked all
+// elements the sums alone took 17-20 us whatever the grid, besides 9 us for the rest;
+// now 12 us in all at 256 shells, 18 at 4096.)
 constexpr int CELLS = 8;
 // Length of a population row: whole warps' shells (64 of two per lane, 32 up to 32
 // shells, which are one per lane).
@@ -586,10 +593,11 @@ __device__ __forceinline__ double bb_expfac(const OpacArgs& A, int igs, double h
 // FS shells per lane share a line record's load and index work; the warps of a
 // block walk the same lines, so they share the records in L1 and end together;
 // lines ordered by row leave one multiplication and one population load per row.
-// Seven blocks per SM (72 registers) measured best of four to eight.  4096
-// shells x 10000 groups x 2e6 lines: 9.6 -> 8.9 ms, 256 x 2000 x 5e5: 184 -> 165 us
-// (lines in file order, four shells per lane, populations staged in shared
-// memory, exp without the scaled argument and the spread table).
+// Seven blocks per SM (72 registers) measured best of four to eight.  Whole builds
+// in a loop on B200, before (lines in file order, four shells per lane, populations
+// staged in shared memory, exp without the scaled argument and the spread table) and
+// now: 4096 shells x 10000 groups x 2e6 lines 10.6 -> 9.65 ms, 256 x 2000 x 5e5 253 ->
+// 173 us, 190 -> 134 where few ions are populated.
 template <int FS>
 __global__ void __launch_bounds__(kOpacWarps * 32, 7) opacity_fwd_kernel(const OpacArgs A, const ExpConst C, int gpb) {
   constexpr int FC = FS * OPAC_CT;

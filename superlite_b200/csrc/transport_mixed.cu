@@ -392,9 +392,9 @@ __device__ inline void diffusion11_mix(const TrnArgs& A, const MView& v, PtclM& 
                                             (right ? A.T.cdf32_right : A.T.cdf32_left) + off, glump, rng.draw())];
     // IMC in the neighbour for the group that leaks: the sign bit of this
     // group's leak rate, or the neighbour's rate sentinel for a resolved group
-    const bool to_imc = glump == 0 ? signbit(right ? rt.z : rt.y)
-                                   : __ldg(&A.mrate[(size_t)(v.co + l - 1) * ng + iiig - 1].x) == kRateIMC;
-    if (to_imc) {
+    const bool face_imc = glump == 0 ? signbit(right ? rt.z : rt.y)
+                                    : __ldg(&A.mrate[(size_t)(v.co + l - 1) * ng + iiig - 1].x) == kRateIMC;
+    if (face_imc) {
       p.itype = 1;
       const float r = rng.draw();
       wl = 1.0f / (r * (float)A.wlinv[iiig] + (1.0f - r) * (float)A.wlinv[iiig - 1]);
