@@ -378,7 +378,9 @@ constexpr int kMixedVariants = 4;
 // v < 0 (nobody chose): the one without spills for one model (variants 0 / 1 / 2
 // / 3: 86 / 91 / 102 / 105 ms at 256 shells x 2000 groups, 4e5 particles; 48 /
 // 51 / 54 / 57 ms at 64 x 100, 1e6 particles), five blocks per SM for several,
-// whose kernel holds more state (2.04 / 1.80 / 2.11 / 2.42 s, 64 models).
+// whose kernel holds more state (2.04 / 1.80 / 2.11 / 2.42 s, 64 models at full
+// budgets; batches that end sooner favour variant 0: 64 models of 1e5 particles 415 /
+// 449 / 480 / 555 ms, two of 1e6 493 / 576 / 646 / 753).  All give the same bits.
 constexpr int kTransportVariants = 4;
 int launch_transport_variant(int v, bool trace, int num_sms, long long npart, cudaStream_t st, const TrnArgs& A) {
   if (v < 0) v = A.nmodel > 1 ? 1 : 0;
